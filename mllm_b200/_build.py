@@ -50,7 +50,7 @@ _COMMON = ["bindings_common.h", "common.cuh", "kernels.h", "mma.cuh", "row.cuh"]
 EXTENSIONS: Dict[str, Dict[str, List[str]]] = {
     "mllm_b200_C": {
         "sources": ["bindings.cpp", "runtime.cu", "elementwise.cu", "row_ops.cu", "depth.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "attention.cu",
-                    "attention_rows.cu", "sampling.cu", "no_alloc.cu"],
+                    "attention_decode.cu", "attention_rows.cu", "sampling.cu", "no_alloc.cu"],
         "headers": _COMMON + ["no_alloc.h"],
         "cuda": True,
     },

@@ -1,6 +1,7 @@
 // Attention over the slot-indexed KV pool on tcgen05 tensor cores.  The single-role kernel described first is
 // instantiated for head sizes 64, 128 and 256 (one, two or four 64-feature halves per row; the figures below
-// are those of 128); the warp-specialised prefill and decode kernels further down are for head size 128.
+// are those of 128); the warp-specialised prefill kernel further down is for head size 128.  Decode over 16-bit caches is in
+// attention_decode.cu; the single-role kernel decodes over 8-bit caches and for wider groups of query heads.
 //
 // One kernel serves prefill (ragged new tokens after an optional cached prefix, causal) and
 // decode (one token per request, split over the KV length): a CTA owns one request, one KV
@@ -504,45 +505,6 @@ __global__ void __launch_bounds__(kAttnThreads, FwdCfg<NH>::kCtasPerSm) attn_fwd
 }
 
 
-template <int N>
-__device__ __forceinline__ float m_used_at(const float (&m)[N], int idx) {
-  float v = 0.f;
-#pragma unroll
-  for (int c = 0; c < N; ++c) v = (c == idx) ? m[c] : v;
-  return v;
-}
-
-// ---------------------------------------------------------------------------------------------
-// Decode-specialised kernel: one query token per request, so the roles of the MMA dimensions are
-// swapped - the 128 KV tokens of a tile are the MMA M dimension and the (padded) query heads of
-// the GQA group are the N dimension:
-//   S^T[tok, q] = K[tok, d] Q^T          (A = K tile, K-major; B = Q, K-major)
-//   O^T[d, q]  += V^T[d, tok] P^T[tok, q] (A = V tile as gathered, used MN-major; B = P^T, K-major)
-// A softmax thread owns one token (only the per-head maximum crosses threads, once per tile; the
-// row sums stay per-thread until the end) and one feature d of the output, so the final store is
-// coalesced.  The CTA is warp-specialised and coupled by mbarriers only:
-//   warps 0-3  softmax: tcgen05.ld S^T, running max, exponentials, P^T to shared memory
-//   warp  4    producer: reads the request's slot table and moves K and V rows with the TMA engine into
-//              two three-deep rings, in the 128-byte-swizzled operand layout.  Groups of 16 tokens whose
-//              slots are consecutive (paged allocation, or a prompt that was given one run of slots) are
-//              plain 2 KB boxes when the pool is stored head-major; other groups are gathered row by row
-//              (cp.async.bulk.tensor ... tile::gather4: four pool rows, given by index, per copy).
-//   warp  5    one thread issues the MMAs: S^T of tile t is queued before P*V of tile t-1, so the
-//              tensor-core and barrier latency of S^T hides behind the softmax of the tile before
-// ---------------------------------------------------------------------------------------------
-constexpr int kDT = 128;                       // tokens per decode tile
-constexpr int kDecHalf = kDT * 128;            // bytes of one 64-feature half of a K or V tile
-constexpr int kDecTileBytes = 2 * kDecHalf;    // 32 KB per tensor
-constexpr int kDecBufs = 3;
-constexpr int kDecThreads = 192;
-
-template <int NQ>
-struct DecCfg {
-  static constexpr int kQBytes = 2 * NQ * 128;   // Q^T operand: two halves of NQ rows x 128 B
-  static constexpr int kPBytes = 2 * NQ * 128;   // P^T operand: two halves (64 tokens each)
-  static constexpr int kSmem = kDecBufs * 2 * kDecTileBytes + kQBytes + kPBytes + 1024 + 256 + 9 * NQ * 4;
-};
-
 // Four rows of a 2-D tensor (row indices r[0..3], 64 16-bit columns starting at column x: one 128-byte
 // swizzle span per row) to four consecutive 128-byte rows of shared memory.  The tensor map's box is
 // {64, 1}; the copy signals 512 bytes on `bar`.  x * 2 bytes must be a multiple of 16.
@@ -556,420 +518,12 @@ __device__ __forceinline__ void tma_gather4(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
-template <int NQ>
-__global__ void __launch_bounds__(kDecThreads, 1)
-attn_decode_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
-                   const __grid_constant__ CUtensorMap tm_k_run, const __grid_constant__ CUtensorMap tm_v_run,
-                   const AttnParams p) {
-  using C = DecCfg<NQ>;
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sK = smem;                                   // kDecBufs tiles
-  uint8_t* sV = sK + kDecBufs * kDecTileBytes;          // kDecBufs tiles
-  uint8_t* sQ = sV + kDecBufs * kDecTileBytes;
-  uint8_t* sP = sQ + C::kQBytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sP + C::kPBytes);
-  uint64_t* k_full = bars;            // [3] TMA transaction bytes
-  uint64_t* k_empty = bars + 3;       // [3] tcgen05.commit
-  uint64_t* v_full = bars + 6;        // [3]
-  uint64_t* v_empty = bars + 9;       // [3]
-  uint64_t* s_full = bars + 12;       // [2] tcgen05.commit
-  uint64_t* s_empty = bars + 14;      // [2] 128 softmax threads
-  uint64_t* p_full = bars + 16;       // 128 softmax threads
-  uint64_t* p_empty = bars + 17;      // tcgen05.commit (P*V of the tile finished)
-  uint64_t* q_full = bars + 18;       // producer warp: Q^T operand written
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 19);
-  int* fail_flag = reinterpret_cast<int*>(tmem_holder + 1);
-  float* red = reinterpret_cast<float*>(bars + 20);     // [2][4 warps][NQ] tile maxima, double buffered
-  float* red2 = red + 8 * NQ;                           // [NQ] totals
-
-  const int tid = threadIdx.x;
-  const int warp = tid >> 5;
-  const int lane = tid & 31;
-  const int b = blockIdx.z;
-  const int hk = blockIdx.y;
-  const int split = blockIdx.x;
-  const int g = p.group;
-
-  if (tid == 0) {
-    for (int i = 0; i < 3; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
-      mbar_init(&v_full[i], 1);
-      mbar_init(&v_empty[i], 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&s_full[i], 1);
-      mbar_init(&s_empty[i], 128);
-    }
-    mbar_init(p_full, 128);
-    mbar_init(p_empty, 1);
-    mbar_init(q_full, 1);
-    *fail_flag = 0;
-    fence_barrier_init();
-    tma_prefetch_desc(&tm_k);
-    tma_prefetch_desc(&tm_v);
-    tma_prefetch_desc(&tm_k_run);
-    tma_prefetch_desc(&tm_v_run);
-  }
-  // rows of P^T beyond the group are never written again: clear them once
-  for (int i = tid; i < C::kPBytes / 16; i += kDecThreads) reinterpret_cast<uint4*>(sP)[i] = make_uint4(0, 0, 0, 0);
-  fence_proxy_async_smem();
-  __syncthreads();
-  if (warp == 5) {
-    tmem_alloc(tmem_holder, 128);
-    tmem_relinquish();
-  }
-  tc_fence_before_sync();
-  __syncthreads();
-  tc_fence_after_sync();
-  const uint32_t tmem_base = *tmem_holder;
-  const uint32_t tmem_s = tmem_base;            // two buffers of NQ columns
-  const uint32_t tmem_o = tmem_base + 2 * NQ;   // NQ columns
-  // everything above touched no global memory; sequence lengths, slot table, Q and the KV pool are
-  // written by earlier kernels of the stream
-  pdl_wait();
-
-  const int req = p.req_pool_indices[b];
-  const int seq_len = p.seq_lens[b];
-  const int kv_lo = first_key(p, seq_len - 1);   // first key the (single) query sees
-  const int lo_tile = kv_lo / kDT * kDT;
-  const int tiles = (seq_len - lo_tile + kDT - 1) / kDT;
-  const int per = (tiles + p.num_splits - 1) / p.num_splits;
-  const int kv_begin = lo_tile + split * per * kDT;
-  const int kv_end = min(seq_len, kv_begin + per * kDT);
-  const int n_tiles = kv_begin < kv_end ? (kv_end - kv_begin + kDT - 1) / kDT : 0;
-
-  if (n_tiles == 0) {
-    // nothing to attend to: a neutral partial for the merge, or an all-zero output row
-    if (p.num_splits > 1) {
-      for (int i = tid; i < g * kD; i += kDecThreads) {
-        const int head = hk * g + i / kD;
-        p.part_o[((static_cast<int64_t>(b) * p.hq + head) * p.num_splits + split) * kD + (i % kD)] = 0.f;
-      }
-      if (tid < g) p.part_lse[(static_cast<int64_t>(b) * p.hq + hk * g + tid) * p.num_splits + split] = -INFINITY;
-    } else {
-      for (int i = tid; i < g * kD; i += kDecThreads)
-        static_cast<uint16_t*>(p.out)[b * p.out_stride + hk * g * kD + i] = 0;
-    }
-  } else if (warp == 4) {
-    // =============================== producer warp ===============================
-    const int* rtt = p.req_to_token + static_cast<int64_t>(req) * p.rtt_stride;
-    bool ok_all = true, bad = false;
-    // A lane owns four consecutive tokens of the tile; the four lanes of a quad own a group of 16.  When the
-    // 16 slots of a group are consecutive and the storage is head-major, the group's K and V rows are four
-    // plain 2 KB boxes (K low / high feature half, V low / high) and each lane of the quad issues one of them;
-    // otherwise every lane gathers its own four rows, four at a time by index.
-    const int grp = lane >> 2, sub = lane & 3;
-    auto load_slots = [&](int tile, int (&sl4)[4]) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int tk = min(kv_begin + tile * kDT + grp * 16 + sub * 4 + j, kv_end - 1);
-        sl4[j] = tile < n_tiles ? __ldg(rtt + tk) : 0;
-      }
-    };
-    int cur[4], nxt[4];
-    load_slots(0, cur);
-    for (int t = 0; t < n_tiles && ok_all; ++t) {
-      const int sl = t % kDecBufs;
-      const uint32_t ph = (t / kDecBufs) & 1;
-      load_slots(t + 1, nxt);   // used one tile from now
-      bool run = p.kv_runs != 0;
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        if (cur[j] < 0 || cur[j] >= p.num_slots) {
-          bad = true;
-          cur[j] = 0;
-        }
-      }
-      const int first = __shfl_sync(0xffffffffu, cur[0], lane & ~3);   // slot of the group's first token
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int tk = kv_begin + t * kDT + grp * 16 + sub * 4 + j;
-        // tokens past the end repeat the last slot and are masked: they do not break a run
-        run = run && (tk >= kv_end || cur[j] == first + sub * 4 + j);
-      }
-      const uint32_t votes = __ballot_sync(0xffffffffu, run);
-      run = ((votes >> (lane & ~3)) & 0xFu) == 0xFu && first + 16 <= p.num_slots;
-      if (!mbar_wait(&k_empty[sl], ph ^ 1, fail_flag)) ok_all = false;
-      if (!mbar_wait(&v_empty[sl], ph ^ 1, fail_flag)) ok_all = false;
-      if (!__all_sync(0xffffffffu, ok_all)) {
-        ok_all = false;
-        break;
-      }
-      if (lane == 0) {
-        mbar_arrive_expect_tx(&k_full[sl], kDecTileBytes);
-        mbar_arrive_expect_tx(&v_full[sl], kDecTileBytes);
-      }
-      __syncwarp();
-      uint8_t* tile_k = sK + sl * kDecTileBytes;
-      uint8_t* tile_v = sV + sl * kDecTileBytes;
-      if (run) {
-        const int row0 = first * p.kv_row_mul + hk * p.kv_row_add;
-        const int half = sub & 1;
-        uint8_t* dst = (sub < 2 ? tile_k : tile_v) + half * kDecHalf + grp * 16 * 128;
-        tma_load_2d(dst, sub < 2 ? &tm_k_run : &tm_v_run, sub < 2 ? &k_full[sl] : &v_full[sl], half * 64, row0);
-      } else {
-        int rows[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) rows[j] = cur[j] * p.kv_row_mul + hk * p.kv_row_add;
-        const int off = (grp * 16 + sub * 4) * 128;
-        tma_gather4(tile_k + off, &tm_k, &k_full[sl], 0, rows);
-        tma_gather4(tile_k + kDecHalf + off, &tm_k, &k_full[sl], 64, rows);
-        tma_gather4(tile_v + off, &tm_v, &v_full[sl], 0, rows);
-        tma_gather4(tile_v + kDecHalf + off, &tm_v, &v_full[sl], 64, rows);
-      }
-      if (t == 0) {   // the first K and V tiles are on their way: stage the Q^T operand meanwhile
-      {  // Q^T operand: NQ rows (query heads, zero beyond the group) x 16 chunks of 16 bytes
-        const uint16_t* qbase = static_cast<const uint16_t*>(p.q);
-        for (int c = lane; c < NQ * 16; c += 32) {
-          const int r = c >> 4, qc = c & 15;
-          uint4 v = make_uint4(0, 0, 0, 0);
-          if (r < g)
-            v = *reinterpret_cast<const uint4*>(qbase + static_cast<int64_t>(b) * p.q_stride +
-                                                static_cast<int64_t>(hk * g + r) * kD + qc * 8);
-          *reinterpret_cast<uint4*>(sQ + swz_off(r, qc, NQ * 128)) = v;
-        }
-        fence_proxy_async_smem();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(q_full);
-      }
-      }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) cur[j] = nxt[j];
-    }
-    if (bad && p.status != nullptr) atomicExch(p.status, kStatusBadIndex);
-    if (!ok_all) *fail_flag = 1;
-  } else if (warp == 5) {
-    // =============================== MMA issuer ===============================
-    if (lane == 0) {
-      bool ok_all = mbar_wait(q_full, 0, fail_flag);
-      auto issue_pv = [&](int u) {
-        const int sl = u % kDecBufs;
-        if (!mbar_wait(&v_full[sl], (u / kDecBufs) & 1, fail_flag)) ok_all = false;
-        if (!mbar_wait(p_full, u & 1, fail_flag)) ok_all = false;
-        if (!ok_all) return;
-        tc_fence_after_sync();
-        const uint32_t va = smem_u32(sV + sl * kDecTileBytes);
-        const uint32_t pa = smem_u32(sP);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t a_desc = umma_desc_mn_sw128(va + kk * 2048, kDecHalf, 1024);
-          const uint64_t b_desc = umma_desc_k_sw128(pa + (kk >> 2) * (NQ * 128) + (kk & 3) * 32);
-          umma_f16(tmem_o, a_desc, b_desc, p.idesc_o, (u > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(&v_empty[sl]);
-        umma_commit(p_empty);
-      };
-      for (int t = 0; t < n_tiles && ok_all; ++t) {
-        const int sl = t % kDecBufs;
-        if (!mbar_wait(&k_full[sl], (t / kDecBufs) & 1, fail_flag)) ok_all = false;
-        if (!mbar_wait(&s_empty[t & 1], ((t >> 1) & 1) ^ 1, fail_flag)) ok_all = false;
-        if (!ok_all) break;
-        tc_fence_after_sync();
-        const uint32_t ka = smem_u32(sK + sl * kDecTileBytes);
-        const uint32_t qa = smem_u32(sQ);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t a_desc = umma_desc_k_sw128(ka + (kk >> 2) * kDecHalf + (kk & 3) * 32);
-          const uint64_t b_desc = umma_desc_k_sw128(qa + (kk >> 2) * (NQ * 128) + (kk & 3) * 32);
-          umma_f16(tmem_s + (t & 1) * NQ, a_desc, b_desc, p.idesc_s, kk > 0 ? 1u : 0u);
-        }
-        umma_commit(&k_empty[sl]);
-        umma_commit(&s_full[t & 1]);
-        if (t > 0) issue_pv(t - 1);
-      }
-      if (ok_all) issue_pv(n_tiles - 1);
-      if (!ok_all) *fail_flag = 1;
-    }
-  } else {
-    // =============================== softmax warps ===============================
-    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
-    float m_used[NQ];
-    float l_part[NQ];
-#pragma unroll
-    for (int c = 0; c < NQ; ++c) {
-      m_used[c] = 0.f;
-      l_part[c] = 0.f;
-    }
-    bool ok_all = true;
-    for (int t = 0; t < n_tiles; ++t) {
-      if (!mbar_wait(&s_full[t & 1], (t >> 1) & 1, fail_flag)) {
-        ok_all = false;
-        break;
-      }
-      tc_fence_after_sync();
-      float sc[NQ];
-      {
-        uint32_t raw[16];
-#pragma unroll
-        for (int c0 = 0; c0 < NQ; c0 += 16) {
-          tmem_ld_32x16(tmem_s + (t & 1) * NQ + lane_base + c0, raw);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) sc[c0 + i] = __uint_as_float(raw[i]);
-        }
-      }
-      tc_fence_before_sync();
-      mbar_arrive(&s_empty[t & 1]);  // the S^T buffer may be overwritten by tile t+2
-      const int tok_pos = kv_begin + t * kDT + tid;
-      const bool tok_ok = tok_pos < kv_end && tok_pos >= kv_lo;
-      float* redt = red + (t & 1) * 4 * NQ;
-      if (p.logit_cap > 0.f) {   // uniform branch outside the loop: plain scores pay one multiply
-#pragma unroll
-        for (int c = 0; c < NQ; ++c) sc[c] = p.cap_post * tanhf(sc[c] * p.cap_pre);
-      } else {
-#pragma unroll
-        for (int c = 0; c < NQ; ++c) sc[c] *= p.scale_log2;
-      }
-#pragma unroll
-      for (int c = 0; c < NQ; ++c) {
-        if (c < g) {
-          sc[c] = tok_ok ? sc[c] : -INFINITY;
-          const float wm = warp_max(sc[c]);
-          if (lane == 0) redt[warp * NQ + c] = wm;
-        }
-      }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      bool need = false;
-      float factor[NQ];
-#pragma unroll
-      for (int c = 0; c < NQ; ++c) {
-        factor[c] = 1.f;
-        if (c < g) {
-          const float mt = fmaxf(fmaxf(redt[c], redt[NQ + c]), fmaxf(redt[2 * NQ + c], redt[3 * NQ + c]));
-          if (t == 0) {
-            m_used[c] = mt;  // the first tile of a non-empty range always holds a visible token
-          } else if (mt > m_used[c] + kRescaleThreshold) {
-            factor[c] = fast_exp2(m_used[c] - mt);
-            m_used[c] = mt;
-            l_part[c] *= factor[c];
-            need = true;
-          }
-        }
-      }
-      // P*V of the previous tile must be finished before P^T and O^T are touched again
-      if (t > 0) {
-        if (!mbar_wait(p_empty, (t - 1) & 1, fail_flag)) {
-          ok_all = false;
-          break;
-        }
-        tc_fence_after_sync();
-      }
-      if (need) {  // uniform over the four warps: every thread sees the same maxima
-        uint32_t o[16];
-#pragma unroll
-        for (int c0 = 0; c0 < NQ; c0 += 16) {
-          tmem_ld_32x16(tmem_o + lane_base + c0, o);
-          tmem_ld_wait();
-#pragma unroll
-          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor[c0 + i]);
-          tmem_st_32x16(tmem_o + lane_base + c0, o);
-        }
-        tmem_st_wait();
-      }
-      // P^T operand: row = query head, 128 tokens in two 64-token halves; this thread writes column tid
-      {
-        uint8_t* pbase = sP + (tid >> 6) * (NQ * 128);
-        const int tk = tid & 63;
-#pragma unroll
-        for (int c = 0; c < NQ; ++c) {
-          if (c < g) {
-            const float pv = fast_exp2(sc[c] - m_used[c]);
-            uint16_t bits;
-            float back;
-            if (p.out_f16) {
-              const __half ph = __float2half_rn(pv);
-              bits = *reinterpret_cast<const uint16_t*>(&ph);
-              back = __half2float(ph);
-            } else {
-              const __nv_bfloat16 pb = __float2bfloat16_rn(pv);
-              bits = *reinterpret_cast<const uint16_t*>(&pb);
-              back = __bfloat162float(pb);
-            }
-            l_part[c] += back;
-            *reinterpret_cast<uint16_t*>(pbase + c * 128 + (((tk >> 3) ^ (c & 7)) << 4) + (tk & 7) * 2) = bits;
-          }
-        }
-      }
-      fence_proxy_async_smem();
-      tc_fence_before_sync();
-      mbar_arrive(p_full);
-    }
-    if (ok_all && !mbar_wait(p_empty, (n_tiles - 1) & 1, fail_flag)) ok_all = false;
-    tc_fence_after_sync();
-    if (!ok_all) *fail_flag = 1;
-
-    // ---- totals of the row sums over the 128 token-threads ----
-    float* redt = red;
-#pragma unroll
-    for (int c = 0; c < NQ; ++c) {
-      if (c < g) {
-        const float ws = warp_sum(l_part[c]);
-        if (lane == 0) redt[warp * NQ + c] = ws;
-      }
-    }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    if (tid < g) {
-      float l = redt[tid] + redt[NQ + tid] + redt[2 * NQ + tid] + redt[3 * NQ + tid];
-      if (p.sink != nullptr && p.num_splits == 1) l += sink_term(p.sink, hk * g + tid, m_used_at(m_used, tid));
-      red2[tid] = l;
-    }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
-    const bool good = ok_all && (*fail_flag == 0);
-
-    // ---- output: this thread owns feature d = tid of every head of the group ----
-    uint32_t o[16];
-#pragma unroll
-    for (int c0 = 0; c0 < NQ; c0 += 16) {
-      tmem_ld_32x16(tmem_o + lane_base + c0, o);
-      tmem_ld_wait();
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const int c = c0 + i;
-        if (c < g && good) {
-          const float l = red2[c];
-          const float v = l > 0.f ? __uint_as_float(o[i]) / l : 0.f;
-          const int head = hk * g + c;
-          if (p.num_splits > 1) {
-            p.part_o[((static_cast<int64_t>(b) * p.hq + head) * p.num_splits + split) * kD + tid] = v;
-          } else {
-            const int64_t oi = b * p.out_stride + head * kD + tid;
-            if (p.out_f16)
-              static_cast<__half*>(p.out)[oi] = __float2half_rn(v);
-            else
-              static_cast<__nv_bfloat16*>(p.out)[oi] = __float2bfloat16_rn(v);
-          }
-        }
-      }
-    }
-    if (p.num_splits > 1 && tid < g) {
-      const float l = red2[tid];
-      p.part_lse[(static_cast<int64_t>(b) * p.hq + hk * g + tid) * p.num_splits + split] =
-          l > 0.f ? (m_used_at(m_used, tid) + log2f(l)) : -INFINITY;
-    }
-  }
-
-  tc_fence_before_sync();
-  __syncthreads();
-  if (*fail_flag) {
-    if (tid == 0 && p.status != nullptr) atomicExch(p.status, kStatusPipelineTimeout);
-    // copies of the producer may still be in flight: give them time to land before the CTA's memory is reused
-    for (int i = 0; i < 64; ++i) __nanosleep(1000);
-    __syncthreads();
-  }
-  if (warp == 5) {
-    tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 128);
-  }
-}
-
 // ---------------------------------------------------------------------------------------------
 // Prefill kernel, warp-specialised.  A CTA owns one request, one KV head and TWO tiles of 128 rows (a row is a
 // (query token, query head of the GQA group) pair, as above), so every K/V tile that reaches shared memory
 // serves both; KV tiles hold 128 tokens.  The CTA's roles meet only at mbarriers:
 //   warps 0-3  softmax of row tile A      warps 4-7  softmax of row tile B
-//   warp  8    producer: the decode kernel's TMA path (2 KB boxes over runs of 16 consecutive slots, else
+//   warp  8    producer: moves rows by slot with the TMA engine (2 KB boxes over runs of 16 consecutive slots, else
 //              gather4 by row index) into a two-slot K ring and a single V slot
 //   warp  9    one thread issues the MMAs.  Tensor memory holds S_A, S_B (128 columns each) and O_A, O_B.
 // A softmax thread pulls its whole S row (128 scores) into registers with four tcgen05.ld and releases the S
@@ -1436,7 +990,7 @@ int launch_fwd_cfg(const AttnParams& p, dim3 grid, cudaStream_t s) {
 int decode_num_splits(int batch, int hkv, int max_seq_len, int num_sms) {
   const int ctas = std::max(1, batch * hkv);
   // one resident CTA per SM: fill a single wave, never start a second one for a remainder
-  const int tiles = std::max(1, (max_seq_len + kDT - 1) / kDT);
+  const int tiles = std::max(1, (max_seq_len + 2 * kKV - 1) / (2 * kKV));
   int splits = num_sms / ctas;
   splits = std::min(splits, std::max(1, tiles / 2));
   return std::max(1, std::min(splits, 64));
@@ -1468,31 +1022,11 @@ int launch_prefill_ws(AttnParams p, const AttnArgs& a, cudaStream_t s) {
   return err == cudaSuccess ? 0 : -4;
 }
 
-template <int NQ>
-int launch_decode_cfg(const AttnParams& p, const AttnArgs& a, dim3 grid, cudaStream_t s) {
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(attn_decode_kernel<NQ>), DecCfg<NQ>::kSmem) != cudaSuccess)
-    return -3;
-  // the K and V pools as 2-D tensors [slots * kv heads, 128] with one 64-column row per box: the form
-  // the gather copies take
-  CUtensorMap tm_k, tm_v, tm_k_run, tm_v_run;
-  const int type = a.dt == kF16 ? 1 : 0;
-  const int64_t rows = a.num_slots * static_cast<int64_t>(a.hkv);
-  if (rows >= (int64_t(1) << 31)) return -1;
-  if (!make_tma_operand_map(&tm_k, a.k_cache, rows, kD, kD, 2, type, 1)) return -2;
-  if (!make_tma_operand_map(&tm_v, a.v_cache, rows, kD, kD, 2, type, 1)) return -2;
-  if (!make_tma_operand_map(&tm_k_run, a.k_cache, rows, kD, kD, 2, type, 16)) return -2;
-  if (!make_tma_operand_map(&tm_v_run, a.v_cache, rows, kD, kD, 2, type, 16)) return -2;
-  const cudaError_t err = launch_pdl(attn_decode_kernel<NQ>, grid, dim3(kDecThreads), DecCfg<NQ>::kSmem, s, tm_k, tm_v,
-                                     tm_k_run, tm_v_run, p);
-  note_launch();
-  return err == cudaSuccess ? 0 : -4;
-}
-
 int launch_attention(const AttnArgs& a, cudaStream_t s) {
   // head size 128 has the specialised prefill and decode kernels; 64 and 256 run on the single-role kernel
   const int hd = a.head_dim;
   if ((hd != 64 && hd != 128 && hd != 256) || a.hq % a.hkv != 0) return -1;
-  // the specialised kernels move K and V with the TMA engine as they are stored: a cache of the activation dtype
+  // the specialised kernels read K and V as they are stored: a cache of the activation dtype
   const bool specialised = hd == kD && a.kv_fmt == 0;
   const int g = a.hq / a.hkv;
   if (g > kRows) return -1;
@@ -1526,7 +1060,11 @@ int launch_attention(const AttnArgs& a, cudaStream_t s) {
     p.kv_row_add = static_cast<int>(a.num_slots);
     p.kv_runs = 1;
   } else if (a.is_decode && specialised && g <= 32) {
-    return -1;                   // the decode kernel reads the caches through 2-D tensor maps
+    return -1;                   // decode at this head size is for the two layouts that the pools have
+  }
+  if (a.is_decode && decode_streams(hd, g, a.kv_fmt)) {
+    if ((reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache)) & 15) return -2;
+    return a.batch <= 0 ? 0 : launch_decode_stream(a, s);
   }
   p.hq = a.hq;
   p.hkv = a.hkv;
@@ -1549,19 +1087,6 @@ int launch_attention(const AttnArgs& a, cudaStream_t s) {
   p.idesc_o = umma_idesc(kRows, hd, 1, fmt, fmt, 0, 1);
   if (a.batch <= 0) return 0;
   dim3 grid;
-  if (specialised && a.is_decode && g <= 32) {
-    const int nq = g <= 16 ? 16 : 32;
-    p.idesc_s = umma_idesc(kRows, nq, 1, fmt, fmt, 0, 0);
-    p.idesc_o = umma_idesc(kRows, nq, 1, fmt, fmt, 1, 0);
-    grid = dim3(p.num_splits, a.hkv, a.batch);
-    const int rc = nq == 16 ? launch_decode_cfg<16>(p, a, grid, s) : launch_decode_cfg<32>(p, a, grid, s);
-    if (rc != 0) return rc;
-    if (p.num_splits > 1) {
-      launch_pdl(attn_merge_kernel, dim3(a.hq, a.batch), dim3(kD), 0, s, a.part_o, a.part_lse, a.out, p.out_stride, a.hq, p.num_splits, p.out_f16, a.sink);
-      note_launch();
-    }
-    return cudaGetLastError() == cudaSuccess ? 0 : -4;
-  }
   if (specialised && !a.is_decode) {
     const int rc = launch_prefill_ws(p, a, s);
     if (rc <= 0) return rc;

@@ -894,9 +894,13 @@ void attention_decode(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
   int64_t longest = max_seq_len > 0 ? max_seq_len : req_to_token.size(1);
   const int64_t seen = window > 0 ? window : chunk;
   if (seen > 0) longest = std::min(longest, seen + 128);     // keys read, up to the tiles' alignment
-  a.num_splits = mb200::decode_num_splits(a.batch, a.hkv, longest, st.num_sms);
   Tensor part_o, part_lse;
-  if (a.num_splits > 1) {
+  const int group = a.hkv > 0 ? a.hq / a.hkv : 0;
+  if (mb200::decode_streams(hd, group, kv_fmt)) {
+    a.num_splits = mb200::decode_stream_ctas(hd, st.num_sms);
+    part_o = torch::empty({mb200::decode_stream_floats(hd, group, a.num_splits)}, q.options().dtype(torch::kFloat32));
+    a.part_o = part_o.data_ptr<float>();
+  } else if ((a.num_splits = mb200::decode_num_splits(a.batch, a.hkv, longest, st.num_sms)) > 1) {
     part_o = torch::empty({a.batch, a.hq, a.num_splits, hd}, q.options().dtype(torch::kFloat32));
     part_lse = torch::empty({a.batch, a.hq, a.num_splits}, q.options().dtype(torch::kFloat32));
     a.part_o = part_o.data_ptr<float>();

@@ -386,6 +386,12 @@ struct AttnArgs {
   int kv_fmt;               // 0: the caches hold dt; 1 / 2: unscaled e4m3 / e5m2 bytes (strides then count bytes)
 };
 int launch_attention(const AttnArgs& args, cudaStream_t s);
+// Decode by the streaming kernel (attention_decode.cu): whether it takes a shape, how many CTAs it wants, the fp32 numbers
+// of its partial results (AttnArgs::part_o; num_splits then holds the CTAs).
+bool decode_streams(int head_dim, int group, int kv_fmt);
+int decode_stream_ctas(int head_dim, int num_sms);
+int64_t decode_stream_floats(int head_dim, int group, int ctas);
+int launch_decode_stream(const AttnArgs& args, cudaStream_t s);
 int decode_num_splits(int batch, int hkv, int max_seq_len, int num_sms);
 
 // ----- attention of single rows, any head sizes, fp32 arithmetic (attention_rows.cu) -----------

@@ -1,11 +1,12 @@
 // Allocation-free decode attention: see no_alloc.h for who needs it and for the contract.
 //
-// The split-KV decode kernel writes one partial (output row, log-sum-exp) per request, head
-// and split and a second kernel merges them.  The allocating op gets that buffer from the
+// The decode kernel writes partial results (output row, log-sum-exp) where a request's keys are dealt to
+// several CTAs, and a second kernel merges them.  The allocating op gets that buffer from the
 // framework's allocator; here it lives in a file-scope __device__ array.  In host code the
 // array's name is only a stand-in for the symbol - it is not a device address - so the
 // address is resolved once per device with cudaGetSymbolAddress and that pointer is what the
 // kernel receives.
+#include <algorithm>
 #include <cstdio>
 #include <mutex>
 
@@ -89,7 +90,7 @@ extern "C" int mllm_b200_attention_decode_noalloc(const void* q, const void* k_c
   a.kv_tok_stride = static_cast<int64_t>(hkv) * head_dim;   // the documented slot-major layout
   a.kv_head_stride = head_dim;
   a.out = out;
-  a.part_o = splits > 1 ? pd->scratch : nullptr;
+  a.part_o = pd->scratch;
   a.part_lse = splits > 1 ? pd->scratch + static_cast<size_t>(batch) * hq * splits * 128 : nullptr;
   a.req_to_token = req_to_token;
   a.req_pool_indices = req_pool_indices;
@@ -106,6 +107,9 @@ extern "C" int mllm_b200_attention_decode_noalloc(const void* q, const void* k_c
   a.head_dim = head_dim;
   a.max_q_len = 1;
   a.num_splits = splits;
+  if (mb200::decode_streams(head_dim, hq / hkv, 0))   // as many CTAs as the array has room for partial results
+    a.num_splits = static_cast<int>(std::min<int64_t>(mb200::decode_stream_ctas(head_dim, pd->num_sms),
+                                                      kScratchFloats / mb200::decode_stream_floats(head_dim, hq / hkv, 1)));
   a.is_decode = 1;
   a.scale = scale;
   a.dt = is_fp16 ? mb200::kF16 : mb200::kBF16;
