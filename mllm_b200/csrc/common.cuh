@@ -358,8 +358,18 @@ __device__ __forceinline__ uint32_t ld_acquire_cta_smem(const uint32_t* p) {
 // previous kernel in the stream is still draining; everything it does before pdl_wait() must
 // not touch global memory written by earlier kernels (barrier set-up, tensor-memory allocation,
 // descriptor prefetch are fine).  Both calls are no-ops for ordinary launches.
+//
+// A CTA that waits is on its SM while earlier kernels still read and write there, and the L1 cache may then hold lines that those
+// kernels fetched before the producer of this kernel's input wrote it (a buffer that changed in place, or memory that was handed
+// out again).  Ordinary loads are ordered by the wait; loads through the read-only path (__ldg, and what the compiler makes of
+// `const T* __restrict__`) are not.  pdl_wait() therefore drops what the L1 cache holds; pdl_wait_loads() does not, for kernels
+// that read their inputs by ordinary loads, cp.async.cg, __ldcg or TMA only.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait_loads() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() {
+  pdl_wait_loads();
+  asm volatile("fence.acq_rel.gpu;" ::: "memory");
+}
 __device__ __forceinline__ void pdl_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }

@@ -5,7 +5,9 @@
 // All of them move 16 bytes per thread per access and touch every byte once
 // (the norm kernels keep a row in registers between the reduction and the
 // scaling pass), so their ceiling is HBM bandwidth.
+#include <algorithm>
 #include <cstdlib>
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -95,7 +97,7 @@ template <typename T, bool kAdd>
 __global__ void rmsnorm_kernel(T* __restrict__ x, T* __restrict__ residual, const T* __restrict__ w,
                                T* __restrict__ out, int hidden, int64_t x_stride, int64_t out_stride, float eps) {
   pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait_loads();
   __shared__ float red[33];
   const int row = blockIdx.x;
   const int nvec = hidden >> 3;
@@ -111,10 +113,10 @@ __global__ void rmsnorm_kernel(T* __restrict__ x, T* __restrict__ residual, cons
     const int v = threadIdx.x + it * blockDim.x;
     if (v < nvec) {
       float f[8];
-      unpack8<T>(xr[v], f);
+      unpack8<T>(__ldcg(xr + v), f);
       if (kAdd) {
         float g[8];
-        unpack8<T>(rr[v], g);
+        unpack8<T>(__ldcg(rr + v), g);
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = round_to<T>(f[i] + g[i]);
         rr[v] = pack8<T>(f);
@@ -144,7 +146,7 @@ template <typename T>
 __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ w, const T* __restrict__ b,
                                  T* __restrict__ out, int hidden, float eps) {
   pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait_loads();
   __shared__ float red[33];
   const int row = blockIdx.x;
   const int nvec = hidden >> 3;
@@ -156,7 +158,7 @@ __global__ void layernorm_kernel(const T* __restrict__ x, const T* __restrict__ 
   for (int it = 0; it < kMaxVecPerThread; ++it) {
     const int v = threadIdx.x + it * blockDim.x;
     if (v < nvec) {
-      unpack8<T>(xr[v], cache[it]);
+      unpack8<T>(__ldcg(xr + v), cache[it]);
 #pragma unroll
       for (int i = 0; i < 8; ++i) s += cache[it][i];
     }
@@ -196,7 +198,7 @@ __device__ __forceinline__ float silu_f(float v) { return v / (1.f + __expf(-v))
 template <typename T, int kAct>
 __global__ void act_and_mul_kernel(const T* __restrict__ x, T* __restrict__ out, int rows, int inter, float limit) {
   pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait_loads();
   const int vec_per_row = inter >> 3;
   const int64_t total = static_cast<int64_t>(rows) * vec_per_row;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < total;
@@ -205,8 +207,8 @@ __global__ void act_and_mul_kernel(const T* __restrict__ x, T* __restrict__ out,
     const int v = static_cast<int>(i - r * vec_per_row);
     const uint4* row = reinterpret_cast<const uint4*>(x + r * 2 * inter);
     float g[8], u[8], o[8];
-    unpack8<T>(row[v], g);
-    unpack8<T>(row[vec_per_row + v], u);
+    unpack8<T>(__ldcg(row + v), g);
+    unpack8<T>(__ldcg(row + vec_per_row + v), u);
 #pragma unroll
     for (int j = 0; j < 8; ++j) o[j] = kAct == 2 ? clamped_gate(g[j], u[j], limit) : (kAct == 0 ? silu_f(g[j]) : gelu_tanh_f(g[j])) * u[j];
     reinterpret_cast<uint4*>(out + r * inter)[v] = pack8<T>(o);
@@ -314,11 +316,11 @@ __global__ void embedding_f32_kernel(const int64_t* __restrict__ ids, const T* _
 template <typename T>
 __global__ void gelu_tanh_kernel(const T* __restrict__ x, T* __restrict__ out, int64_t nvec) {
   pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait_loads();
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < nvec;
        i += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     float f[8];
-    unpack8<T>(reinterpret_cast<const uint4*>(x)[i], f);
+    unpack8<T>(__ldcg(reinterpret_cast<const uint4*>(x) + i), f);
 #pragma unroll
     for (int j = 0; j < 8; ++j) f[j] = gelu_tanh_f(f[j]);
     reinterpret_cast<uint4*>(out)[i] = pack8<T>(f);
@@ -345,14 +347,13 @@ __global__ void embedding_kernel(const int64_t* __restrict__ ids, const uint4* _
 
 // ---------------------------------------------------------------------------
 // fused per-head RMSNorm (q,k) + NeoX RoPE (q,k) + KV-cache write. head_dim = 128.
-// A warp owns one token and every `hsplit`-th head of it; lane l owns features 4l..4l+3, its rotation
-// partner (feature +-64) lives in lane l^16.  The sines and cosines depend on the token and the feature
-// only, so the warp computes its four pairs once and reuses them for all its heads (with one warp per
-// (token, head) the kernel was bound by sincosf: 355 us for 16384 tokens of 48 heads, against 60 us of
-// memory traffic).  The host picks hsplit = all heads for a handful of tokens (decode: parallelism
-// matters) and a few for long prefills.
+// A warp owns one token and every `hsplit`-th step of its heads: two heads of half a warp each (V = 8 features per lane), or one
+// head (V = 4); a feature's rotation partner (+-64) lives half a head's lanes away.  The sines and cosines depend on the token and
+// the feature only: the warp forms each of the 64 once, two per lane, and hands them round (with one warp per (token, head) the
+// kernel was bound by sincosf: 355 us for 16384 tokens of 48 heads; with four per lane and two warps per token, whose loads
+// waited for the stores before them, 172; now 115).
 // ---------------------------------------------------------------------------
-template <typename T>
+template <typename T, int V>
 __global__ void qk_norm_rope_kv_write_kernel(T* __restrict__ qkv, const T* __restrict__ q_w,
                                              const T* __restrict__ k_w, const int64_t* __restrict__ positions,
                                              int pos_rows, const int8_t* __restrict__ axis_map,
@@ -362,83 +363,89 @@ __global__ void qk_norm_rope_kv_write_kernel(T* __restrict__ qkv, const T* __res
                                              int64_t kv_head_stride, int tokens, int hq, int hkv, int hsplit,
                                              int64_t qkv_stride, int64_t num_slots, float eps, int* status) {
   pdl_launch_dependents();
-  pdl_wait();
-  constexpr int D = 128;
+  pdl_wait_loads();
+  constexpr int D = 128, kLanes = D / V, kHeads = 32 / kLanes;      // lanes of a head, heads of a warp's step
+  using Pack = typename std::conditional<V == 8, uint4, uint2>::type;
   const int heads = hq + 2 * hkv;
   const int64_t warp = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
   if (warp >= static_cast<int64_t>(tokens) * hsplit) return;
   const int t = static_cast<int>(warp / hsplit);
-  const int h_first = static_cast<int>(warp - static_cast<int64_t>(t) * hsplit);
-  const int lane = lane_id();
+  const int first = static_cast<int>(warp - static_cast<int64_t>(t) * hsplit);
+  const int lane = lane_id(), l = lane % kLanes;
+  const int step = hsplit * kHeads;
+  int h = first * kHeads + lane / kLanes;
 
-  const int64_t slot = cache_loc[t];
+  T* row = qkv + t * qkv_stride + l * V;
+  Pack next{};
+  if (h < heads) next = __ldcg(reinterpret_cast<const Pack*>(row + h * D));
+  const int64_t slot = __ldcg(cache_loc + t);
   const bool slot_ok = slot >= 0 && slot < num_slots;
-  if (!slot_ok && h_first == 0 && lane == 0 && status != nullptr) atomicExch(status, kStatusBadIndex);
+  if (!slot_ok && first == 0 && lane == 0 && status != nullptr) atomicExch(status, kStatusBadIndex);
 
-  float cs[4], sn[4];
-  if (h_first < hq + hkv) {   // this warp has at least one head to rotate
+  float cs[V], sn[V];
+  if (first * kHeads < hq + hkv) {   // this warp has at least one head to rotate
+    // every lane forms the sines and cosines of two of the 64 frequencies
+    float s2[2], c2[2];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int fi = (lane * 4 + i) & 63;
+    for (int i = 0; i < 2; ++i) {
+      const int fi = lane * 2 + i;
       const int ax = (axis_map != nullptr && pos_rows > 1) ? axis_map[fi] : 0;
-      const float ang = static_cast<float>(positions[static_cast<int64_t>(ax) * tokens + t]) * inv_freq[fi];
-      sincosf(ang, &sn[i], &cs[i]);
-      if (lane < 16) sn[i] = -sn[i];   // first half: x cos - partner sin; second half: x cos + partner sin
+      const float ang = static_cast<float>(__ldcg(positions + static_cast<int64_t>(ax) * tokens + t)) * inv_freq[fi];
+      sincosf(ang, &s2[i], &c2[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      const int from = ((l * V) & 63) / 2 + i / 2;
+      sn[i] = __shfl_sync(0xffffffffu, s2[i & 1], from);
+      cs[i] = __shfl_sync(0xffffffffu, c2[i & 1], from);
+      if (l < kLanes / 2) sn[i] = -sn[i];   // first half: x cos - partner sin; second half: x cos + partner sin
     }
   }
-  float wq[4], wk[4];
+  float wq[V], wk[V];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) wq[i] = wk[i] = 1.f;
-  if (q_w != nullptr) {
-    const uint2 wr = *reinterpret_cast<const uint2*>(q_w + lane * 4);
-    const T* we = reinterpret_cast<const T*>(&wr);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) wq[i] = to_f32(we[i]);
-  }
-  if (k_w != nullptr) {
-    const uint2 wr = *reinterpret_cast<const uint2*>(k_w + lane * 4);
-    const T* we = reinterpret_cast<const T*>(&wr);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) wk[i] = to_f32(we[i]);
+  for (int i = 0; i < V; ++i) {
+    wq[i] = q_w != nullptr ? to_f32(q_w[l * V + i]) : 1.f;
+    wk[i] = k_w != nullptr ? to_f32(k_w[l * V + i]) : 1.f;
   }
 
-  T* row = qkv + t * qkv_stride + lane * 4;
-#pragma unroll 4
-  for (int h = h_first; h < heads; h += hsplit) {
-    T* src = row + h * D;
-    uint2 raw = *reinterpret_cast<const uint2*>(src);
+  for (int h0 = first * kHeads; h0 < heads; h0 += step, h += step) {
+    Pack raw = next;
+    if (h + step < heads) next = __ldcg(reinterpret_cast<const Pack*>(row + (h + step) * D));
     const bool is_q = h < hq, is_k = !is_q && h < hq + hkv;
-    if (is_q || is_k) {
-      float f[4];
-      {
-        const T* e = reinterpret_cast<const T*>(&raw);
+    T* e = reinterpret_cast<T*>(&raw);
+    if (h0 < hq + hkv) {             // the warp has a head to rotate
+      float f[V], ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) f[i] = to_f32(e[i]);
+      for (int i = 0; i < V; ++i) {
+        f[i] = to_f32(e[i]);
+        ss += f[i] * f[i];
       }
+#pragma unroll
+      for (int o = kLanes / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
       if ((is_q ? q_w : k_w) != nullptr) {
-        const float ss = f[0] * f[0] + f[1] * f[1] + f[2] * f[2] + f[3] * f[3];
-        const float rstd = rsqrtf(warp_sum(ss) / static_cast<float>(D) + eps);
+        const float rstd = rsqrtf(ss / static_cast<float>(D) + eps);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) f[i] = round_to<T>(f[i] * rstd * (is_q ? wq[i] : wk[i]));
+        for (int i = 0; i < V; ++i) f[i] = round_to<T>(f[i] * rstd * (is_q ? wq[i] : wk[i]));
       }
-      T* e = reinterpret_cast<T*>(&raw);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float partner = __shfl_xor_sync(0xffffffffu, f[i], 16);
-        e[i] = from_f32<T>(f[i] * cs[i] + partner * sn[i]);
+      for (int i = 0; i < V; ++i) {
+        const float partner = __shfl_xor_sync(0xffffffffu, f[i], kLanes / 2);
+        if (is_q || is_k) e[i] = from_f32<T>(f[i] * cs[i] + partner * sn[i]);
       }
-      *reinterpret_cast<uint2*>(src) = raw;
+      if (is_q || is_k) *reinterpret_cast<Pack*>(row + h * D) = raw;
     }
-    if (!is_q && slot_ok) {
+    if (!is_q && h < heads && slot_ok) {
       void* cache = is_k ? k_cache : v_cache;
       const int kvh = is_k ? h - hq : h - hq - hkv;
-      const int64_t at = slot * kv_tok_stride + kvh * kv_head_stride + lane * 4;
+      const int64_t at = slot * kv_tok_stride + kvh * kv_head_stride + l * V;
       if (kv_fmt == kKvSame) {
-        *reinterpret_cast<uint2*>(static_cast<T*>(cache) + at) = raw;
+        *reinterpret_cast<Pack*>(static_cast<T*>(cache) + at) = raw;
       } else {   // 8-bit cache: the 16-bit values that attention would have read, rounded once more
-        const T* e = reinterpret_cast<const T*>(&raw);
-        const uint32_t packed = pack_fp8x2(to_f32(e[0]), to_f32(e[1]), kv_fmt) | (pack_fp8x2(to_f32(e[2]), to_f32(e[3]), kv_fmt) << 16);
-        *reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(cache) + at) = packed;
+#pragma unroll
+        for (int i = 0; i < V; i += 4) {
+          const uint32_t packed = pack_fp8x2(to_f32(e[i]), to_f32(e[i + 1]), kv_fmt) | (pack_fp8x2(to_f32(e[i + 2]), to_f32(e[i + 3]), kv_fmt) << 16);
+          *reinterpret_cast<uint32_t*>(static_cast<uint8_t*>(cache) + at + i) = packed;
+        }
       }
     }
   }
@@ -492,7 +499,7 @@ template <typename T>
 __global__ void per_token_quant_int8_kernel(const T* __restrict__ x, int8_t* __restrict__ q,
                                             float* __restrict__ scale, int k) {
   pdl_launch_dependents();
-  pdl_wait();
+  pdl_wait_loads();
   __shared__ float red[33];
   const int row = blockIdx.x;
   const int nvec = k >> 3;
@@ -503,7 +510,7 @@ __global__ void per_token_quant_int8_kernel(const T* __restrict__ x, int8_t* __r
   for (int it = 0; it < kMaxVecPerThread; ++it) {
     const int v = threadIdx.x + it * blockDim.x;
     if (v < nvec) {
-      unpack8<T>(xr[v], cache[it]);
+      unpack8<T>(__ldcg(xr + v), cache[it]);
 #pragma unroll
       for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(cache[it][i]));
     }
@@ -597,6 +604,12 @@ inline int norm_threads(int hidden) {
   if (t < 32) t = 32;
   return t;
 }
+// Threads of a CTA that holds a row: from 1024 rows on, enough to fill the GPU, up to four 16-byte vectors per thread instead of
+// one (more loads in flight per SM, fewer warps to meet at the barriers).
+inline int row_threads(int hidden, int rows) {
+  const int t = norm_threads(hidden);
+  return rows < 1024 ? t : std::min(t, std::max(64, ((hidden >> 3) + 127) / 128 * 32));
+}
 
 constexpr int kArgmaxChunks = 32;
 
@@ -677,7 +690,7 @@ __global__ void argmax_final_kernel(const float* __restrict__ part_val, const in
 void launch_rmsnorm(const void* x, const void* w, void* out, int rows, int hidden, int64_t x_stride,
                     int64_t out_stride, float eps, DType dt, cudaStream_t s) {
   if (rows == 0) return;
-  const int threads = norm_threads(hidden);
+  const int threads = row_threads(hidden, rows);
   MB200_DISPATCH_HALF(dt, (launch_pdl(rmsnorm_kernel<T, false>, dim3(rows), dim3(threads), 0, s, 
                               const_cast<T*>(static_cast<const T*>(x)), nullptr, static_cast<const T*>(w),
                               static_cast<T*>(out), hidden, x_stride, out_stride, eps)));
@@ -687,7 +700,7 @@ void launch_rmsnorm(const void* x, const void* w, void* out, int rows, int hidde
 void launch_fused_add_rmsnorm(void* x, void* residual, const void* w, int rows, int hidden, float eps, DType dt,
                               cudaStream_t s) {
   if (rows == 0) return;
-  const int threads = norm_threads(hidden);
+  const int threads = row_threads(hidden, rows);
   MB200_DISPATCH_HALF(dt, (launch_pdl(rmsnorm_kernel<T, true>, dim3(rows), dim3(threads), 0, s, 
                               static_cast<T*>(x), static_cast<T*>(residual), static_cast<const T*>(w),
                               static_cast<T*>(x), hidden, hidden, hidden, eps)));
@@ -697,7 +710,7 @@ void launch_fused_add_rmsnorm(void* x, void* residual, const void* w, int rows, 
 void launch_layernorm(const void* x, const void* w, const void* b, void* out, int rows, int hidden, float eps,
                       DType dt, cudaStream_t s) {
   if (rows == 0) return;
-  const int threads = norm_threads(hidden);
+  const int threads = row_threads(hidden, rows);
   MB200_DISPATCH_HALF(dt, (launch_pdl(layernorm_kernel<T>, dim3(rows), dim3(threads), 0, s, static_cast<const T*>(x),
                                                                          static_cast<const T*>(w),
                                                                          static_cast<const T*>(b),
@@ -826,18 +839,27 @@ void launch_qk_norm_rope_kv_write(void* qkv, const void* q_w, const void* k_w, c
                                   int num_q_heads, int num_kv_heads, int head_dim, int64_t qkv_stride,
                                   int64_t num_slots, float eps, DType dt, int kv_fmt, int* status, cudaStream_t s) {
   if (tokens == 0 || head_dim != 128) return;
-  // warps per token: every head its own warp for a few tokens, a handful of warps per token for long prefills
-  // (each then amortises its sines and cosines over heads / hsplit heads)
+  // A half warp per head, 16 bytes per lane, where rows and caches allow 16-byte accesses; a warp per head elsewhere.  Warps per
+  // token: every step its own warp for a few tokens, one warp for long prompts, which forms its sines and cosines once; they are
+  // most of the work of a warp with few heads.
   const int heads = num_q_heads + 2 * num_kv_heads;
-  const int hsplit = static_cast<int>(std::min<int64_t>(heads, std::max<int64_t>(1, 32768 / tokens)));
+  const uintptr_t ptrs = reinterpret_cast<uintptr_t>(qkv) | reinterpret_cast<uintptr_t>(k_cache) | reinterpret_cast<uintptr_t>(v_cache);
+  const bool wide = ptrs % 16 == 0 && qkv_stride % 8 == 0 && kv_tok_stride % 8 == 0 && kv_head_stride % 8 == 0;
+  const int steps = wide ? (heads + 1) / 2 : heads;
+  const int hsplit = static_cast<int>(std::min<int64_t>(steps, std::max<int64_t>(1, (wide ? 16384 : 32768) / tokens)));
   const int64_t warps = static_cast<int64_t>(tokens) * hsplit;
   const int threads = 128;
   const int blocks = static_cast<int>((warps * 32 + threads - 1) / threads);
-  MB200_DISPATCH_HALF(dt, (launch_pdl(qk_norm_rope_kv_write_kernel<T>, dim3(blocks), dim3(threads), 0, s, 
-                              static_cast<T*>(qkv), static_cast<const T*>(q_w), static_cast<const T*>(k_w),
-                              positions, pos_rows, axis_map, inv_freq, cache_loc, k_cache,
-                              v_cache, kv_fmt, kv_tok_stride, kv_head_stride, tokens, num_q_heads,
-                              num_kv_heads, hsplit, qkv_stride, num_slots, eps, status)));
+  auto go = [&](auto kernel, auto unit) {
+    using T = decltype(unit);
+    launch_pdl(kernel, dim3(blocks), dim3(threads), 0, s, static_cast<T*>(qkv), static_cast<const T*>(q_w), static_cast<const T*>(k_w),
+               positions, pos_rows, axis_map, inv_freq, cache_loc, k_cache, v_cache, kv_fmt, kv_tok_stride, kv_head_stride, tokens,
+               num_q_heads, num_kv_heads, hsplit, qkv_stride, num_slots, eps, status);
+  };
+  MB200_DISPATCH_HALF(dt, {
+    if (wide) go(qk_norm_rope_kv_write_kernel<T, 8>, T{});
+    else go(qk_norm_rope_kv_write_kernel<T, 4>, T{});
+  });
   note_launch();
 }
 
@@ -859,7 +881,7 @@ void launch_kv_write(const void* k, const void* v, const int64_t* loc, void* k_c
 void launch_per_token_quant_int8(const void* x, int8_t* q, float* scale, int rows, int k, DType dt,
                                  cudaStream_t s) {
   if (rows == 0) return;
-  const int threads = norm_threads(k);
+  const int threads = row_threads(k, rows);
   MB200_DISPATCH_HALF(dt, (launch_pdl(per_token_quant_int8_kernel<T>, dim3(rows), dim3(threads), 0, s, static_cast<const T*>(x), q,
                                                                                     scale, k)));
   note_launch();

@@ -27,11 +27,16 @@ __device__ __forceinline__ float silu(float v) {
   return v / (1.f + expf(-v));
 }
 
-// V neighbouring elements (V * sizeof(T) a power of two, aligned) as floats, and back
+// V neighbouring elements (V * sizeof(T) a power of two, aligned) as floats, and back.  The load is from the L2, so that a CTA
+// that was resident before its inputs were written sees them without a fence that empties the SM's L1.
 template <typename T, int V>
 __device__ __forceinline__ void load_v(const T* p, float (&f)[V]) {
   struct alignas(sizeof(T) * V) Pack { T e[V]; };
-  const Pack r = *reinterpret_cast<const Pack*>(p);
+  Pack r;
+  if constexpr (sizeof(Pack) == 16) *reinterpret_cast<uint4*>(&r) = __ldcg(reinterpret_cast<const uint4*>(p));
+  else if constexpr (sizeof(Pack) == 8) *reinterpret_cast<uint2*>(&r) = __ldcg(reinterpret_cast<const uint2*>(p));
+  else if constexpr (sizeof(Pack) == 4) *reinterpret_cast<uint32_t*>(&r) = __ldcg(reinterpret_cast<const uint32_t*>(p));
+  else *reinterpret_cast<uint16_t*>(&r) = __ldcg(reinterpret_cast<const uint16_t*>(p));
 #pragma unroll
   for (int i = 0; i < V; ++i) f[i] = to_f32(r.e[i]);
 }
@@ -53,18 +58,18 @@ __global__ void gdn_conv1d_silu_kernel(const T* __restrict__ x, int64_t x_ld, co
                                        const int* __restrict__ has_state, const int* __restrict__ q_start,
                                        T* __restrict__ out, int channels, int taps, int chunk_tokens, int own_state,
                                        const T* __restrict__ bias, int add_input) {
-  pdl_wait();
+  pdl_wait_loads();
   constexpr int kCap = KT > 0 ? KT : kMaxConvK;
   const int K = KT > 0 ? KT : taps;
   const int c = (blockIdx.x * blockDim.x + threadIdx.x) * V;
   const int b = blockIdx.z;
-  const int n = lens[b];
+  const int n = __ldcg(lens + b);
   const int t0 = blockIdx.y * chunk_tokens;
   if (c >= channels || t0 >= n) return;
   const int t1 = min(n, t0 + chunk_tokens);
-  const int64_t row0 = q_start[b];
-  T* st = conv_state + (static_cast<int64_t>(slots[b]) * channels + c) * (K - 1);
-  const bool hist = has_state[b] != 0;
+  const int64_t row0 = __ldcg(q_start + b);
+  T* st = conv_state + (static_cast<int64_t>(__ldcg(slots + b)) * channels + c) * (K - 1);
+  const bool hist = __ldcg(has_state + b) != 0;
   float wv[kCap][V], win[kCap][V], bv[V];
 #pragma unroll
   for (int i = 0; i < V; ++i) bv[i] = bias != nullptr ? to_f32(bias[c + i]) : 0.f;
@@ -78,27 +83,47 @@ __global__ void gdn_conv1d_silu_kernel(const T* __restrict__ x, int64_t x_ld, co
   for (int j = 0; j < kCap - 1; ++j) {
     if (j < K - 1) {
       const int t = t0 - (K - 1) + j;
+      if (t >= 0) {
+        load_v<T, V>(x + (row0 + t) * x_ld + c, win[j]);
+      } else {
 #pragma unroll
-      for (int i = 0; i < V; ++i)
-        win[j][i] = t >= 0 ? to_f32(x[(row0 + t) * x_ld + c + i]) : (hist ? to_f32(st[i * (K - 1) + K - 1 + t]) : 0.f);
+        for (int i = 0; i < V; ++i) win[j][i] = hist ? to_f32(st[i * (K - 1) + K - 1 + t]) : 0.f;
+      }
     }
   }
-#pragma unroll 4
-  for (int t = t0; t < t1; ++t) {
-    float cur[V], acc[V];
-    load_v<T, V>(x + (row0 + t) * x_ld + c, cur);
+  // eight tokens are in flight while eight are worked on: a thread's loads, not its arithmetic, set the rate
+  constexpr int kAhead = 8;
+  float nxt[kAhead][V];
+  auto fetch = [&](int t) {
 #pragma unroll
-    for (int i = 0; i < V; ++i) {
-      acc[i] = bv[i];
+    for (int u = 0; u < kAhead; ++u)
+      if (t + u < t1) load_v<T, V>(x + (row0 + t + u) * x_ld + c, nxt[u]);
+  };
+  fetch(t0);
+  for (int t = t0; t < t1; t += kAhead) {
+    float cur[kAhead][V];
 #pragma unroll
-      for (int j = 0; j < kCap; ++j)
-        if (j < K) acc[i] = fmaf(wv[j][i], j == K - 1 ? cur[i] : win[j][i], acc[i]);
-      acc[i] = add_input ? cur[i] + acc[i] : silu<T>(acc[i]);
+    for (int u = 0; u < kAhead; ++u)
 #pragma unroll
-      for (int j = 0; j < kCap - 1; ++j)
-        if (j < K - 1) win[j][i] = j == K - 2 ? cur[i] : win[j + 1][i];
+      for (int i = 0; i < V; ++i) cur[u][i] = nxt[u][i];
+    fetch(t + kAhead);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u) {
+      if (t + u >= t1) break;
+      float acc[V];
+#pragma unroll
+      for (int i = 0; i < V; ++i) {
+        acc[i] = bv[i];
+#pragma unroll
+        for (int j = 0; j < kCap; ++j)
+          if (j < K) acc[i] = fmaf(wv[j][i], j == K - 1 ? cur[u][i] : win[j][i], acc[i]);
+        acc[i] = add_input ? cur[u][i] + acc[i] : silu<T>(acc[i]);
+#pragma unroll
+        for (int j = 0; j < kCap - 1; ++j)
+          if (j < K - 1) win[j][i] = j == K - 2 ? cur[u][i] : win[j + 1][i];
+      }
+      store_v<T, V>(out + (row0 + t + u) * channels + c, acc);
     }
-    store_v<T, V>(out + (row0 + t) * channels + c, acc);
   }
   if (own_state) {
 #pragma unroll
@@ -318,24 +343,38 @@ __global__ void __launch_bounds__(256) gdn_recurrent_kernel(const GdnRuleParams 
 template <typename T, int V, bool SIG>
 __global__ void rmsnorm_gated_kernel(const T* __restrict__ x, const T* __restrict__ gate, int64_t gate_ld, const T* __restrict__ w,
                                      T* __restrict__ out, int64_t rows, int heads, int width, float eps, int round_norm) {
-  pdl_wait();
+  pdl_wait_loads();
   const int64_t r = blockIdx.x * static_cast<int64_t>(blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (r >= rows) return;
   const T* xr = x + r * width;
   const T* gr = gate + (r / heads) * gate_ld + (r % heads) * width;
+  // a lane's first V columns (all that it has, up to a width of 32 V) stay in registers, with their gate and weight: one trip
+  // to memory
   float ss = 0.f, f[V], g[V], wv[V];
-  for (int c = lane * V; c < width; c += 32 * V) {
-    load_v<T, V>(xr + c, f);
+  if (lane * V < width) {
+    load_v<T, V>(xr + lane * V, f);
+    load_v<T, V>(gr + lane * V, g);
+#pragma unroll
+    for (int i = 0; i < V; ++i) wv[i] = to_f32(w[lane * V + i]);
 #pragma unroll
     for (int i = 0; i < V; ++i) ss = fmaf(f[i], f[i], ss);
+  }
+  for (int c = (lane + 32) * V; c < width; c += 32 * V) {
+    float e[V];
+    load_v<T, V>(xr + c, e);
+#pragma unroll
+    for (int i = 0; i < V; ++i) ss = fmaf(e[i], e[i], ss);
   }
   ss = warp_sum(ss);
   const float rstd = 1.f / sqrtf(ss / static_cast<float>(width) + eps);
   for (int c = lane * V; c < width; c += 32 * V) {
-    load_v<T, V>(xr + c, f);
-    load_v<T, V>(gr + c, g);
-    load_v<T, V>(w + c, wv);
+    if (c >= 32 * V) {
+      load_v<T, V>(xr + c, f);
+      load_v<T, V>(gr + c, g);
+#pragma unroll
+      for (int i = 0; i < V; ++i) wv[i] = to_f32(w[c + i]);
+    }
 #pragma unroll
     for (int i = 0; i < V; ++i) {
       float nrm = f[i] * rstd;

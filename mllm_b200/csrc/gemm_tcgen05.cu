@@ -268,7 +268,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_con
   // weight stream then starts while the previous kernel is still draining.
   const bool early_weights = SWAP && p.row_static != 0;
   if (SWAP && p.early_trigger) pdl_launch_dependents();
-  if (!(early_weights && threadIdx.x == 0)) pdl_wait();
+  if (!(early_weights && threadIdx.x == 0)) pdl_wait_loads();
 
   const int total_tiles = p.tiles_r * p.tiles_c;
   // swap tiling: this CTA's contiguous range of the (tile, k-block) iteration space
@@ -352,7 +352,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_con
                           (kb * KD + kd) * k_elems_per_block, tr * kBM * C::R);
           }
         }
-        pdl_wait();
+        pdl_wait_loads();
       }
     }
     int seen = 0;   // iterations handled so far by the loop below
@@ -959,7 +959,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
   cluster_sync_all();   // both CTAs' barriers are initialised before either signals the other's
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_holder;
-  pdl_wait();
+  pdl_wait_loads();
 
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;

@@ -390,17 +390,31 @@ moe_align_kernel(const int* __restrict__ topk_ids, int pairs, int top_k, int exp
   }
 }
 
-// xs[pos, :] = x[src_token[pos], :] for the local pairs
+// xs[pos, :] = x[src_token[pos], :] for the local pairs.  A warp has a row, and eight of its loads are in flight before the first
+// store: 65536 rows of 4 KB take 57 us, and 80 with a block per row that
+// loads and stores in turn.
+constexpr int kGatherWarps = 4;
 template <typename V>
 __global__ void moe_gather_kernel(const V* __restrict__ x, int64_t x_stride_v, const int* __restrict__ src_token,
                                   const int* __restrict__ expert_offsets, int experts, V* __restrict__ xs,
-                                  int row_vecs) {
-  pdl_wait();
-  const int pos = blockIdx.x;
-  if (pos >= expert_offsets[experts]) return;
-  const V* src = x + static_cast<int64_t>(src_token[pos]) * x_stride_v;
+                                  int row_vecs, int pairs) {
+  pdl_wait_loads();
+  const int pos = blockIdx.x * kGatherWarps + (threadIdx.x >> 5), lane = threadIdx.x & 31;
+  if (pos >= pairs) return;
+  const int local = __ldcg(expert_offsets + experts), token = __ldcg(src_token + pos);
+  if (pos >= local) return;
+  const V* src = x + static_cast<int64_t>(token) * x_stride_v;
   V* dst = xs + static_cast<int64_t>(pos) * row_vecs;
-  for (int i = threadIdx.x; i < row_vecs; i += blockDim.x) dst[i] = __ldg(src + i);
+  constexpr int kAhead = 8;
+  for (int i = lane; i < row_vecs; i += 32 * kAhead) {
+    V r[kAhead];
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i + 32 * u < row_vecs) r[u] = __ldcg(src + i + 32 * u);
+#pragma unroll
+    for (int u = 0; u < kAhead; ++u)
+      if (i + 32 * u < row_vecs) dst[i + 32 * u] = r[u];
+  }
 }
 
 // the same with every row times the weight of its pair
@@ -427,15 +441,16 @@ __global__ void moe_gather_scaled_kernel(const T* __restrict__ x, int64_t x_stri
 template <typename T>
 __global__ void moe_combine_kernel(const T* __restrict__ y, const int* __restrict__ sorted_pos,
                                    const float* __restrict__ topk_w, T* __restrict__ out, int hidden, int top_k) {
-  pdl_wait();
+  pdl_wait_loads();
   const int t = blockIdx.x;
   for (int c = threadIdx.x * 8; c < hidden; c += blockDim.x * 8) {
     float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 4
     for (int j = 0; j < top_k; ++j) {
-      const int pos = sorted_pos[t * top_k + j];
+      const int pos = __ldcg(sorted_pos + t * top_k + j);
       if (pos < 0) continue;
-      const float w = topk_w[t * top_k + j];
-      const uint4 raw = *reinterpret_cast<const uint4*>(y + static_cast<int64_t>(pos) * hidden + c);
+      const float w = __ldcg(topk_w + t * top_k + j);
+      const uint4 raw = __ldcg(reinterpret_cast<const uint4*>(y + static_cast<int64_t>(pos) * hidden + c));
       const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
       for (int i = 0; i < 8; ++i) acc[i] += w * to_f32(e[i]);
@@ -790,8 +805,8 @@ void launch_moe_gather(const void* x, int64_t x_stride, const int* src_token, co
   auto go = [&](auto unit) {
     using V = decltype(unit);
     const int per = static_cast<int>(sizeof(V)) / elem_bytes;
-    launch_pdl(moe_gather_kernel<V>, dim3(pairs), dim3(128), 0, s, static_cast<const V*>(x), x_stride / per, src_token, expert_offsets,
-               experts, static_cast<V*>(xs), hidden / per);
+    launch_pdl(moe_gather_kernel<V>, dim3((pairs + kGatherWarps - 1) / kGatherWarps), dim3(32 * kGatherWarps), 0, s, static_cast<const V*>(x), x_stride / per, src_token, expert_offsets,
+               experts, static_cast<V*>(xs), hidden / per, pairs);
   };
   const uintptr_t ptrs = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(xs);
   if (ptrs % 16 == 0 && (hidden * elem_bytes) % 16 == 0 && (x_stride * elem_bytes) % 16 == 0) go(uint4{});
