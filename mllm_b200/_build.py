@@ -51,7 +51,7 @@ EXTENSIONS: Dict[str, Dict[str, List[str]]] = {
     "mllm_b200_C": {
         "sources": ["bindings.cpp", "runtime.cu", "elementwise.cu", "row_ops.cu", "depth.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "attention.cu",
                     "attention_decode.cu", "attention_rows.cu", "sampling.cu", "no_alloc.cu"],
-        "headers": _COMMON + ["no_alloc.h"],
+        "headers": _COMMON + ["gemm_stream.cuh", "no_alloc.h"],
         "cuda": True,
     },
     "mllm_b200_R": {
@@ -76,7 +76,7 @@ EXTENSIONS: Dict[str, Dict[str, List[str]]] = {
     },
     "mllm_b200_X": {
         "sources": ["bindings_extra.cpp", "runtime.cu", "comm.cu", "ep_a2a.cu", "gemm_w4a16.cu", "gemm_smallm_w4.cu", "vision.cu"],
-        "headers": _COMMON,
+        "headers": _COMMON + ["gemm_stream.cuh"],
         "cuda": True,
     },
     "mllm_b200_host": {

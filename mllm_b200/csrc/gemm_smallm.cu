@@ -1,37 +1,21 @@
-// out[m, n] = a[m, k] * b[n, k]^T for a handful of rows (m <= 8): the decode step of a small batch.
+// out[m, n] = a[m, k] * b[n, k]^T for a handful of rows (m <= 8), 16-bit operands: the projections of a decode step.  The kernel
+// is the weight stream of gemm_stream.cuh.  A second kernel takes the fused add + RMSNorm prologue (opt-in: ops.add_rmsnorm_linear):
+//   * a unit of work is 8 weight rows over the whole k range; a CTA (one per SM) owns a contiguous run of units, its 16 warps take
+//     the 32-element k steps of a unit round-robin;
+//   * weight loads run 16 steps ahead as cp.async copies into a slice of shared memory that belongs to the lane alone;
+//   * the batch's rows are normalised by every CTA for itself while its weight copies are in flight, and stay in shared memory
+//     (rows 64 bytes apart modulo 128: no bank conflicts), hence k <= 4096;
+//   * at the end of a unit the warps' 8 x 8 partial sums meet in shared memory.
 //
-// With eight activation rows the product is a stream of the weight matrix through the SMs; the arithmetic
-// is negligible and the cost of the tcgen05 path (tensor-memory allocation, a TMA ring to fill, a tile of
-// 128 weight rows per CTA and therefore a split of k with partial sums exchanged between CTAs) is a fixed
-// 6-8 us per launch, as much again as the streaming time of a 4096 x 4096 projection.  This kernel keeps
-// nothing but registers between the load and the sum:
-//   * a unit of work is 8 weight rows over the whole k range; a CTA (one per SM) owns a contiguous run of
-//     units, its 16 warps take the 32-element k steps of a unit round-robin, so the warps of a CTA read 1 KB
-//     of each of the 8 rows per round;
-//   * a lane loads 16 bytes of one weight row and the 16 bytes of one activation row at the same k offset
-//     and feeds them to two warp-level MMAs (m16n8k16: activations in the upper 8 rows of A, lower rows zero;
-//     the 8 weight rows are B's columns).  The k positions inside an MMA are permuted the same way for both
-//     operands, which a dot product does not notice, so no shuffling is needed to build fragments;
-//   * weight loads run 16 steps ahead and cross unit boundaries.  They are cp.async copies into a slice of
-//     shared memory that belongs to the lane alone: the lane later reads back exactly the 16 bytes it asked
-//     for, so shared memory is only a deep queue behind the register file (128 KB in flight per SM; a
-//     register ring of 8 steps reached 4.1 TB/s on a 1.2 GB matrix, the tcgen05 path's TMA ring 6.5) and
-//     needs no barrier, just cp.async.wait_group.  Weights are requested before the stream-order wait when
-//     they are model parameters (nothing in the stream writes them);
-//   * the batch's 8 rows are copied to shared memory once per CTA (read through L1 they missed: the ring
-//     leaves L1 too small, and every step then paid an L2 round trip), rows 64 bytes apart modulo 128 so
-//     that a warp's read of 8 rows x 64 bytes has no bank conflict; hence k <= 4096.  (Walking a longer k in
-//     pieces, with the activations of a piece staged at a time, was tried and was slower than the tcgen05
-//     path: 32-43 us against 23 us for a 4096 x 12288 projection; so was a cluster of four CTAs sharing the k range
-//     with one exchange of partial sums at the end: 37 clusters of four 200 KB CTAs do not fit one wave, 42.6 us.)
-//   * at the end of a unit the warps' 8 x 8 partial sums meet in shared memory (double-buffered, one
-//     __syncthreads per unit) and 64 threads add bias / residual or apply SwiGLU and store.
+// Measured (B200, weights from HBM, inside the decode step of an 8B model, 8 rows; the kernel above before the stream took over):
+//   4096 x 12288: 31.9 us (on the tcgen05 path) -> 18.0; 6144, 4096 and 24576 x 4096 together: 63.8 us -> 52.3.
 #include <algorithm>
 #include <cstdint>
 
 #include <type_traits>
 
 #include "common.cuh"
+#include "gemm_stream.cuh"
 #include "kernels.h"
 
 namespace mb200 {
@@ -58,8 +42,7 @@ struct SmallMParams {
   int swiglu;
   float act_limit;
   int b_static;
-  int early_trigger;     // let the kernels behind this one start their set-up as soon as this one runs
-  // fused prologue (norm_w != null): the rows fed to the product are rmsnorm(a + norm_res) * norm_w, with the sum
+  // prologue: the rows fed to the product are rmsnorm(a + norm_res) * norm_w, with the sum
   // rounded to 16 bits first (it is the new residual stream, which CTA 0 also writes to norm_res_out)
   const void* norm_w;
   const uint8_t* norm_res;     // may be null: the rows of `a` are the residual stream already
@@ -107,7 +90,6 @@ __global__ void __launch_bounds__(kSmThreads, 1) gemm_smallm_kernel(const SmallM
   extern __shared__ __align__(16) uint8_t smem_dyn[];
   uint8_t* ring_raw = smem_dyn;
   uint8_t* x_rows = smem_dyn + kSmRingBytes;     // 8 rows of 2 k + kSmRowPad bytes
-  if (p.early_trigger) pdl_launch_dependents();
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const int g = lane >> 2;   // weight row inside the unit, and activation row
@@ -156,17 +138,8 @@ __global__ void __launch_bounds__(kSmThreads, 1) gemm_smallm_kernel(const SmallM
     commit();   // one group per step, empty past the end, so that "all but the newest 15" means step i
   }
   if (p.b_static) pdl_wait();
-  // the batch's rows into shared memory (rows past m are zero); every warp reads all of them again and again
   const int vec_per_row = p.k >> 3;
-  if (p.norm_w == nullptr) {
-    for (int v = threadIdx.x; v < 8 * vec_per_row; v += kSmThreads) {
-      const int r = v / vec_per_row, q = v - r * vec_per_row;
-      uint4 val = make_uint4(0, 0, 0, 0);
-      if (r < p.m) val = __ldg(reinterpret_cast<const uint4*>(p.a + static_cast<int64_t>(r) * p.lda_bytes) + q);
-      *reinterpret_cast<uint4*>(x_rows + r * x_pitch + q * 16) = val;
-    }
-    __syncthreads();
-  } else {
+  {
     // Fused add + RMSNorm: every CTA normalises the same 8 rows for itself (a few tens of KB from L2, while
     // its weight copies are already in flight); CTA 0 also stores the new residual stream.
     float ss[8];
@@ -321,6 +294,36 @@ __global__ void __launch_bounds__(kSmThreads, 1) gemm_smallm_kernel(const SmallM
   }
 }
 
+template <bool F16>
+int launch_stream(const GemmArgs& a, cudaStream_t s) {
+  stream::Params p{};
+  p.x = static_cast<const uint8_t*>(a.a);
+  p.w = static_cast<const uint8_t*>(a.b);
+  p.bias = a.bias;
+  p.residual = a.residual;
+  p.out = a.out;
+  p.m = a.m;
+  p.n = a.n;
+  p.steps = a.k / 32;
+  p.units = (a.n + 15) / 16;
+  p.up_rows = p.gate_block = 128;
+  p.w_static = a.b_static;
+  p.act_limit = a.act_limit;
+  p.ldx = a.lda * 2;
+  p.ldw = a.ldb * 2;
+  p.ldc = a.ldc;
+  p.ld_res = a.ld_res;
+  const int sms = std::max(1, a.num_sms);
+  switch (a.swiglu) {
+    case 0: return stream::launch<F16, stream::kHalf, stream::kNone>(p, sms, s);
+    case 1: return stream::launch<F16, stream::kHalf, stream::kSilu>(p, sms, s);
+    case 2: return stream::launch<F16, stream::kHalf, stream::kGelu>(p, sms, s);
+    case 3: return stream::launch<F16, stream::kHalf, stream::kRelu2>(p, sms, s);
+    case 4: return stream::launch<F16, stream::kHalf, stream::kClamped>(p, sms, s);
+  }
+  return 1;
+}
+
 }  // namespace
 
 // Returns 0 when launched, 1 when the shape is not for this kernel (the caller goes on to the tcgen05 path).
@@ -330,15 +333,16 @@ int launch_gemm_smallm(const GemmArgs& a, cudaStream_t s) {
     return e == nullptr ? 1 : std::atoi(e);
   }();
   if (!knob || a.m > 8 || a.is_int8 || a.gate_flags != nullptr || a.rs_tp > 0) return 1;
-  if (a.k % (32 * kSmWarps) != 0 || a.k > kSmMaxK || a.n % 8 != 0) return 1;
+  if (a.k % 32 != 0 || a.n % 8 != 0) return 1;
   // matrices of hundreds of MB (the vocabulary head) stream at the full copy rate through the TMA ring of the
   // tcgen05 path, whose set-up cost no longer shows; this kernel is for the projections of a layer
   if (static_cast<int64_t>(a.n) * a.k * 2 > (int64_t(384) << 20)) return 1;
   const bool relu2 = a.swiglu == 3, clamped = a.swiglu == 4;
   if (a.swiglu && !relu2 && (a.n % 256 != 0 || (a.bias != nullptr && !clamped) || a.residual != nullptr)) return 1;
   if ((a.lda * 2) % 16 != 0 || (a.ldb * 2) % 16 != 0) return 1;
-  if (a.norm_weight != nullptr &&
-      ((a.norm_residual_ld * 2) % 16 != 0 || (a.norm_residual_out_ld * 2) % 16 != 0 ||
+  if (a.norm_weight == nullptr) return a.dt == kF16 ? launch_stream<true>(a, s) : launch_stream<false>(a, s);
+  if (a.k % (32 * kSmWarps) != 0 || a.k > kSmMaxK) return 1;
+  if (((a.norm_residual_ld * 2) % 16 != 0 || (a.norm_residual_out_ld * 2) % 16 != 0 ||
        ((reinterpret_cast<uintptr_t>(a.norm_weight) | reinterpret_cast<uintptr_t>(a.norm_residual) |
          reinterpret_cast<uintptr_t>(a.norm_residual_out)) & 15) != 0 ||
        (a.norm_residual != nullptr && a.norm_residual == a.norm_residual_out)))
@@ -367,12 +371,6 @@ int launch_gemm_smallm(const GemmArgs& a, cudaStream_t s) {
   p.norm_res_ld_bytes = a.norm_residual_ld * 2;
   p.norm_res_out_ld_bytes = a.norm_residual_out_ld * 2;
   p.norm_eps = a.norm_eps;
-  static const int trigger_knob = [] {
-    // measured on the decode step of an 8B model: 5.22 ms per step with the trigger at the start, 4.95 ms without
-    const char* e = std::getenv("MLLM_B200_GEMM_SMALLM_TRIGGER");
-    return e == nullptr ? 0 : std::atoi(e);
-  }();
-  p.early_trigger = trigger_knob;
   // one CTA per SM, every CTA the same number of units (the stream is bound by memory, not by the number of SMs
   // that pull on it, as long as enough loads are in flight)
   const int slots = std::max(1, a.num_sms);

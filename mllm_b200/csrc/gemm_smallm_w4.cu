@@ -22,6 +22,7 @@
 #include <cstdlib>
 
 #include "common.cuh"
+#include "gemm_stream.cuh"
 #include "kernels.h"
 
 namespace mb200 {
@@ -273,6 +274,33 @@ int launch_w4_cfg(W4SmallParams p, const W4A16Args& a, cudaStream_t s) {
   return err == cudaSuccess ? 0 : -4;
 }
 
+template <bool F16>
+int launch_stream(const W4A16Args& a, cudaStream_t s) {
+  stream::Params p{};
+  p.x = static_cast<const uint8_t*>(a.x);
+  p.w = static_cast<const uint8_t*>(a.qweight);
+  p.scales = static_cast<const uint8_t*>(a.scales);
+  p.zeros = a.zeros;
+  p.bias = a.bias;
+  p.out = a.out;
+  p.m = a.m;
+  p.n = a.n;
+  p.steps = a.k / 128;
+  p.groups = a.k / a.group;
+  p.steps_per_group = a.group / 128;
+  p.units = (a.n + 15) / 16;
+  p.w_static = 1;
+  p.ldx = a.ldx * 2;
+  p.ldw = a.k / 2;
+  p.ldc = a.ldc;
+  const int sms = a.num_sms > 0 ? a.num_sms : 148;
+  if (a.zeros != nullptr)
+    return a.interleaved ? stream::launch<F16, stream::kInt4Zeros, stream::kNone>(p, sms, s)
+                         : stream::launch<F16, stream::kInt4NaturalZeros, stream::kNone>(p, sms, s);
+  return a.interleaved ? stream::launch<F16, stream::kInt4, stream::kNone>(p, sms, s)
+                       : stream::launch<F16, stream::kInt4Natural, stream::kNone>(p, sms, s);
+}
+
 }  // namespace
 
 // Returns 0 when launched, 1 when the shape is not for this kernel (the caller goes on to the tcgen05 kernel).
@@ -282,6 +310,11 @@ int launch_w4a16_smallm(const W4A16Args& a, cudaStream_t s) {
     return e == nullptr ? 1 : std::atoi(e);
   }();
   if (!knob || a.m > 8 || a.n % 8 != 0) return 1;
+  if (a.group % 128 == 0 && a.k % a.group == 0 && a.k % 128 == 0 && (a.ldx * 2) % 16 == 0 && (reinterpret_cast<uintptr_t>(a.scales) & 1) == 0 &&
+      ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.qweight)) & 15) == 0) {
+    const int rc = a.dt == kF16 ? launch_stream<true>(a, s) : launch_stream<false>(a, s);
+    if (rc <= 0) return rc;
+  }
   const bool small_k = a.k <= QSmall::kMaxK && a.k % (128 * QSmall::kWarps) == 0;
   const bool long_k = a.k <= QLong::kMaxK && a.k % (128 * QLong::kWarps) == 0;
   if ((!small_k && !long_k) || a.group % 32 != 0 || a.k % a.group != 0) return 1;

@@ -1,0 +1,76 @@
+"""Products that fit one wave of thread blocks: the weight stream for up to 8 rows (16-bit and 4-bit weights) and the small tiles with
+their k range over a cluster, at the edges of their units, steps, tiles and splits."""
+
+import pytest
+import torch
+
+from mllm_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+# the result is rounded to 8 bits (bf16), by at most 2^-9 of itself
+TOLERANCE = 2 ** -8
+
+
+def _rand(*shape, seed=0, std=1.0, dtype=torch.bfloat16):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    return (torch.randn(shape, generator=g, device="cuda") * std).to(dtype)
+
+
+def _close(got, want):
+    error = (got.double() - want).norm() / want.norm()
+    assert error < TOLERANCE, float(error)
+    assert torch.isfinite(got.float()).all()
+
+
+# n: part of a unit of 16 rows, several units per block; k: less than the eight warps' steps, a last step that some warps lack,
+# registers' limit (4096), two and eight blocks of a cluster
+@pytest.mark.parametrize("n,k", [(8, 32), (24, 96), (1000, 544), (4096, 4096), (520, 4128), (264, 12288), (40, 32768), (9472, 512)])
+@pytest.mark.parametrize("m", [1, 3, 8])
+def test_stream(m, n, k):
+    x, w = _rand(m, k), torch.nn.Parameter(_rand(n, k, seed=1, std=0.05), requires_grad=False)
+    _close(ops.linear(x, w), x.double() @ w.double().t())
+    b, r = _rand(n, seed=2), _rand(m, n, seed=3)
+    _close(ops.linear(x, w, b, r), x.double() @ w.double().t() + b.double() + r.double())
+
+
+# 9 rows and more: every width of a tile, part of a tile in each direction, every split of k, a k that is no multiple of 64
+@pytest.mark.parametrize("n,k", [(8, 64), (136, 520), (1024, 2048), (1000, 544), (4096, 4096), (384, 8192)])
+@pytest.mark.parametrize("m", [9, 16, 17, 33, 65, 129, 256, 300, 784])
+def test_tiles(m, n, k):
+    x, w = _rand(m, k), torch.nn.Parameter(_rand(n, k, seed=1, std=0.05), requires_grad=False)
+    _close(ops.linear(x, w), x.double() @ w.double().t())
+    b, r = _rand(n, seed=2), _rand(m, n, seed=3)
+    _close(ops.linear(x, w, b, r), x.double() @ w.double().t() + b.double() + r.double())
+
+
+@pytest.mark.parametrize("n,k", [(256, 64), (2048, 1024), (512, 4160), (768, 12288)])
+@pytest.mark.parametrize("m", [1, 8, 20, 100, 300])
+def test_gated(m, n, k):
+    x, w = _rand(m, k), torch.nn.Parameter(_rand(n, k, seed=1, std=0.05), requires_grad=False)
+    y = (x.double() @ w.double().t()).view(m, -1, 2, ops.SWIGLU_BLOCK)
+    _close(ops.linear_swiglu(x, w), (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(m, -1))
+
+
+@pytest.mark.parametrize("m", [9, 40, 200, 400])
+def test_tiles_int8(m):
+    n, k = 328, 1056
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a, w = (torch.randint(-127, 128, (r, k), generator=g, device="cuda", dtype=torch.int8) for r in (m, n))
+    sa, sw = (torch.rand((r,), generator=g, device="cuda") * 0.01 + 0.001 for r in (m, n))
+    _close(ops.int8_scaled_mm(a, w, sa, sw, torch.bfloat16), (a.double() @ w.double().t()) * sa.double()[:, None] * sw.double())
+
+
+@pytest.mark.parametrize("n,k,group", [(8, 128, 128), (1000, 1280, 128), (4096, 4096, 128), (264, 12288, 256), (40, 2048, 2048), (136, 2048, 64)])
+@pytest.mark.parametrize("m", [1, 5, 8])
+@pytest.mark.parametrize("zeros,interleaved", [(False, True), (True, True), (True, False), (False, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_stream_4bit(m, n, k, group, zeros, interleaved, dtype):
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    words = torch.randint(-2 ** 31, 2 ** 31, (n, k // 8), generator=g, device="cuda", dtype=torch.int32)
+    scale = (torch.rand((n, k // group), generator=g, device="cuda") * 0.01 + 0.005).to(dtype)
+    z = torch.randint(0, 16, (n, k // group), generator=g, device="cuda", dtype=torch.uint8) if zeros else None
+    x = _rand(m, k, dtype=dtype)
+    codes = ((words.unsqueeze(-1) >> torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)) & 15).flatten(1).double().view(n, -1, group)
+    w = ((codes - (8 if z is None else z.double().unsqueeze(-1))) * scale.double().unsqueeze(-1)).flatten(1)
+    _close(ops.w4a16_gemm(x, ops.w4a16_interleave(words) if interleaved else words, scale, z, group, None, interleaved=interleaved), x.double() @ w.t())
