@@ -1432,6 +1432,11 @@ int launch_gemm(const GemmArgs& a, cudaStream_t s) {
       return gated ? launch_pair_cfg<1>(tm_row, tm_col, p, pairs, s)
                       : launch_pair_cfg<0>(tm_row, tm_col, p, pairs, s);
     }
+    // ---- too few of those: one wave of small tiles ----
+    {
+      const int rc = launch_gemm_tile(a, s);
+      if (rc <= 0) return rc;
+    }
     // ---- normal tiling: activations are the 128-row operand ----
     int bn = 256;
     if (!gated) {
@@ -1459,7 +1464,11 @@ int launch_gemm(const GemmArgs& a, cudaStream_t s) {
     const int rc = launch_gemm_smallm(a, s);
     if (rc <= 0) return rc;
   }
-  if (relu2) return 1;                       // 9 to 256 rows: the caller applies the activation itself
+  {
+    const int rc = launch_gemm_tile(a, s);
+    if (rc <= 0) return rc;
+  }
+  if (relu2) return 1;                       // more tiles than one wave: the caller applies the activation itself
   if (a.norm_weight != nullptr) return -1;   // the fused norm prologue exists in that kernel only
 
   // ---- swap tiling: weights are the 128-row operand, the batch is MMA N ----
