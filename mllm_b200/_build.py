@@ -55,7 +55,7 @@ EXTENSIONS: Dict[str, Dict[str, List[str]]] = {
         "cuda": True,
     },
     "mllm_b200_R": {
-        "sources": ["bindings_recurrent.cpp", "runtime.cu", "gdn.cu", "gdn_chunk.cu", "gdn_channel.cu"],
+        "sources": ["bindings_recurrent.cpp", "runtime.cu", "gdn.cu", "gdn_chunk.cu", "gdn_prefill.cu", "gdn_channel.cu"],
         "headers": _COMMON,
         "cuda": True,
     },

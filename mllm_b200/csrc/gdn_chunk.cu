@@ -1,4 +1,6 @@
-// Chunk-parallel prefill of the gated delta rule (the hybrid models' linear attention), 64 tokens at a time.
+// Chunk-parallel prefill of the gated delta rule (the hybrid models' linear attention), 64 tokens at a time, for fp16 inputs and
+// for recurrences whose fp32 operands are carried as two tf32 terms (21 bits); bf16 inputs otherwise take gdn_prefill.cu, whose
+// two bf16 terms hold 16 bits and whose remainders would underflow in fp16.
 //
 // The token recurrence  S *= exp(g_t);  S += k_t (x) ((v_t - S^T k_t) beta_t);  o_t = S^T q_t  is evaluated per
 // chunk with matrix products.  With G_i the running sum of g inside the chunk and S0 the incoming state:
@@ -22,6 +24,8 @@
 // The 64 x 64 x BV tiles and the chunk-to-chunk dependency are too small and too serial for a tcgen05 pipeline
 // (tensor-memory round trips between the six dependent products would dominate), hence the warp-level path.
 #include <mma.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 #include "kernels.h"
@@ -402,7 +406,8 @@ int launch_chunk_cfg(const GdnRuleParams& p, cudaStream_t s) {
 template <typename T>
 int launch_chunk_t(const GdnRuleParams& p, bool narrow, cudaStream_t s) {
   if (p.split_tf32) return narrow ? launch_chunk_cfg<T, 32, true>(p, s) : launch_chunk_cfg<T, 64, true>(p, s);
-  return narrow ? launch_chunk_cfg<T, 32, false>(p, s) : launch_chunk_cfg<T, 64, false>(p, s);
+  if constexpr (std::is_same<T, __half>::value) return narrow ? launch_chunk_cfg<T, 32, false>(p, s) : launch_chunk_cfg<T, 64, false>(p, s);
+  return -1;      // bf16 without the split: gdn_prefill.cu
 }
 
 }  // namespace

@@ -1122,12 +1122,12 @@ def _heads_like(t: torch.Tensor, heads: int) -> torch.Tensor:
 
 
 def gated_delta_rule(q, k, v, g, beta, state, state_indices, seq_lens, has_state, q_start=None, raw_gates=None,
-                     split_tf32: bool = False) -> torch.Tensor:
+                     split_tf32: bool = False, max_len: int = 0) -> torch.Tensor:
     """Gated delta rule over ragged sequences with per-request recurrent state (read when ``has_state``,
     always written back).  q, k [T, Hk, Dk] (Hk divides H: value head h uses head ``h // (H / Hk)``), v [T, H, Dv],
     g / beta [T, H] fp32; ``raw_gates = (b, a, a_log, dt_bias)`` instead of g and beta lets the kernel form them.
     Tokens may be rows of wider matrices (heads of a token contiguous).  ``split_tf32``: the chunk-parallel kernel
-    carries its fp32 operands as two tf32 terms instead of one."""
+    carries its fp32 operands as two tf32 terms.  ``max_len``: the longest run of new tokens, when the host knows it."""
     H = v.shape[1]
     if use_kernels(q) and q.shape[-1] <= _GDN_MAX_DK and _GDN_EXTEND_BACKEND != "pytorch":
         dev = q.device
@@ -1145,7 +1145,7 @@ def gated_delta_rule(q, k, v, g, beta, state, state_indices, seq_lens, has_state
                 g, beta = gdn_gates(*raw_gates)
                 raw_gates = None
             g, beta = g.float().contiguous(), beta.float().contiguous()
-            if ext().gdn_chunk(q, k, v, g, beta, *meta, split_tf32) == 0:
+            if ext().gdn_chunk(q, k, v, g, beta, *meta, split_tf32, int(max_len)) == 0:
                 return out
         if raw_gates is not None:
             ext().gdn_recurrent_raw(q, k, v, *raw_gates, *meta)

@@ -1,0 +1,72 @@
+"""Prefill of the gated delta rule in two kernels: chunks of 64 tokens at their edges, head sizes that are padded, several value
+blocks, decays from almost none to almost all, spans of a bounded workspace."""
+
+import pytest
+import torch
+
+from mllm_b200 import ops
+
+pytestmark = pytest.mark.gpu
+
+
+def _rule(q, k, v, g, beta, state, lens, has):
+    q, k, v = q.double(), k.double(), v.double()
+    rep = v.shape[1] // q.shape[1]
+    q, k = (t * torch.rsqrt(t.square().sum(-1, keepdim=True) + 1e-6) for t in (q, k))
+    q, k = q.repeat_interleave(rep, 1) * q.shape[-1] ** -0.5, k.repeat_interleave(rep, 1)
+    out, states, at = [], [], 0
+    for b, n in enumerate(lens):
+        s = state[b].double() * (1 if has[b] else 0)
+        for t in range(at, at + n):
+            s = s * g[t].double().exp()[:, None, None]
+            u = (v[t] - torch.einsum("hkv,hk->hv", s, k[t])) * beta[t].double()[:, None]
+            s = s + k[t].unsqueeze(-1) * u.unsqueeze(-2)
+            out.append(torch.einsum("hkv,hk->hv", s, q[t]))
+        at += n
+        states.append(s)
+    return torch.stack(out), torch.stack(states)
+
+
+def _check(lens, heads, key_heads, dk, dv, decay=0.1, max_len=None):
+    gen = torch.Generator(device="cuda").manual_seed(sum(lens) + heads)
+    T = sum(lens)
+    q, k = (torch.randn((T, key_heads, dk), generator=gen, device="cuda").bfloat16() for _ in range(2))
+    v = torch.randn((T, heads, dv), generator=gen, device="cuda").bfloat16()
+    g = -torch.rand((T, heads), generator=gen, device="cuda") * decay
+    beta = torch.rand((T, heads), generator=gen, device="cuda")
+    state = torch.randn((len(lens) + 1, heads, dk, dv), generator=gen, device="cuda") * 0.1
+    has = [i % 2 for i in range(len(lens))]
+    want, after = _rule(q, k, v, g, beta, state, lens, has)
+    spare = state[len(lens)].clone()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    ops.set_gdn_extend_backend("cuda_chunkwise")
+    try:
+        got = ops.gated_delta_rule(q, k, v, g, beta, state, torch.arange(len(lens), **i32), torch.tensor(lens, **i32), torch.tensor(has, **i32),
+                                   max_len=max(lens) if max_len is None else max_len)
+    finally:
+        ops.set_gdn_extend_backend("auto")
+    ops.check_status()
+    # outputs are rounded to 8 bits; the state is fp32, and the operands of its products hold 16 bits
+    assert (got.double() - want).norm() / want.norm() < 2 ** -8
+    assert (state[:len(lens)].double() - after).norm() / after.norm() < 2 ** -14
+    assert torch.equal(state[len(lens)], spare)
+
+
+@pytest.mark.parametrize("lens", [[1], [63], [64], [65], [128, 1, 129], [300, 7, 64, 2]], ids=str)
+def test_chunks(lens):
+    _check(lens, 4, 4, 128, 128)
+
+
+@pytest.mark.parametrize("heads,key_heads,dk,dv", [(4, 2, 128, 128), (2, 2, 64, 96), (2, 1, 40, 24), (2, 2, 128, 256), (80, 80, 128, 128), (6, 2, 8, 8)])
+def test_heads(heads, key_heads, dk, dv):
+    _check([100, 33], heads, key_heads, dk, dv)
+
+
+@pytest.mark.parametrize("decay", [0.0, 1e-3, 5.0, 60.0])
+def test_decays(decay):
+    _check([200], 2, 2, 128, 128, decay=decay)
+
+
+def test_spans_of_the_workspace():
+    """Enough heads that the 512 MB of the workspace hold two chunks at a time."""
+    _check([330, 129], 1700, 100, 8, 128, max_len=0)
