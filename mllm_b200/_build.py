@@ -49,7 +49,7 @@ _COMMON = ["bindings_common.h", "common.cuh", "kernels.h", "mma.cuh", "row.cuh"]
 
 EXTENSIONS: Dict[str, Dict[str, List[str]]] = {
     "mllm_b200_C": {
-        "sources": ["bindings.cpp", "runtime.cu", "elementwise.cu", "row_ops.cu", "depth.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "gemm_tile.cu", "attention.cu",
+        "sources": ["bindings.cpp", "runtime.cu", "elementwise.cu", "row_ops.cu", "depth.cu", "gemm_tcgen05.cu", "gemm_smallm.cu", "gemm_tile.cu", "gated_heads.cu", "attention.cu",
                     "attention_decode.cu", "attention_rows.cu", "sampling.cu", "no_alloc.cu"],
         "headers": _COMMON + ["gemm_stream.cuh", "no_alloc.h"],
         "cuda": True,

@@ -933,6 +933,74 @@ void attention_decode(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
   TORCH_CHECK(rc == 0, "mllm_b200 attention_decode: unsupported configuration (code ", rc, ")");
 }
 
+// row [T, hq * 2 D + 2 hkv * D]: per query head [query | gate], key heads, value heads -> q_out [T, hq, D] and the cache rows
+void gated_head_prologue(const Tensor& row, const Tensor& q_w, const Tensor& k_w, const Tensor& positions, const c10::optional<Tensor>& axis_map,
+                         const Tensor& inv_freq, const Tensor& loc, Tensor& q_out, Tensor& k_cache, Tensor& v_cache, double eps) {
+  check_half(row, "row");
+  TORCH_CHECK(q_out.dim() == 3 && q_out.is_contiguous() && q_out.scalar_type() == row.scalar_type() && q_out.is_cuda(), "q_out [T, Hq, D]");
+  const int64_t T = q_out.size(0), hq = q_out.size(1), D = q_out.size(2), hkv = k_cache.size(1), half = inv_freq.numel();
+  TORCH_CHECK((D == 64 || D == 128 || D == 256) && row.dim() == 2 && row.size(0) == T && row.stride(1) == 1 && row.stride(0) % 8 == 0 &&
+                  row.size(1) == (2 * hq + 2 * hkv) * D && (reinterpret_cast<uintptr_t>(row.data_ptr()) & 15) == 0,
+              "gated_head_prologue: row [T, (2 Hq + 2 Hkv) * D], 16-byte rows");
+  TORCH_CHECK(check_kv_cache(k_cache, v_cache, row.scalar_type(), hkv, D) == 0 &&
+                  ((reinterpret_cast<uintptr_t>(k_cache.data_ptr()) | reinterpret_cast<uintptr_t>(v_cache.data_ptr())) & 15) == 0,
+              "gated_head_prologue: caches of the rows' type");
+  for (const Tensor* t : {&q_w, &k_w})
+    TORCH_CHECK(t->is_cuda() && t->is_contiguous() && t->numel() == D && t->scalar_type() == row.scalar_type() &&
+                    (reinterpret_cast<uintptr_t>(t->data_ptr()) & 15) == 0,
+                "gated_head_prologue: gains [D]");
+  const int64_t lanes = half / (D / 32);
+  TORCH_CHECK(half % (D / 32) == 0 && lanes >= 1 && lanes <= 16 && (lanes & (lanes - 1)) == 0 && inv_freq.scalar_type() == at::kFloat &&
+                  inv_freq.is_cuda() && inv_freq.is_contiguous(),
+              "gated_head_prologue: rotated part");
+  const bool axes = axis_map.has_value();
+  TORCH_CHECK(positions.is_cuda() && positions.scalar_type() == at::kLong && positions.is_contiguous() && positions.numel() == (axes ? 3 * T : T) &&
+                  loc.is_cuda() && loc.scalar_type() == at::kLong && loc.is_contiguous() && loc.numel() == T,
+              "gated_head_prologue: positions int64 [T] or [3, T], loc int64 [T]");
+  if (axes)
+    TORCH_CHECK(axis_map->is_cuda() && axis_map->scalar_type() == at::kChar && axis_map->is_contiguous() && axis_map->numel() == half, "axis_map int8 [half]");
+  c10::cuda::CUDAGuard g(row.device());
+  auto& st = device_state(row.get_device());
+  mb200::GatedHeadArgs a{};
+  a.row = row.data_ptr();
+  a.q_w = q_w.data_ptr();
+  a.k_w = k_w.data_ptr();
+  a.positions = positions.data_ptr<int64_t>();
+  a.axis_map = axes ? axis_map->data_ptr<int8_t>() : nullptr;
+  a.inv_freq = inv_freq.data_ptr<float>();
+  a.loc = loc.data_ptr<int64_t>();
+  a.q_out = q_out.data_ptr();
+  a.k_cache = k_cache.data_ptr();
+  a.v_cache = v_cache.data_ptr();
+  a.status = st.status.data_ptr<int>();
+  a.row_stride = row.stride(0);
+  a.kv_tok_stride = k_cache.stride(0);
+  a.kv_head_stride = k_cache.stride(1);
+  a.num_slots = k_cache.size(0);
+  a.tokens = T;
+  a.hq = hq;
+  a.hkv = hkv;
+  a.dim = D;
+  a.half = half;
+  a.eps = static_cast<float>(eps);
+  a.dt = dtype_of(row);
+  const int rc = mb200::launch_gated_head_prologue(a, st.num_sms, stream_of(row));
+  TORCH_CHECK(rc == 0, "gated_head_prologue: launch failed (code ", rc, ")");
+}
+
+// x [T, Hq, D] *= sigmoid of the gates in `row`
+void gated_head_epilogue(Tensor& x, const Tensor& row) {
+  check_half(x, "x");
+  TORCH_CHECK(x.dim() == 3 && x.is_contiguous() && x.size(2) % 8 == 0 && (reinterpret_cast<uintptr_t>(x.data_ptr()) & 15) == 0 && row.dim() == 2 &&
+                  row.is_cuda() && row.size(0) == x.size(0) && row.size(1) >= 2 * x.size(1) * x.size(2) && row.stride(1) == 1 &&
+                  row.stride(0) % 8 == 0 && row.scalar_type() == x.scalar_type() && (reinterpret_cast<uintptr_t>(row.data_ptr()) & 15) == 0,
+              "gated_head_epilogue: x [T, Hq, D], row [T, ..] of one type");
+  c10::cuda::CUDAGuard g(x.device());
+  const int rc = mb200::launch_gated_head_epilogue(x.data_ptr(), row.data_ptr(), row.stride(0), x.size(0), x.size(1), x.size(2), dtype_of(x),
+                                                   device_state(x.get_device()).num_sms, stream_of(x));
+  TORCH_CHECK(rc == 0, "gated_head_epilogue: launch failed (code ", rc, ")");
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
@@ -944,6 +1012,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("embedding", &embedding);
   m.def("qk_norm_rope_kv_write", &qk_norm_rope_kv_write);
   m.def("kv_write", &kv_write);
+  m.def("gated_head_prologue", &gated_head_prologue);
+  m.def("gated_head_epilogue", &gated_head_epilogue);
   m.def("per_token_quant_int8", &per_token_quant_int8);
   m.def("argmax", &argmax);
   m.def("sample", &sample);

@@ -397,6 +397,28 @@ int64_t decode_stream_floats(int head_dim, int group, int ctas);
 int launch_decode_stream(const AttnArgs& args, cudaStream_t s);
 int decode_num_splits(int batch, int hkv, int max_seq_len, int num_sms);
 
+// ----- norm, partial rotation and cache write in front of attention with gated query heads, the gate behind it (gated_heads.cu) -----
+struct GatedHeadArgs {
+  const void* row;          // [tokens, row_stride]: per query head [query | gate], then the key heads, then the value heads
+  const void* q_w;          // gains of the norms [dim]
+  const void* k_w;
+  const int64_t* positions; // [tokens], or [3, tokens] with axis_map
+  const int8_t* axis_map;   // [half] row of positions per frequency, or null
+  const float* inv_freq;    // [half]
+  const int64_t* loc;       // [tokens] cache slots
+  void* q_out;              // [tokens, hq, dim]
+  void* k_cache;
+  void* v_cache;
+  int* status;
+  int64_t row_stride, kv_tok_stride, kv_head_stride, num_slots;
+  int tokens, hq, hkv, dim, half, hsplit;   // features i and i + half turn together, i < half; dim 64, 128 or 256
+  float eps;
+  DType dt;
+};
+int launch_gated_head_prologue(GatedHeadArgs args, int num_sms, cudaStream_t s);
+// x [tokens, hq, dim] *= sigmoid(gates of the projected rows)
+int launch_gated_head_epilogue(void* x, const void* row, int64_t row_stride, int tokens, int hq, int dim, DType dt, int num_sms, cudaStream_t s);
+
 // ----- attention of single rows, any head sizes, fp32 arithmetic (attention_rows.cu) -----------
 struct RowAttnArgs {
   const void* q;            // [rows, heads, dim], rows q_stride apart

@@ -120,27 +120,41 @@ class GatedDeltaNet(nn.Module):
         recurrent, conv = pool.layer(self.gdn_index)
         T = x.shape[0]
         m = gdn_batch(fb)
-        qkv = ops.linear(x, self.in_proj_qkv.weight)
-        z = ops.linear(x, self.in_proj_z.weight)
-        ba = ops.linear(x, torch.cat([self.in_proj_b.weight, self.in_proj_a.weight], 0)) if not hasattr(self, "_ba") else \
-            ops.linear(x, self._ba)
-        b, a = ba[:, : self.num_v_heads], ba[:, self.num_v_heads:]
+        H, C = self.num_v_heads, self.conv_dim
+        if "_fused" in self.__dict__:       # views of one product's rows
+            y = ops.linear(x, self._fused)
+            qkv, z, b, a = y[:, :C], y[:, C:C + self.value_dim], y[:, C + self.value_dim:C + self.value_dim + H], \
+                y[:, C + self.value_dim + H:C + self.value_dim + 2 * H]
+        else:
+            qkv = ops.linear(x, self.in_proj_qkv.weight)
+            z = ops.linear(x, self.in_proj_z.weight)
+            ba = ops.linear(x, torch.cat([self.in_proj_b.weight, self.in_proj_a.weight], 0))
+            b, a = ba[:, :H], ba[:, H:]
         qkv = ops.causal_conv1d_silu(qkv, self.conv1d.weight, conv, m.slots, m.lens, m.has_state, m.q_start, m.max_len)
         q, k, v = torch.split(qkv, [self.key_dim, self.key_dim, self.value_dim], dim=-1)
         # views of the convolution's rows; value head h uses query / key head h // (value heads / key heads)
         q = q.unflatten(1, (self.num_k_heads, self.head_k_dim))
         k = k.unflatten(1, (self.num_k_heads, self.head_k_dim))
         v = v.unflatten(1, (self.num_v_heads, self.head_v_dim))
-        beta = torch.sigmoid(b.float())
-        g = -torch.exp(self.A_log.float()) * torch.nn.functional.softplus(a.float() + self.dt_bias.float())
-        o = ops.gated_delta_rule(q, k, v, g, beta, recurrent, m.slots, m.lens, m.has_state, m.q_start)
-        o = ops.rmsnorm_gated(o.reshape(-1, self.head_v_dim), z.reshape(-1, self.head_v_dim), self.norm.weight, self.eps)
+        o = ops.gated_delta_rule(q, k, v, None, None, recurrent, m.slots, m.lens, m.has_state, m.q_start,
+                                 raw_gates=(b, a, self.A_log, self.dt_bias), max_len=m.max_len)
+        o = ops.rmsnorm_gated(o.reshape(T, self.value_dim), z, self.norm.weight, self.eps)
         y = ops.linear(o.reshape(T, self.value_dim), self.out_proj.weight)
         return pstate.tensor_model_parallel_all_reduce(y) if self.tp > 1 else y
 
-    def fuse_small_projections(self) -> None:
-        """One GEMM for the beta / decay projections (call after loading)."""
-        self._ba = torch.cat([self.in_proj_b.weight.data, self.in_proj_a.weight.data], 0).contiguous()
+    def fuse_projections(self) -> None:
+        """One matrix for everything that is taken of the layer input (call after loading); the parameters become views of it."""
+        parts = [m.weight for m in (self.in_proj_qkv, self.in_proj_z, self.in_proj_b, self.in_proj_a)]
+        rows = sum(w.shape[0] for w in parts)
+        # rows up to whole 256-column tiles of the large product, unless that is more than a twentieth of them
+        pad = 256 if -rows % 256 * 20 <= rows else 8
+        fused = parts[0].data.new_zeros((-(-rows // pad) * pad, parts[0].shape[1]))
+        at = 0
+        for w in parts:
+            fused[at:at + w.shape[0]].copy_(w.data)
+            w.data = fused[at:at + w.shape[0]]
+            at += w.shape[0]
+        self.__dict__["_fused"] = nn.Parameter(fused, requires_grad=False)
 
 
 class FusedGatedDeltaNet(nn.Module):

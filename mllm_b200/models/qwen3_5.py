@@ -77,6 +77,22 @@ class Qwen3_5Attention(nn.Module):
         self.k_norm = GemmaRMSNorm(self.head_dim, eps, dt)
         self.scale = self.head_dim ** -0.5
 
+    def fuse_projections(self) -> None:
+        """One matrix for the three projections (call after loading); the parameters become views of it."""
+        parts = [m.weight for m in (self.q_proj, self.k_proj, self.v_proj)]
+        fused = torch.cat([w.data for w in parts], 0)
+        at = 0
+        for w in parts:
+            w.data = fused[at:at + w.shape[0]]
+            at += w.shape[0]
+        self.__dict__["_fused"] = nn.Parameter(fused, requires_grad=False)
+        half = self.rotary_dim // 2
+        inv = 1.0 / (self.theta ** (torch.arange(0, self.rotary_dim, 2, device=fused.device, dtype=torch.float32) / self.rotary_dim))
+        axes = torch.zeros(half, dtype=torch.int8)
+        for axis in (1, 2):
+            axes[axis:min(self.mrope_section[axis] * 3, half):3] = axis
+        self.__dict__["_rotary"] = (inv, axes.to(fused.device))
+
     def _cos_sin(self, fb: ForwardBatch):
         half = self.rotary_dim // 2
         inv = 1.0 / (self.theta ** (torch.arange(0, self.rotary_dim, 2, device=fb.positions.device, dtype=torch.float32) / self.rotary_dim))
@@ -94,6 +110,15 @@ class Qwen3_5Attention(nn.Module):
 
     def forward(self, x: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:
         T, D = x.shape[0], self.head_dim
+        kc, vc = fb.token_to_kv_pool.get_kv_buffer(self.layer_id)
+        if "_fused" in self.__dict__ and ops.gated_heads_ok(x, kc, D, self.rotary_dim // 2):
+            row = ops.linear(x, self._fused)
+            inv, axes = self._rotary
+            mrope = fb.mrope_positions is not None
+            q = ops.gated_head_prologue(row, self.q_norm.weight, self.k_norm.weight, fb.mrope_positions if mrope else fb.positions,
+                                        axes if mrope else None, inv, fb.out_cache_loc, kc, vc, self.num_heads, D, self.q_norm.eps)
+            o = ops.gated_head_epilogue(self._attend(q, kc, vc, fb), row).view(T, self.num_heads * D)
+            return self._project(o)
         qg = ops.linear(x, self.q_proj.weight).view(T, self.num_heads, 2 * D)
         q, gate = qg[..., :D], qg[..., D:].reshape(T, self.num_heads * D)
         k = ops.linear(x, self.k_proj.weight).view(T, self.num_kv_heads, D)
@@ -103,19 +128,21 @@ class Qwen3_5Attention(nn.Module):
         cos, sin = self._cos_sin(fb)
         q = ref.apply_rope_neox(q.float(), cos, sin).to(x.dtype).contiguous()
         k = ref.apply_rope_neox(k.float(), cos, sin).to(x.dtype).contiguous()
-        kc, vc = fb.token_to_kv_pool.get_kv_buffer(self.layer_id)
         ops.kv_write(k.reshape(T, -1), v.reshape(T, -1), fb.out_cache_loc, kc, vc)
+        o = self._attend(q, kc, vc, fb).reshape(T, self.num_heads * D) * torch.sigmoid(gate.float()).to(x.dtype)
+        return self._project(o)
+
+    def _attend(self, q: torch.Tensor, kc: torch.Tensor, vc: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:
         rtt = fb.req_to_token_pool.req_to_token
         # head sizes 64 / 128 / 256 run on the attention kernels; ops falls back to library / PyTorch paths otherwise
         if fb.forward_mode.is_decode():
-            o = ops.attention_decode(q, kc, vc, rtt, fb.req_pool_indices, fb.seq_lens, self.scale, max_seq_len=fb.max_seq_len)
-        else:
-            ext_cpu, pre_cpu = getattr(fb, "extend_seq_lens_cpu", None), getattr(fb, "extend_prefix_lens_cpu", None)
-            seq_cpu = [a + b for a, b in zip(ext_cpu, pre_cpu)] if ext_cpu is not None and pre_cpu is not None else None
-            o = ops.attention_prefill(q, kc, vc, rtt, fb.req_pool_indices, fb.seq_lens, fb.extend_prefix_lens,
-                                      fb.extend_start_loc, self.scale, max_q_len=fb.max_extend_len,
-                                      seq_lens_cpu=seq_cpu, prefix_lens_cpu=pre_cpu)
-        o = o.reshape(T, self.num_heads * D) * torch.sigmoid(gate.float()).to(x.dtype)
+            return ops.attention_decode(q, kc, vc, rtt, fb.req_pool_indices, fb.seq_lens, self.scale, max_seq_len=fb.max_seq_len)
+        ext_cpu, pre_cpu = getattr(fb, "extend_seq_lens_cpu", None), getattr(fb, "extend_prefix_lens_cpu", None)
+        seq_cpu = [a + b for a, b in zip(ext_cpu, pre_cpu)] if ext_cpu is not None and pre_cpu is not None else None
+        return ops.attention_prefill(q, kc, vc, rtt, fb.req_pool_indices, fb.seq_lens, fb.extend_prefix_lens, fb.extend_start_loc, self.scale,
+                                     max_q_len=fb.max_extend_len, seq_lens_cpu=seq_cpu, prefix_lens_cpu=pre_cpu)
+
+    def _project(self, o: torch.Tensor) -> torch.Tensor:
         y = ops.linear(o, self.o_proj.weight)
         return pstate.tensor_model_parallel_all_reduce(y) if self.tp > 1 else y
 
@@ -277,8 +304,8 @@ class Qwen3_5ForCausalLM(nn.Module):
 
     def post_load(self) -> None:
         for m in self.modules():
-            if isinstance(m, GatedDeltaNet):
-                m.fuse_small_projections()
+            if isinstance(m, (GatedDeltaNet, Qwen3_5Attention)):
+                m.fuse_projections()
 
 
 class Qwen3_5ForConditionalGeneration(VisionLanguageMixin, Qwen3_5ForCausalLM):

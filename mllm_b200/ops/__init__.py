@@ -758,6 +758,30 @@ def kv_write(k, v, loc, k_cache, v_cache) -> None:
     ext().kv_write(k, v, loc.to(torch.int64).contiguous(), k_cache, v_cache)
 
 
+def gated_heads_ok(row: torch.Tensor, k_cache: torch.Tensor, dim: int, half: int) -> bool:
+    """Whether :func:`gated_head_prologue` has a kernel for these sizes: heads of 64, 128 or 256 features of which the first
+    ``2 half`` turn, 16-bit rows and a cache of their type."""
+    lanes = half // max(1, dim // 32)
+    return (use_kernels(row) and row.dtype in (torch.bfloat16, torch.float16) and k_cache.dtype == row.dtype and dim in (64, 128, 256)
+            and half % (dim // 32) == 0 and lanes in (1, 2, 4, 8, 16))
+
+
+def gated_head_prologue(row, q_weight, k_weight, positions, axis_map, inv_freq, loc, k_cache, v_cache, heads: int, dim: int, eps: float):
+    """``row`` [T, ..] holds per query head ``[query | gate]``, then the key and the value heads: queries and keys are normed per
+    head with a gain, their first ``2 * inv_freq.numel()`` features turn (feature i with feature i + half; ``axis_map`` names the
+    row of ``positions`` [3, T] of a frequency), keys and values go to ``loc`` of the caches.  Returns the queries [T, heads, dim]."""
+    q = torch.empty((row.shape[0], heads, dim), dtype=row.dtype, device=row.device)
+    ext().gated_head_prologue(row, q_weight, k_weight, positions.to(torch.int64).contiguous(), axis_map, inv_freq,
+                              loc.to(torch.int64).contiguous(), q, k_cache, v_cache, eps)
+    return q
+
+
+def gated_head_epilogue(x: torch.Tensor, row: torch.Tensor) -> torch.Tensor:
+    """``x[t, h] *= sigmoid(gate of head h in row t)``, in place; x [T, heads, dim]."""
+    ext().gated_head_epilogue(x, row)
+    return x
+
+
 # --------------------------------------------------------------------------
 # tensor-parallel reduction fused with residual add + RMSNorm
 # --------------------------------------------------------------------------
