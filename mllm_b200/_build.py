@@ -70,7 +70,7 @@ EXTENSIONS: Dict[str, Dict[str, List[str]]] = {
         "cuda": True,
     },
     "mllm_b200_E": {
-        "sources": ["bindings_moe.cpp", "runtime.cu", "moe.cu"],
+        "sources": ["bindings_moe.cpp", "runtime.cu", "moe.cu", "moe_pair.cu"],
         "headers": _COMMON,
         "cuda": True,
     },

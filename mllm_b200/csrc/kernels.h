@@ -355,6 +355,7 @@ struct MoeGemmArgs {
   DType dt;
 };
 int launch_moe_grouped_gemm(const MoeGemmArgs& args, cudaStream_t s);
+int launch_moe_pair_gemm(const MoeGemmArgs& args, cudaStream_t s);   // bn = 256 and n a multiple of 256 (moe_pair.cu)
 // the plain product (no SwiGLU) for fp32 and for sizes that the tensor-core kernel does not take
 int launch_moe_grouped_gemm_any(const MoeGemmArgs& args, cudaStream_t s);
 

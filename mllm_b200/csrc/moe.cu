@@ -340,44 +340,96 @@ int launch_router_mma_t(const void* x, int64_t x_ld, const void* w, float* logit
 }
 
 // --------------------------------------------------------------------------------------------
-// align: counting sort of the pairs by local expert + work list, one CTA
+// align: counting sort of the pairs by local expert + work list, one CTA or a cluster
 // --------------------------------------------------------------------------------------------
+__device__ __forceinline__ void align_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ int ld_cluster_s32(const int* local, uint32_t rank) {
+  uint32_t a;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(smem_u32(local)), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+  return v;
+}
+// The CTAs of a cluster (a power of two, or one CTA alone) take equal runs of the pairs, count them, exchange the counts through
+// distributed shared memory, and place them; what bounds a long list is the turn-around of two passes over it (65536 pairs of 128
+// experts: 70 us by one CTA).
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(const int* __restrict__ topk_ids, int pairs, int top_k, int expert_offset, int experts, int bn,
                  int* __restrict__ sorted_pos, int* __restrict__ src_token, int* __restrict__ expert_offsets,
                  int2* __restrict__ work, int* __restrict__ n_work, int max_work, const float* __restrict__ topk_w, float* __restrict__ src_w) {
   pdl_wait();
   __shared__ int cnt[kMaxExperts], off[kMaxExperts + 1], wbase[kMaxExperts + 1], fill[kMaxExperts];
-  for (int e = threadIdx.x; e < kMaxExperts; e += blockDim.x) {
-    cnt[e] = 0;
-    fill[e] = 0;
-  }
+  const int ctas = gridDim.x, rank = blockIdx.x;
+  const int i0 = static_cast<int>(static_cast<int64_t>(pairs) * rank / ctas), i1 = static_cast<int>(static_cast<int64_t>(pairs) * (rank + 1) / ctas);
+  for (int e = threadIdx.x; e < kMaxExperts; e += blockDim.x) cnt[e] = 0;
   __syncthreads();
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
     const int e = topk_ids[i] - expert_offset;
     if (e >= 0 && e < experts) atomicAdd(&cnt[e], 1);
   }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int o = 0, w = 0;
-    for (int e = 0; e < experts; ++e) {
-      off[e] = o;
-      wbase[e] = w;
-      o += cnt[e];
-      w += (cnt[e] + bn - 1) / bn;
+  if (ctas > 1) align_cluster_sync();
+  else __syncthreads();
+  if (threadIdx.x < kMaxExperts) {
+    int total = cnt[threadIdx.x], before = 0;
+    if (ctas > 1) {
+      total = 0;
+      for (int r = 0; r < ctas; ++r) {
+        const int c = ld_cluster_s32(&cnt[threadIdx.x], r);
+        before += r < rank ? c : 0;
+        total += c;
+      }
     }
-    off[experts] = o;
-    wbase[experts] = w;
-    *n_work = min(w, max_work);
+    off[threadIdx.x] = total;
+    fill[threadIdx.x] = before;
+  }
+  if (ctas > 1) align_cluster_sync();     // every count has been read: a CTA may leave
+  else __syncthreads();
+  if (threadIdx.x < 32) {                 // both running sums, eight experts per lane
+    constexpr int kPer = kMaxExperts / 32;
+    int c[kPer], o = 0, w = 0;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      c[i] = off[threadIdx.x * kPer + i];
+      o += c[i];
+      w += (c[i] + bn - 1) / bn;
+    }
+    int io = o, iw = w;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int uo = __shfl_up_sync(0xffffffffu, io, d), uw = __shfl_up_sync(0xffffffffu, iw, d);
+      if (static_cast<int>(threadIdx.x) >= d) {
+        io += uo;
+        iw += uw;
+      }
+    }
+    o = io - o;
+    w = iw - w;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) {
+      off[threadIdx.x * kPer + i] = o;
+      wbase[threadIdx.x * kPer + i] = w;
+      o += c[i];
+      w += (c[i] + bn - 1) / bn;
+    }
+    if (threadIdx.x == 31) {
+      off[kMaxExperts] = o;
+      wbase[kMaxExperts] = w;
+      if (rank == 0) *n_work = min(w, max_work);
+    }
   }
   __syncthreads();
-  for (int e = threadIdx.x; e <= experts; e += blockDim.x) expert_offsets[e] = off[e];
-  for (int e = threadIdx.x; e < experts; e += blockDim.x) {
-    const int chunks = wbase[e + 1] - wbase[e];
-    for (int c = 0; c < chunks; ++c)
-      if (wbase[e] + c < max_work) work[wbase[e] + c] = make_int2(e, c);
+  if (rank == 0) {
+    for (int e = threadIdx.x; e <= experts; e += blockDim.x) expert_offsets[e] = off[e];
+    for (int e = threadIdx.x; e < experts; e += blockDim.x) {
+      const int chunks = wbase[e + 1] - wbase[e];
+      for (int c = 0; c < chunks; ++c)
+        if (wbase[e] + c < max_work) work[wbase[e] + c] = make_int2(e, c);
+    }
   }
-  for (int i = threadIdx.x; i < pairs; i += blockDim.x) {
+  for (int i = i0 + threadIdx.x; i < i1; i += blockDim.x) {
     const int e = topk_ids[i] - expert_offset;
     if (e >= 0 && e < experts) {
       const int pos = off[e] + atomicAdd(&fill[e], 1);
@@ -794,8 +846,23 @@ int launch_moe_router_logits(const void* x, int64_t x_ld, const void* w, float* 
 void launch_moe_align(const int* topk_ids, int pairs, int top_k, int expert_offset, int experts, int bn, int* sorted_pos,
                       int* src_token, int* expert_offsets, int* work, int* n_work, int max_work, const float* topk_w, float* src_w,
                        cudaStream_t s) {
-  launch_pdl(moe_align_kernel, dim3(1), dim3(1024), 0, s, topk_ids, pairs, top_k, expert_offset, experts, bn, sorted_pos,
-             src_token, expert_offsets, reinterpret_cast<int2*>(work), n_work, max_work, topk_w, src_w);
+  // a cluster of eight from 4096 pairs on (four a thread)
+  const int ctas = pairs >= 4096 ? 8 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(ctas);
+  cfg.blockDim = dim3(1024);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = pdl_enabled() ? 1 : 0;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = static_cast<unsigned>(ctas);
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ctas > 1 ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, moe_align_kernel, topk_ids, pairs, top_k, expert_offset, experts, bn, sorted_pos, src_token, expert_offsets,
+                     reinterpret_cast<int2*>(work), n_work, max_work, topk_w, src_w);
   note_launch();
 }
 
@@ -846,6 +913,7 @@ int launch_moe_grouped_gemm(const MoeGemmArgs& a, cudaStream_t s) {
   if (a.k % 8 != 0 || a.ldc % 8 != 0 || a.n % 8 != 0) return -1;
   if (a.swiglu && (a.n % 256 != 0 || a.gelu)) return -1;
   if ((reinterpret_cast<uintptr_t>(a.x) | reinterpret_cast<uintptr_t>(a.w) | reinterpret_cast<uintptr_t>(a.out)) & 15) return -1;
+  if (a.bn == 256) return launch_moe_pair_gemm(a, s);
   const int r = a.swiglu ? 2 : 1;
   GroupedParams p{};
   p.out = a.out;

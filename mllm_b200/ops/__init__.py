@@ -1336,6 +1336,9 @@ def _moe_sorted_rows(x, w13, w2, topk_ids, expert_offset: int, swiglu_block: int
     dev = x.device
     any_size = x.dtype == torch.float32 or H % 8 != 0 or inter % 8 != 0
     bn = 16 if any_size else moe_chunk_rows(T, k, num_experts_global or E)
+    # 160 rows and more per expert on average: chunks of 256, multiplied by pairs of CTAs
+    if bn == 128 and P >= 160 * (num_experts_global or E) and N13 % 256 == 0 and H % 256 == 0 and (not gated or swiglu_block):
+        bn = 256
     max_work = E + (P + bn - 1) // bn
     i32 = dict(dtype=torch.int32, device=dev)
     sorted_pos = torch.empty(P, **i32)
