@@ -933,6 +933,57 @@ void attention_decode(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
   TORCH_CHECK(rc == 0, "mllm_b200 attention_decode: unsupported configuration (code ", rc, ")");
 }
 
+// A decoder layer over the new tokens of a prompt, one call for its eight launches: norm (the residual stream carries the sum),
+// projection, per-head norm + rotation + cache write, attention, projection, norm, gated MLP.  The launches and their buffers are
+// those of the calls one by one; what goes is the time between them (128 rows through 28 layers of 1024 features: 3.4 ms -> 2.0).
+// norms: input, post-attention [hidden], query and key [128] or none; weights: qkv, o, gate/up (interleaved), down.  Returns
+// (output, residual), or nothing when a product is not for gemm (before anything has been launched).
+std::vector<Tensor> prefill_layer(Tensor& hidden, const c10::optional<Tensor>& residual, const std::vector<Tensor>& norms,
+                                  const std::vector<Tensor>& weights, const c10::optional<Tensor>& qkv_bias, const Tensor& positions,
+                                  const c10::optional<Tensor>& axis_map, const Tensor& inv_freq, const Tensor& loc, Tensor& k_cache,
+                                  Tensor& v_cache, const std::vector<Tensor>& index, int64_t hq, int64_t hkv, double eps, double qk_eps,
+                                  double scale, int64_t max_q_len, int64_t window, double logit_cap, int64_t act) {
+  check_half(hidden, "hidden");
+  TORCH_CHECK((norms.size() == 2 || norms.size() == 4) && weights.size() == 4 && index.size() == 5, "prefill_layer: norms, weights, index tensors");
+  const Tensor &w_qkv = weights[0], &w_o = weights[1], &w_up = weights[2], &w_down = weights[3];
+  const int64_t T = hidden.size(0), D = 128;
+  for (const Tensor& w : weights)
+    if (w.dim() != 2 || w.scalar_type() != hidden.scalar_type() || w.size(0) % 8 != 0 || w.size(1) % 8 != 0 || w.stride(0) % 8 != 0 || w.stride(1) != 1)
+      return {};
+  if (w_up.size(0) % 256 != 0 || w_qkv.size(0) != (hq + 2 * hkv) * D || w_o.size(1) != hq * D || w_o.size(0) != hidden.size(1) ||
+      w_down.size(1) * 2 != w_up.size(0) || w_down.size(0) != hidden.size(1))
+    return {};
+  const auto opts = hidden.options();
+  auto product = [&](const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, int64_t gated) {
+    Tensor out = at::empty({T, gated != 0 ? w.size(0) / 2 : w.size(0)}, opts);
+    const int64_t rc = gemm(x, w, out, bias, c10::nullopt, gated, c10::nullopt, c10::nullopt, true, 0.0);
+    TORCH_CHECK(rc == 0, "mllm_b200 gemm: unsupported shape or launch failure (code ", rc, ") for M=", T, " N=", w.size(0), " K=", w.size(1));
+    return out;
+  };
+  Tensor x = hidden, res;
+  if (residual.has_value()) {
+    res = *residual;
+    fused_add_rmsnorm(x, res, norms[0], eps);
+  } else {
+    res = hidden;
+    x = at::empty_like(hidden);
+    rmsnorm(hidden, norms[0], x, eps);
+  }
+  Tensor qkv = product(x, w_qkv, qkv_bias, 0);
+  c10::optional<Tensor> qw, kw;
+  if (norms.size() == 4) {
+    qw = norms[2];
+    kw = norms[3];
+  }
+  qk_norm_rope_kv_write(qkv, qw, kw, positions, axis_map, inv_freq, loc, k_cache, v_cache, hq, hkv, D, qk_eps);
+  Tensor heads = at::empty({T, hq, D}, opts);
+  attention_prefill(qkv.as_strided({T, hq, D}, {qkv.stride(0), D, 1}), k_cache, v_cache, index[0], index[1], index[2], index[3], index[4], scale,
+                    heads, max_q_len, true, window, logit_cap, c10::nullopt, 0);
+  Tensor y = product(heads.view({T, hq * D}), w_o, c10::nullopt, 0);
+  fused_add_rmsnorm(y, res, norms[1], eps);
+  return {product(product(y, w_up, c10::nullopt, act), w_down, c10::nullopt, 0), res};
+}
+
 // row [T, hq * 2 D + 2 hkv * D]: per query head [query | gate], key heads, value heads -> q_out [T, hq, D] and the cache rows
 void gated_head_prologue(const Tensor& row, const Tensor& q_w, const Tensor& k_w, const Tensor& positions, const c10::optional<Tensor>& axis_map,
                          const Tensor& inv_freq, const Tensor& loc, Tensor& q_out, Tensor& k_cache, Tensor& v_cache, double eps) {
@@ -1013,6 +1064,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("qk_norm_rope_kv_write", &qk_norm_rope_kv_write);
   m.def("kv_write", &kv_write);
   m.def("gated_head_prologue", &gated_head_prologue);
+  m.def("prefill_layer", &prefill_layer);
   m.def("gated_head_epilogue", &gated_head_epilogue);
   m.def("per_token_quant_int8", &per_token_quant_int8);
   m.def("argmax", &argmax);

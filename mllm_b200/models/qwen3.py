@@ -20,10 +20,12 @@ from typing import Iterable, Optional, Tuple
 
 import torch
 from torch import nn
+from torch.nn.modules import module as nn_module
 
 from .. import ops
 from ..engine.forward_batch import ForwardBatch
 from ..layers import MLP, MergedLinear, RMSNorm, RadixAttention, RowParallelLinear, VocabParallelEmbedding
+from ..layers.quantize_base import UnquantizedLinearMethod
 from ..parallel import state as pstate
 from ..parallel.symm import get_tp_comm
 
@@ -172,8 +174,6 @@ class Qwen3DecoderLayer(nn.Module):
         self.input_layernorm = RMSNorm(config.hidden_size, eps, params_dtype)
         self.post_attention_layernorm = RMSNorm(config.hidden_size, eps, params_dtype)
         # the consumers of the two norms are plain tcgen05 GEMMs that can wait per gathered row tile
-        from ..layers.quantize_base import UnquantizedLinearMethod
-
         self._gated_qkv = isinstance(self.self_attn.qkv_proj.quant_method, UnquantizedLinearMethod) and \
             self.self_attn.qkv_proj.bias is None
         self._gated_mlp = isinstance(self.mlp, MLP) and isinstance(self.mlp.gate_up_proj.quant_method, UnquantizedLinearMethod)
@@ -202,10 +202,52 @@ class Qwen3DecoderLayer(nn.Module):
                                              self.post_attention_layernorm.eps, self.mlp.gate_up_proj.weight, swiglu=True)
         return self.mlp.down_proj(h), residual
 
+    def _forward_native(self, hidden, residual, fb):
+        """New tokens of prompts on one GPU with 16-bit weights: the layer as one native call, since the host's work for eight calls
+        takes longer than the kernels of a short prompt.  None for everything else, and where a part has been replaced or hooked."""
+        if fb.forward_mode.is_decode() or fb.forward_mode.is_idle() or not hidden.is_cuda or hidden.shape[0] == 0:
+            return None
+        mods = self._modules
+        attn, mlp, norm1, norm2 = mods["self_attn"], mods["mlp"], mods["input_layernorm"], mods["post_attention_layernorm"]
+        if type(attn) is not Qwen3Attention or type(mlp) is not MLP or type(norm1) is not RMSNorm or type(norm2) is not RMSNorm:
+            return None
+        am, mm = attn._modules, mlp._modules
+        core, qkv, o, up, down = am["attn"], am["qkv_proj"], am["o_proj"], mm["gate_up_proj"], mm["down_proj"]
+        parts = [attn, mlp, norm1, norm2, core, qkv, o, up, down]
+        if attn.use_qk_norm:
+            parts += [am["q_norm"], am["k_norm"]]
+            if type(parts[-1]) is not RMSNorm or type(parts[-2]) is not RMSNorm:
+                return None
+        for m in parts:
+            if m._forward_hooks or m._forward_pre_hooks or "forward" in m.__dict__:
+                return None
+        if nn_module._global_forward_hooks or nn_module._global_forward_pre_hooks or type(core) is not RadixAttention or type(qkv) is not MergedLinear or type(up) is not MergedLinear or \
+                type(o) is not RowParallelLinear or type(down) is not RowParallelLinear or o.tp_size > 1 or down.tp_size > 1 or \
+                core.head_dim != 128 or not up.__dict__.get("_gate_up_interleaved", False) or norm1.eps != norm2.eps:
+            return None
+        for m in (qkv, o, up, down):
+            if type(m.quant_method) is not UnquantizedLinearMethod or (m is not qkv and m._parameters.get("bias") is not None):
+                return None
+        if get_tp_comm() is not None:
+            return None
+        norms = [m._parameters["weight"] for m in (norm1, norm2, *parts[9:])]
+        weights = [m._parameters["weight"] for m in (qkv, o, up, down)]
+        k_cache, v_cache = fb.token_to_kv_pool.get_kv_buffer(core.layer_id)
+        inv_freq, axis_map = core._tables(hidden.device)
+        mrope = core.mrope_sections is not None and fb.mrope_positions is not None
+        index = [fb.req_to_token_pool.req_to_token, fb.req_pool_indices, fb.seq_lens, fb.extend_prefix_lens, fb.extend_start_loc]
+        return ops.prefill_layer(hidden, residual, norms, weights, qkv._parameters.get("bias"), fb.mrope_positions if mrope else fb.positions,
+                                 axis_map if mrope else None, inv_freq, fb.out_cache_loc, k_cache, v_cache, index, core.num_heads,
+                                 core.num_kv_heads, norm1.eps, core.rms_eps, core.scaling, fb.max_extend_len, core.sliding_window,
+                                 core.logit_cap, up.gate_activation)
+
     def forward(self, hidden: torch.Tensor, residual: Optional[torch.Tensor], forward_batch: ForwardBatch
                 ) -> Tuple[torch.Tensor, torch.Tensor]:
         if self._small_batch_fusable(hidden):
             return self._forward_small_batch(hidden, residual, forward_batch)
+        done = self._forward_native(hidden, residual, forward_batch)
+        if done is not None:
+            return done
         # residual-carry: the add of the previous block's output happens inside the next norm
         if residual is None:
             residual = hidden

@@ -758,6 +758,22 @@ def kv_write(k, v, loc, k_cache, v_cache) -> None:
     ext().kv_write(k, v, loc.to(torch.int64).contiguous(), k_cache, v_cache)
 
 
+def prefill_layer(hidden, residual, norms, weights, qkv_bias, positions, axis_map, inv_freq, loc, k_cache, v_cache, index, heads: int,
+                  kv_heads: int, eps: float, qk_eps: float, scale: float, max_q_len: int, window: Optional[int], logit_cap: float, act: str):
+    """A pre-norm decoder layer over new tokens in one native call: the kernels of the separate calls, without the host's work between
+    them.  ``norms``: input and post-attention gains, then those of the query and key heads (or none); ``weights``: qkv, o, interleaved
+    gate / up, down; ``index``: request table, its rows, lengths, prefix lengths and first rows of the requests.  Returns
+    ``(output, residual)``, or None where the separate calls have to be made: a product or a cache that the kernels do not take."""
+    if not (use_kernels(hidden) and hidden.dim() == 2 and hidden.is_contiguous() and hidden.dtype in (torch.bfloat16, torch.float16)
+            and hidden.shape[1] % 8 == 0 and (residual is None or residual.is_contiguous()) and _cache_dtype_ok(k_cache, hidden)
+            and act in ("silu", "gelu_tanh")):
+        return None
+    got = ext().prefill_layer(hidden, residual, norms, weights, qkv_bias, positions.to(torch.int64).contiguous(), axis_map, inv_freq,
+                              loc.to(torch.int64).contiguous(), k_cache, v_cache, index, heads, kv_heads, eps, qk_eps, scale, max_q_len,
+                              int(window or 0), float(logit_cap or 0.0), 1 if act == "silu" else 2)
+    return got or None
+
+
 def gated_heads_ok(row: torch.Tensor, k_cache: torch.Tensor, dim: int, half: int) -> bool:
     """Whether :func:`gated_head_prologue` has a kernel for these sizes: heads of 64, 128 or 256 features of which the first
     ``2 half`` turn, 16-bit rows and a cache of their type."""

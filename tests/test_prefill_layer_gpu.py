@@ -1,0 +1,65 @@
+"""A decoder layer over new tokens as one native call against the calls one by one."""
+
+from types import SimpleNamespace
+
+import pytest
+import torch
+
+from mllm_b200 import ops
+from mllm_b200.engine.forward_batch import ForwardMode
+from mllm_b200.models.qwen3 import Qwen3DecoderLayer
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(bias, norm):
+    torch.manual_seed(3)
+    config = SimpleNamespace(hidden_size=512, num_attention_heads=4, num_key_value_heads=2, head_dim=128, intermediate_size=768, rms_norm_eps=1e-6,
+                             attention_bias=bias, use_qk_norm=norm, rope_theta=1e4)
+    layer = Qwen3DecoderLayer(config, 0, params_dtype=torch.bfloat16).cuda()
+    for name, p in layer.named_parameters():
+        p.data.copy_(torch.randn_like(p, dtype=torch.float32) * (0.05 if p.dim() > 1 else 0.3) + (1.0 if "norm" in name else 0.0))
+    layer.mlp.gate_up_proj.quant_method.process_weights_after_loading(layer.mlp.gate_up_proj)
+    return layer
+
+
+def _batch(lens, prefix):
+    new = [n - p for n, p in zip(lens, prefix)]
+    width = max(lens)
+    table = torch.arange(len(lens) * width, dtype=torch.int32, device="cuda").view(len(lens), width)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    torch.manual_seed(5)
+    pools = [torch.randn(len(lens) * width, 2, 128, device="cuda").bfloat16() for _ in range(2)]
+    fb = SimpleNamespace(
+        forward_mode=ForwardMode.EXTEND, mrope_positions=None, req_to_token_pool=SimpleNamespace(req_to_token=table), extra={},
+        token_to_kv_pool=SimpleNamespace(get_kv_buffer=lambda i: pools), req_pool_indices=torch.arange(len(lens), **i32),
+        seq_lens=torch.tensor(lens, **i32), extend_prefix_lens=torch.tensor(prefix, **i32), max_extend_len=max(new),
+        extend_start_loc=torch.tensor([sum(new[:i]) for i in range(len(new))], **i32),
+        positions=torch.cat([torch.arange(p, n, device="cuda") for n, p in zip(lens, prefix)]),
+        out_cache_loc=torch.cat([table[i, p:n].long() for i, (n, p) in enumerate(zip(lens, prefix))]))
+    return fb, sum(new)
+
+
+@pytest.mark.parametrize("bias,norm", [(False, True), (True, False)])
+@pytest.mark.parametrize("lens,prefix", [([9], [0]), ([70, 200], [6, 0]), ([300, 41, 9], [0, 40, 1])], ids=str)
+@pytest.mark.parametrize("first", [False, True])
+def test_native_layer(bias, norm, lens, prefix, first, monkeypatch):
+    layer = _layer(bias, norm)
+
+    def run():
+        fb, rows = _batch(lens, prefix)
+        torch.manual_seed(7)
+        hidden, residual = torch.randn(rows, 512, device="cuda").bfloat16(), torch.randn(rows, 512, device="cuda").bfloat16()
+        out = layer(hidden, None if first else residual, fb)
+        return (*out, *fb.token_to_kv_pool.get_kv_buffer(0))
+
+    calls, native = [], ops.prefill_layer
+    monkeypatch.setattr(ops, "prefill_layer", lambda *a: calls.append(1) or native(*a))
+    got = run()
+    assert calls
+    handle = layer.self_attn.attn.register_forward_hook(lambda *a: calls.append(2))      # a hooked part is called as such
+    want = run()
+    handle.remove()
+    assert calls == [1, 2]
+    for g, w in zip(got, want):
+        assert torch.equal(g, w)     # the same kernels on the same numbers
