@@ -375,8 +375,17 @@ int launch_gemm_tile(const GemmArgs& a, cudaStream_t s) {
   // few weight rows: narrower tiles, until a cluster of eight per tile would fill the GPU
   while (bn > 32 && tiles(bn) * 8 <= sms) bn /= 2;
   if (tiles(bn) > 2 * sms) return 1;
-  p.cluster = 1;
-  while (p.cluster < 8 && tiles(bn) * p.cluster * 2 <= 2 * sms && p.k_blocks >= 4 * p.cluster) p.cluster *= 2;
+  auto cluster_of = [&](int bn) {
+    int c = 1;
+    while (c < 8 && tiles(bn) * c * 2 <= 2 * sms && p.k_blocks >= 4 * c) c *= 2;
+    return c;
+  };
+  // Short k: what a CTA exchanges grows with the tile's width, what it multiplies with its share of k.  Narrower tiles in smaller
+  // clusters while the share is under bn / 16 stages (128 rows: 4096 x 1024 12.2 us with 128 columns and 2 stages per CTA, 8.4 with
+  // 64 and 4, 8.7 with 32 and 8; 6144 x 1024 gated 12.1, 9.9 with 64 and 8, 11.7 with 32 and 16; 200 rows of 4096 x 2560 14.4 with
+  // 128 and 10, 15.1 with 64 and 20).
+  while (bn > 32 && cluster_of(bn) > 1 && p.k_blocks / cluster_of(bn) * 16 < bn) bn /= 2;
+  p.cluster = cluster_of(bn);
   p.out = a.out;
   p.bias = a.bias;
   p.residual = a.residual;
