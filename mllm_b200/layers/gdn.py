@@ -51,6 +51,19 @@ def gdn_batch(fb) -> GdnBatch:
     return got
 
 
+def views_of(fused: Optional[torch.Tensor], parts) -> bool:
+    """Whether ``parts`` still are the rows of ``fused``, one behind the other: a parameter that has been given other storage since
+    (another device or type, a replaced ``.data``) is read on its own."""
+    if fused is None:
+        return False
+    at = fused.data_ptr()
+    for w in parts:
+        if w.data_ptr() != at:
+            return False
+        at += w.numel() * w.element_size()
+    return True
+
+
 class GatedDeltaNet(nn.Module):
     def __init__(self, config, layer_id: int, gdn_index: int, params_dtype=None, prefix: str = "") -> None:
         super().__init__()
@@ -121,8 +134,9 @@ class GatedDeltaNet(nn.Module):
         T = x.shape[0]
         m = gdn_batch(fb)
         H, C = self.num_v_heads, self.conv_dim
-        if "_fused" in self.__dict__:       # views of one product's rows
-            y = ops.linear(x, self._fused)
+        parts = [m.weight for m in (self.in_proj_qkv, self.in_proj_z, self.in_proj_b, self.in_proj_a)]
+        if views_of(self.__dict__.get("_fused"), parts):
+            y = ops.linear(x, self._fused)      # views of one product's rows
             qkv, z, b, a = y[:, :C], y[:, C:C + self.value_dim], y[:, C + self.value_dim:C + self.value_dim + H], \
                 y[:, C + self.value_dim + H:C + self.value_dim + 2 * H]
         else:

@@ -23,7 +23,7 @@ from torch import nn
 from .. import ops
 from ..engine.forward_batch import ForwardBatch
 from ..layers import MLP, GemmaRMSNorm, VocabParallelEmbedding
-from ..layers.gdn import GatedDeltaNet
+from ..layers.gdn import GatedDeltaNet, views_of
 from ..mem_cache import GDNPool
 from ..ops import reference as ref
 from ..parallel import state as pstate
@@ -111,7 +111,8 @@ class Qwen3_5Attention(nn.Module):
     def forward(self, x: torch.Tensor, fb: ForwardBatch) -> torch.Tensor:
         T, D = x.shape[0], self.head_dim
         kc, vc = fb.token_to_kv_pool.get_kv_buffer(self.layer_id)
-        if "_fused" in self.__dict__ and ops.gated_heads_ok(x, kc, D, self.rotary_dim // 2):
+        parts = [m.weight for m in (self.q_proj, self.k_proj, self.v_proj)]
+        if views_of(self.__dict__.get("_fused"), parts) and ops.gated_heads_ok(x, kc, D, self.rotary_dim // 2):
             row = ops.linear(x, self._fused)
             inv, axes = self._rotary
             mrope = fb.mrope_positions is not None
