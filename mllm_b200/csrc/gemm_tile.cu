@@ -82,7 +82,6 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(acc_full + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_launch_dependents();
   if (threadIdx.x == 0) {
     for (int s = 0; s < n_stages; ++s) {
       mbar_init(&full_bar[s], 1);
@@ -102,6 +101,9 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem = *tmem_holder;
+  // behind the allocation, which waits for as long as the columns are taken: CTAs of the next kernel that took them first would hold
+  // them until this kernel ends
+  pdl_launch_dependents();
 
   const int rank = p.cluster > 1 ? static_cast<int>(my_rank()) : 0;
   const int tile = static_cast<int>(blockIdx.x) / p.cluster;

@@ -1,0 +1,30 @@
+"""Orders inside kernels whose violation would stop a GPU: shown on the sources, never by running a kernel that breaks them."""
+
+import re
+from pathlib import Path
+
+import pytest
+
+CSRC = Path(__file__).resolve().parents[1] / "mllm_b200" / "csrc"
+
+
+def _kernels(path):
+    """(name, body) of the ``__global__`` functions of a source, without comments."""
+    text = re.sub(r"//[^\n]*|/\*.*?\*/", "", path.read_text(), flags=re.S)
+    for m in re.finditer(r"__global__\s+void\s+(?:__launch_bounds__\((?:[^()]|\([^()]*\))*\)\s*)?(\w+)\s*\(", text):
+        at = text.index("{", text.index(")", m.end()))
+        depth, end = 1, at + 1
+        while depth:
+            depth += {"{": 1, "}": -1}.get(text[end], 0)
+            end += 1
+        yield m.group(1), text[at:end]
+
+
+@pytest.mark.parametrize("source", sorted(p.name for p in CSRC.glob("*.cu*")))
+def test_tensor_memory_is_allocated_before_the_next_kernel_may_start(source):
+    """tcgen05.alloc waits until its columns are free.  A kernel that has let the next one start before it has its own would wait for
+    blocks that wait for its end."""
+    for name, body in _kernels(CSRC / source):
+        alloc, trigger = re.search(r"\btmem_alloc(_pair)?\(", body), re.search(r"\bpdl_launch_dependents\(", body)
+        if alloc and trigger:
+            assert alloc.start() < trigger.start(), name
