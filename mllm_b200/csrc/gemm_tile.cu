@@ -113,6 +113,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   // first weight row; a gated tile has 64 gate rows and the up rows 128 behind them
   const int w_row = kGated ? (tn >> 1) * 256 + (tn & 1) * 64 : tn * kTileRows;
 
+  // Only the producer runs ahead of the stream-order wait.  The roles that wait for its copies begin behind it, so that their limits
+  // cover this kernel's own work and not the kernels in front.
   if (warp == 0) {
     if (lane == 0) {
       auto load_w = [&](int s, int kb) {
@@ -148,6 +150,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       }
     }
   } else if (warp == 1) {
+    pdl_wait_loads();
     if (lane == 0) {
       const uint64_t desc0 = umma_desc_k_sw128(smem_u32(smem));
       bool ok = true;
@@ -182,6 +185,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     }
     __syncwarp();
   } else {
+    pdl_wait_loads();
     if (!mbar_wait(acc_full, 0, abort_flag)) {
       *abort_flag = 1;
       if (p.status != nullptr) atomicExch(p.status, kStatusPipelineTimeout);
@@ -189,7 +193,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     tc_fence_after_sync();
   }
   __syncwarp();
-  pdl_wait_loads();        // bias and residual below may come from the kernels in front
+  pdl_wait_loads();        // the other lanes of the producer's warp too: all finish the output from what the kernels in front left
   __syncthreads();
   if (*abort_flag) {
     // copies may still be in flight: give them time to land before the ring is used for the sums

@@ -28,3 +28,31 @@ def test_tensor_memory_is_allocated_before_the_next_kernel_may_start(source):
         alloc, trigger = re.search(r"\btmem_alloc(_pair)?\(", body), re.search(r"\bpdl_launch_dependents\(", body)
         if alloc and trigger:
             assert alloc.start() < trigger.start(), name
+
+
+def _roles(body):
+    """The branches of a kernel's body in their order, statements between them included: (text, whether it is a branch)."""
+    depth, at = 0, 1
+    for i, c in enumerate(body[1:-1], 1):
+        depth += {"{": 1, "}": -1}.get(c, 0)
+        if c == "{" and depth == 1:
+            yield body[at:i], False
+            at = i
+        elif c == "}" and depth == 0:
+            yield body[at:i + 1], True
+            at = i + 1
+    yield body[at:-1], False
+
+
+@pytest.mark.parametrize("source", sorted(p.name for p in CSRC.glob("*.cu*")))
+def test_bounded_waits_begin_behind_the_stream_order_wait(source):
+    """A kernel that is launched early stays resident for as long as the kernels in front run.  A role whose bounded wait began before
+    the stream-order wait would count their time against its limit and give up in a healthy run."""
+    for name, body in _kernels(CSRC / source):
+        ordered = False
+        for text, branch in _roles(body):
+            first = re.search(r"\bmbar_wait\w*\(", text)
+            wait = re.search(r"\bpdl_wait(_loads)?\(\)", text)
+            if branch and first and not ordered:
+                assert wait and wait.start() < first.start(), (name, text[:80])
+            ordered = ordered or (wait is not None and not branch)
