@@ -190,8 +190,8 @@ __device__ __forceinline__ void load_gate_bias8(const KParams& p, int64_t row, f
   for (int j = 0; j < 8; ++j) x[j] = u[j] = 0.f;
   if constexpr (SWIGLU == 4) {
     if (p.bias == nullptr) return;
-    const uint4 raw[2] = {__ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + row)),
-                          __ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + row + kBM))};
+    const uint4 raw[2] = {__ldcg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + row)),
+                          __ldcg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + row + kBM))};
 #pragma unroll
     for (int half = 0; half < 2; ++half) {
       const uint32_t* w = reinterpret_cast<const uint32_t*>(&raw[half]);

@@ -280,11 +280,11 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     }
     if (p.bias != nullptr) {
       float b[8];
-      unpack8(__ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + wr)), p.out_f16, b);
+      unpack8(__ldcg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + wr)), p.out_f16, b);
 #pragma unroll
       for (int j = 0; j < 8; ++j) v[j] += b[j];
       if constexpr (SWIGLU == 4) {
-        unpack8(__ldg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + wr + 128)), p.out_f16, b);
+        unpack8(__ldcg(reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.bias) + wr + 128)), p.out_f16, b);
 #pragma unroll
         for (int j = 0; j < 8; ++j) u[j] += b[j];
       }

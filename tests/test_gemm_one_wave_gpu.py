@@ -52,6 +52,31 @@ def test_gated(m, n, k):
     _close(ops.linear_swiglu(x, w), (torch.nn.functional.silu(y[:, :, 0]) * y[:, :, 1]).reshape(m, -1))
 
 
+# the bias is written by a kernel that lets the product start before it has stored anything, while a product in front still reads
+# what was there
+@pytest.mark.parametrize("m,act", [(4, None), (20, None), (64, None), (200, None), (64, "clamped"), (600, "clamped")])
+def test_bias_of_the_kernel_in_front(m, act):
+    n = k = 4096
+    x, w = _rand(m, k), torch.nn.Parameter(_rand(n, k, seed=1, std=0.01), requires_grad=False)
+    gain, src, bias = torch.ones(n, device="cuda", dtype=torch.bfloat16), _rand(1, n, seed=9), _rand(n, seed=10)
+
+    def product(b):
+        return ops.linear(x, w, b) if act is None else ops.linear_swiglu(x, w, act=act, bias=b, limit=7.0)
+
+    product(bias)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        product(bias)
+        ops.ext().rmsnorm(src, gain, bias.view(1, n), 1e-6)
+        got = product(bias)
+    for i in range(20):
+        src.copy_(_rand(1, n, seed=11 + i))
+        want = product(ops.rmsnorm(src, gain, 1e-6).view(n).clone())
+        graph.replay()
+        assert torch.equal(got, want)
+
+
 @pytest.mark.parametrize("m", [9, 40, 200, 400])
 def test_tiles_int8(m):
     n, k = 328, 1056

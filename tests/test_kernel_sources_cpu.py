@@ -56,3 +56,17 @@ def test_bounded_waits_begin_behind_the_stream_order_wait(source):
             if branch and first and not ordered:
                 assert wait and wait.start() < first.start(), (name, text[:80])
             ordered = ordered or (wait is not None and not branch)
+
+
+# what the kernels read through the read-only path: parameters, which no kernel writes
+PARAMETERS = ("p.scales", "p.zeros")
+
+
+@pytest.mark.parametrize("source", sorted(p.name for p in CSRC.glob("*.cu*")))
+def test_read_only_loads_without_a_fence_are_of_parameters(source):
+    """Loads through the read-only path are not ordered by the stream-order wait: where it stands without its fence they may return
+    what was in a buffer before the kernel in front wrote it."""
+    text = re.sub(r"//[^\n]*|/\*.*?\*/", "", (CSRC / source).read_text(), flags=re.S)
+    if "pdl_wait_loads()" in text and "pdl_wait()" not in text:
+        for m in re.finditer(r"__ldg\(", text):
+            assert any(name in text[m.end():m.end() + 70] for name in PARAMETERS), text[m.start():m.end() + 70]
