@@ -15,9 +15,12 @@
 //   * Every kernel of the chain lets the next one start as soon as it runs itself.  With half an SM per CTA the CTAs of the next
 //     product move in as these leave, and fill their rings with weights, which no kernel writes, before they wait for their
 //     input: the end of one stream and the start of the next overlap.
-//   * 4-bit weights: a nibble under an exponent's bits is 128 + q, the base comes off the sum, and the group's scale multiplies
-//     the fp32 sum of the group's step: four logic operations and three shifts make eight weights.  (Taking the base off and
-//     rounding the product of q and scale to 16 bits for every weight cost eight more and precision.)
+//   * 4-bit weights: a nibble under an exponent's bits is base + q; one operation per pair takes base and zero point off, exactly,
+//     and the group's scale multiplies the fp32 sum of the group's step, so nothing of a weight is rounded (rounding the product of q
+//     and scale to 16 bits cost four operations more per eight weights, and precision).  In bf16 that operation also divides by 2048,
+//     which the sums get back at their end: a group's sum is then no larger than the largest x in it, and x may be as large as the
+//     type allows.  (Taking the base off the sum, as base times the sum of x, turns an infinite x into NaN:
+//     2 rows of 24576 x 4096 24.6 us that way, 24.2 this way, with zero points 26.3 and 25.7.)
 #pragma once
 
 #include "common.cuh"
@@ -80,8 +83,9 @@ __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uin
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// A pair of nibbles under the exponent's bits: base + q.  fp16 (base 1024) takes the base and the zero point off here, exactly; in
-// bf16 (base 128) they come off the sum, see kBias
+// A pair of nibbles under the exponent's bits, base + q, to q - zero (fp16, base 1024) or (q - zero) / 2048 (bf16, base 128); both are
+// exact.  `off2`: base + zero, or -(base + zero) / 2048
+constexpr float kScaled = 2048.f;
 template <bool F16>
 __device__ __forceinline__ uint32_t expand(uint32_t v, uint32_t off2) {
   constexpr uint32_t kMagic = F16 ? 0x64006400u : 0x43004300u;
@@ -89,18 +93,18 @@ __device__ __forceinline__ uint32_t expand(uint32_t v, uint32_t off2) {
   if constexpr (F16) {
     const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&off2));
     return *reinterpret_cast<const uint32_t*>(&r);
-  }
-  return v;
-}
-template <bool F16>
-__device__ __forceinline__ uint32_t splat(float f) {
-  if constexpr (F16) {
-    const __half2 r = __float2half2_rn(f);
-    return *reinterpret_cast<const uint32_t*>(&r);
   } else {
-    const __nv_bfloat162 r = __float2bfloat162_rn(f);
+    const __nv_bfloat162 r = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&v), __float2bfloat162_rn(1.f / kScaled),
+                                     *reinterpret_cast<const __nv_bfloat162*>(&off2));
     return *reinterpret_cast<const uint32_t*>(&r);
   }
+}
+// what `expand` takes off for a zero point: the bits of 1024 + zero, or of -(128 + zero) / 2048, whose last place is 2 / 2048 from
+// zero points of 128 on.  (Conversions from fp32 instead: 2 rows of 24576 x 4096 26.2 us, so 25.7.)
+template <bool F16>
+__device__ __forceinline__ uint32_t zero_bits(int zero) {
+  if constexpr (F16) return (0x6400u + zero) * 0x10001u;
+  return (0xBD80u + zero - ((max(zero, 128) - 127) >> 1)) * 0x10001u;
 }
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
@@ -231,21 +235,6 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
     }
   }
 
-  // 4-bit, bf16: the sum of a step's x for the two rows of x that this lane's accumulators belong to.  The weights enter as
-  // 128 + q, and the accumulators start at -(128 + zero) times that sum: 3e-5 of the result's size in fp32, at no cost per weight
-  constexpr bool kBias = W4 && !F16;
-  float xs[kBias ? JX : 1][2];
-  if constexpr (kBias) {
-#pragma unroll
-    for (int j = 0; j < JX; ++j) {
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int i = 0; i < kXRegs; i += 2) mma<F16>(c, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u, x[j][i], x[j][i + 1]);
-      xs[j][0] = c[0];
-      xs[j][1] = c[1];
-    }
-  }
-
   // sum of the warps' (and the cluster's) parts of one output, activation, bias, residual, store
   auto finish = [&](int u, int tok, int r, float v, float up) {
     if (tok >= p.m) return;
@@ -279,9 +268,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
   int slot = 0, buf = 0, done = 0;
   for (int u = u0; u < u1; ++u) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    constexpr float kBase = F16 ? 1024.f : 128.f;
-    const uint32_t off8 = splat<F16>(kBase + 8.f);
-    float z0f[kZeros ? kSc : 1], z1f[kZeros ? kSc : 1];
+    uint32_t o0[kZeros ? kSc : 1], o1[kZeros ? kSc : 1];
     float f0[kSc], f1[kSc];
     if constexpr (W4) {
 #pragma unroll
@@ -289,8 +276,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
         f0[j] = half_to_f<F16>(sc0[j]);
         f1[j] = half_to_f<F16>(sc1[j]);
         if constexpr (kZeros) {
-          z0f[j] = kBase + static_cast<float>(z0[j]);
-          z1f[j] = kBase + static_cast<float>(z1[j]);
+          o0[j] = zero_bits<F16>(z0[j]);
+          o1[j] = zero_bits<F16>(z1[j]);
         }
       }
       if (u + 1 < u1) fetch_scales(u + 1);
@@ -308,18 +295,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
           asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "r"(at + 512) : "memory");
           if constexpr (W4) {
             float s[2][4] = {};
-            if constexpr (kBias) {
-              const float b0 = kZeros ? z0f[kZeros ? j : 0] : kBase + 8.f, b1 = kZeros ? z1f[kZeros ? j : 0] : kBase + 8.f;
-              s[0][0] = -b0 * xs[j][0];
-              s[0][1] = -b0 * xs[j][1];
-              s[0][2] = -b1 * xs[j][0];
-              s[0][3] = -b1 * xs[j][1];
-            }
-            uint32_t oa = off8, ob = off8;
-            if constexpr (kZeros && F16) {
-              oa = splat<F16>(z0f[kZeros ? j : 0]);
-              ob = splat<F16>(z1f[kZeros ? j : 0]);
-            }
+            const uint32_t oa = kZeros ? o0[kZeros ? j : 0] : zero_bits<F16>(8), ob = kZeros ? o1[kZeros ? j : 0] : oa;
             const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
@@ -364,6 +340,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
       float v = 0.f;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) v += partial[buf][w][tok][r];
+      if constexpr (W4 && !F16) v *= kScaled;
       if (p.cluster > 1) {
         unit_sums[(u - u0) * 128 + threadIdx.x] = v;
       } else if constexpr (kGated) {

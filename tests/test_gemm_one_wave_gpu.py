@@ -99,3 +99,28 @@ def test_stream_4bit(m, n, k, group, zeros, interleaved, dtype):
     codes = ((words.unsqueeze(-1) >> torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)) & 15).flatten(1).double().view(n, -1, group)
     w = ((codes - (8 if z is None else z.double().unsqueeze(-1))) * scale.double().unsqueeze(-1)).flatten(1)
     _close(ops.w4a16_gemm(x, ops.w4a16_interleave(words) if interleaved else words, scale, z, group, None, interleaved=interleaved), x.double() @ w.t())
+
+
+@pytest.mark.parametrize("zeros,interleaved", [(False, True), (True, True), (True, False), (False, False)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_stream_4bit_large_values(zeros, interleaved, dtype):
+    n, k, group, m = 264, 4096, 128, 5
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    words = torch.randint(-2 ** 31, 2 ** 31, (n, k // 8), generator=g, device="cuda", dtype=torch.int32)
+    scale = (torch.rand((n, k // group), generator=g, device="cuda") * 0.01 + 0.005).to(dtype)
+    z = torch.randint(0, 16, (n, k // group), generator=g, device="cuda", dtype=torch.uint8) if zeros else None
+    x = _rand(m, k, dtype=dtype)
+    # infinities and NaN are those of the products; sums have the size of the result, so x may be as large as the type allows
+    x[1, 77] = float("inf")
+    x[2, 900] = -float("inf")
+    x[3, 5] = float("nan")
+    if dtype == torch.bfloat16:
+        x[4] *= 1e37
+    codes = ((words.unsqueeze(-1) >> torch.arange(0, 32, 4, device="cuda", dtype=torch.int32)) & 15).flatten(1).double().view(n, -1, group)
+    w = ((codes - (8 if z is None else z.double().unsqueeze(-1))) * scale.double().unsqueeze(-1)).flatten(1)
+    got = ops.w4a16_gemm(x, ops.w4a16_interleave(words) if interleaved else words, scale, z, group, None, interleaved=interleaved)
+    want = x.double() @ w.t()
+    assert torch.equal(got.isnan(), want.isnan())
+    assert torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[1:3].isinf() & (got[1:3] > 0), want[1:3].isinf() & (want[1:3] > 0))
+    _close(got[[0, 4]], want[[0, 4]])
