@@ -211,10 +211,6 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       uint32_t v[16];
       tmem_ld_32x16(t_base + c0, v);
       tmem_ld_wait();
-      if (p.is_int8) {
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = __float_as_uint(static_cast<float>(static_cast<int32_t>(v[j])));
-      }
       const uint32_t at = inbox + (((rank << cols_log) * kTileRows + row) << 2);
       if (p.cluster == 1) {
 #pragma unroll
@@ -251,21 +247,25 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     const int64_t col = static_cast<int64_t>(tn) * (kGated ? 64 : kTileRows) + grp * 8;
     if (row >= p.m || (!kGated && col >= p.n)) continue;
     float v[8] = {}, u[8] = {};
-    for (int src = 0; src < p.cluster; ++src) {       // in rank order
+    // in rank order; the sums of 8-bit products stay whole numbers, which 24 bits do not hold from a k of 1040 on
+    auto add = [&](float& sum, float part) {
+      sum = p.is_int8 ? __int_as_float(__float_as_int(sum) + __float_as_int(part)) : sum + part;
+    };
+    for (int src = 0; src < p.cluster; ++src) {
       const float4* from = reinterpret_cast<const float4*>(sums + (src * cols + c) * kTileRows + grp * 8);
 #pragma unroll
       for (int q = 0; q < 2; ++q) {
         const float4 x = from[q];
-        v[4 * q] += x.x;
-        v[4 * q + 1] += x.y;
-        v[4 * q + 2] += x.z;
-        v[4 * q + 3] += x.w;
+        add(v[4 * q], x.x);
+        add(v[4 * q + 1], x.y);
+        add(v[4 * q + 2], x.z);
+        add(v[4 * q + 3], x.w);
         if constexpr (kGated) {
           const float4 y = from[16 + q];              // 64 weight rows on
-          u[4 * q] += y.x;
-          u[4 * q + 1] += y.y;
-          u[4 * q + 2] += y.z;
-          u[4 * q + 3] += y.w;
+          add(u[4 * q], y.x);
+          add(u[4 * q + 1], y.y);
+          add(u[4 * q + 2], y.z);
+          add(u[4 * q + 3], y.w);
         }
       }
     }
@@ -274,8 +274,8 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
       const float sa = __ldcg(p.a_scale + row);
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        v[j] *= sa * p.b_scale[wr + j];
-        if constexpr (kGated) u[j] *= sa * p.b_scale[wr + 128 + j];
+        v[j] = static_cast<float>(__float_as_int(v[j])) * (sa * p.b_scale[wr + j]);
+        if constexpr (kGated) u[j] = static_cast<float>(__float_as_int(u[j])) * (sa * p.b_scale[wr + 128 + j]);
       }
     }
     if (p.bias != nullptr) {

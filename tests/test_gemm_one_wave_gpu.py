@@ -86,6 +86,22 @@ def test_tiles_int8(m):
     _close(ops.int8_scaled_mm(a, w, sa, sw, torch.bfloat16), (a.double() @ w.double().t()) * sa.double()[:, None] * sw.double())
 
 
+@pytest.mark.parametrize("m", [9, 64, 200, 300])
+def test_int8_sums_are_whole(m):
+    """Parts of a split k that cancel: whole numbers of 27 bits whose sum is small."""
+    n, k = 136, 16384
+    a = torch.full((m, k), 127, device="cuda", dtype=torch.int8)
+    w = torch.full((n, k), 127, device="cuda", dtype=torch.int8)
+    w[:, k // 2:] = -127
+    w[:, -1] = -126
+    g = torch.Generator(device="cuda").manual_seed(5)
+    a[:, :k // 2 - 1] -= torch.randint(0, 2, (m, k // 2 - 1), generator=g, device="cuda", dtype=torch.int8)
+    a[:, k // 2:-1] = a[:, :k // 2 - 1]
+    one_a, one_w = torch.ones(m, device="cuda"), torch.ones(n, device="cuda")
+    got = ops.int8_scaled_mm(a, w, one_a, one_w, torch.bfloat16)
+    assert torch.equal(got, (a.double() @ w.double().t()).to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("n,k,group", [(8, 128, 128), (1000, 1280, 128), (4096, 4096, 128), (264, 12288, 256), (40, 2048, 2048), (136, 2048, 64)])
 @pytest.mark.parametrize("m", [1, 5, 8])
 @pytest.mark.parametrize("zeros,interleaved", [(False, True), (True, True), (True, False), (False, False)])
