@@ -937,7 +937,8 @@ void attention_decode(const Tensor& q, const Tensor& k_cache, const Tensor& v_ca
 // projection, per-head norm + rotation + cache write, attention, projection, norm, gated MLP.  The launches and their buffers are
 // those of the calls one by one; what goes is the time between them (128 rows through 28 layers of 1024 features: 3.4 ms -> 2.0).
 // norms: input, post-attention [hidden], query and key [128] or none; weights: qkv, o, gate/up (interleaved), down.  Returns
-// (output, residual), or nothing when a product is not for gemm (before anything has been launched).
+// (output, residual), or nothing where a product or the attention is not for these kernels.  What cannot be served is declined or
+// raised before the first launch: the norms change the residual stream in place.
 std::vector<Tensor> prefill_layer(Tensor& hidden, const c10::optional<Tensor>& residual, const std::vector<Tensor>& norms,
                                   const std::vector<Tensor>& weights, const c10::optional<Tensor>& qkv_bias, const Tensor& positions,
                                   const c10::optional<Tensor>& axis_map, const Tensor& inv_freq, const Tensor& loc, Tensor& k_cache,
@@ -947,12 +948,29 @@ std::vector<Tensor> prefill_layer(Tensor& hidden, const c10::optional<Tensor>& r
   TORCH_CHECK((norms.size() == 2 || norms.size() == 4) && weights.size() == 4 && index.size() == 5, "prefill_layer: norms, weights, index tensors");
   const Tensor &w_qkv = weights[0], &w_o = weights[1], &w_up = weights[2], &w_down = weights[3];
   const int64_t T = hidden.size(0), D = 128;
+  const auto misaligned = [](const Tensor& t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15) != 0; };
   for (const Tensor& w : weights)
-    if (w.dim() != 2 || w.scalar_type() != hidden.scalar_type() || w.size(0) % 8 != 0 || w.size(1) % 8 != 0 || w.stride(0) % 8 != 0 || w.stride(1) != 1)
+    if (!w.is_cuda() || w.dim() != 2 || w.scalar_type() != hidden.scalar_type() || w.size(0) % 8 != 0 || w.size(1) % 8 != 0 ||
+        w.stride(0) % 8 != 0 || w.stride(1) != 1 || misaligned(w))
       return {};
-  if (w_up.size(0) % 256 != 0 || w_qkv.size(0) != (hq + 2 * hkv) * D || w_o.size(1) != hq * D || w_o.size(0) != hidden.size(1) ||
+  if (hidden.dim() != 2 || !hidden.is_contiguous() || misaligned(hidden) ||
+      (residual.has_value() && (residual->sizes() != hidden.sizes() || residual->scalar_type() != hidden.scalar_type() || !residual->is_cuda() ||
+                                !residual->is_contiguous() || misaligned(*residual))))
+    return {};
+  if (hkv <= 0 || hq % hkv != 0 || hq / hkv > 128 || w_up.size(0) % 256 != 0 || w_qkv.size(0) != (hq + 2 * hkv) * D || w_o.size(1) != hq * D || w_o.size(0) != hidden.size(1) ||
       w_down.size(1) * 2 != w_up.size(0) || w_down.size(0) != hidden.size(1))
     return {};
+  for (size_t i = 0; i < norms.size(); ++i)
+    TORCH_CHECK(norms[i].is_cuda() && norms[i].is_contiguous() && norms[i].numel() == (i < 2 ? hidden.size(1) : D), "prefill_layer: norm gains");
+  if (qkv_bias.has_value())
+    TORCH_CHECK(qkv_bias->is_cuda() && qkv_bias->scalar_type() == hidden.scalar_type() && qkv_bias->numel() == w_qkv.size(0) && qkv_bias->is_contiguous(), "bias");
+  check_kv_cache(k_cache, v_cache, hidden.scalar_type(), hkv, D);
+  TORCH_CHECK(positions.scalar_type() == at::kLong && positions.is_contiguous() && positions.is_cuda() &&
+                  positions.numel() == T * (positions.dim() == 2 ? positions.size(0) : 1) && loc.scalar_type() == at::kLong && loc.is_contiguous() &&
+                  loc.is_cuda() && loc.numel() == T && inv_freq.scalar_type() == at::kFloat && inv_freq.is_cuda() && inv_freq.numel() == D / 2,
+              "prefill_layer: positions int64 [T] or [3, T], slots int64 [T], inv_freq fp32 [64]");
+  for (const Tensor& t : index) TORCH_CHECK(t.scalar_type() == at::kInt && t.is_cuda(), "index tensors must be int32 CUDA tensors");
+  TORCH_CHECK(index[0].dim() == 2 && index[0].stride(1) == 1, "req_to_token layout");
   const auto opts = hidden.options();
   auto product = [&](const Tensor& x, const Tensor& w, const c10::optional<Tensor>& bias, int64_t gated) {
     Tensor out = at::empty({T, gated != 0 ? w.size(0) / 2 : w.size(0)}, opts);

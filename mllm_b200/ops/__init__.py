@@ -765,7 +765,7 @@ def prefill_layer(hidden, residual, norms, weights, qkv_bias, positions, axis_ma
     gate / up, down; ``index``: request table, its rows, lengths, prefix lengths and first rows of the requests.  Returns
     ``(output, residual)``, or None where the separate calls have to be made: a product or a cache that the kernels do not take."""
     if not (use_kernels(hidden) and hidden.dim() == 2 and hidden.is_contiguous() and hidden.dtype in (torch.bfloat16, torch.float16)
-            and hidden.shape[1] % 8 == 0 and (residual is None or residual.is_contiguous()) and _cache_dtype_ok(k_cache, hidden)
+            and hidden.shape[1] % 8 == 0 and attention_kernels_cover(k_cache.shape[-1], k_cache.dtype, hidden.dtype)
             and act in ("silu", "gelu_tanh")):
         return None
     got = ext().prefill_layer(hidden, residual, norms, weights, qkv_bias, positions.to(torch.int64).contiguous(), axis_map, inv_freq,

@@ -63,3 +63,30 @@ def test_native_layer(bias, norm, lens, prefix, first, monkeypatch):
     assert calls == [1, 2]
     for g, w in zip(got, want):
         assert torch.equal(g, w)     # the same kernels on the same numbers
+
+
+def _misaligned(w):
+    """The same rows two bytes behind a 16-byte boundary."""
+    store = torch.empty(w.numel() + 8, dtype=w.dtype, device=w.device)[1:w.numel() + 1].view(w.shape)
+    return store.copy_(w.data)
+
+
+@pytest.mark.parametrize("part", ["weight", "gains", "head sizes"])
+def test_declined_before_anything_is_launched(part, monkeypatch):
+    """What the native call cannot serve leaves the residual stream as it was."""
+    layer = _layer(False, True)
+    fb, rows = _batch([70], [6])
+    hidden, residual = torch.randn(rows, 512, device="cuda").bfloat16(), torch.randn(rows, 512, device="cuda").bfloat16()
+    before = [t.clone() for t in (hidden, residual, *fb.token_to_kv_pool.get_kv_buffer(0))]
+    if part == "weight":            # no kernel reads it: the calls one by one say so
+        layer.mlp.down_proj.weight.data = _misaligned(layer.mlp.down_proj.weight)
+        assert layer._forward_native(hidden, residual, fb) is None
+    elif part == "gains":
+        layer.post_attention_layernorm.weight.data = torch.ones(511, device="cuda", dtype=torch.bfloat16)
+        with pytest.raises(RuntimeError):
+            layer._forward_native(hidden, residual, fb)
+    else:                           # the switch that takes a head size off the kernels
+        monkeypatch.setattr(ops, "_ATTN_HEAD_SIZES", (64, 256))
+        assert layer._forward_native(hidden, residual, fb) is None
+    for t, b in zip((hidden, residual, *fb.token_to_kv_pool.get_kv_buffer(0)), before):
+        assert torch.equal(t, b)
