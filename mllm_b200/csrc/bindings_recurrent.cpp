@@ -171,10 +171,11 @@ int64_t gdn_channel_chunk(const Tensor& q, const Tensor& k, const Tensor& v, con
   return 0;
 }
 
-// max_len: the longest run of new tokens (0: not known).  Returns 1 (nothing launched) when the shape is not the chunk kernel's.
+// max_len: the longest run of new tokens (0: not known); workspace: bytes that may be allocated.  Returns 1 (nothing launched) when
+// the shape is not the chunk kernel's.
 int64_t gdn_chunk(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& g, const Tensor& beta, Tensor& state,
                   const Tensor& slots, const Tensor& lens, const Tensor& has, const Tensor& q_start, Tensor& out, bool split_tf32,
-                  int64_t max_len) {
+                  int64_t max_len, int64_t workspace) {
   mb200::GdnRuleParams p = rule_params(q, k, v, state, slots, lens, has, q_start, out);
   set_gates(p, g, beta, q.size(0));
   p.split_tf32 = split_tf32 ? 1 : 0;
@@ -182,9 +183,10 @@ int64_t gdn_chunk(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   c10::cuda::CUDAGuard gd(q.device());
   if (mb200::gdn_prefill_covers(p)) {
     const int longest = static_cast<int>(max_len > 0 ? std::min<int64_t>(max_len, q.size(0)) : q.size(0));
-    const mb200::GdnPrefillPlan plan = mb200::gdn_prefill_plan(p, longest);
+    const int sms = device_state(q.get_device()).num_sms;
+    const mb200::GdnPrefillPlan plan = mb200::gdn_prefill_plan(p, longest, workspace);
     Tensor ws = torch::empty({plan.ws_bytes}, state.options().dtype(torch::kUInt8));
-    const int rc = mb200::launch_gdn_prefill(p, ws.data_ptr(), plan.span, longest, device_state(q.get_device()).num_sms, stream_of(q));
+    const int rc = mb200::launch_gdn_prefill(p, ws.data_ptr(), plan, longest, sms, stream_of(q));
     TORCH_CHECK(rc == 0, "gdn_chunk: launch failed (code ", rc, ")");
     return 0;
   }
@@ -204,7 +206,8 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gdn_recurrent", &gdn_recurrent);
   m.def("gdn_recurrent_raw", &gdn_recurrent_raw);
   m.def("gdn_chunk", &gdn_chunk, py::arg("q"), py::arg("k"), py::arg("v"), py::arg("g"), py::arg("beta"), py::arg("state"), py::arg("slots"),
-        py::arg("lens"), py::arg("has"), py::arg("q_start"), py::arg("out"), py::arg("split_tf32"), py::arg("max_len") = 0);
+        py::arg("lens"), py::arg("has"), py::arg("q_start"), py::arg("out"), py::arg("split_tf32"), py::arg("max_len") = 0,
+        py::arg("workspace") = int64_t(512) << 20);
   m.def("gdn_channel_recurrent", &gdn_channel_recurrent);
   m.def("gdn_channel_chunk", &gdn_channel_chunk);
   m.def("read_status", &read_status);

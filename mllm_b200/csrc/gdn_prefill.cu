@@ -554,15 +554,18 @@ int launch_scan(const PrefillParams& pp, cudaStream_t s) {
 
 bool gdn_prefill_covers(const GdnRuleParams& p) { return p.dt == kBF16 && !p.split_tf32 && gdn_chunk_covers(p); }
 
-GdnPrefillPlan gdn_prefill_plan(const GdnRuleParams& p, int max_len) {
-  // up to 512 MB of the workspace at a time; longer runs go over it in spans of chunks
-  constexpr int64_t kMost = int64_t(512) << 20;
-  const int64_t chunk = slot_bytes(p.dv) * p.heads * std::max(1, p.batch);
-  const int64_t span = std::max<int64_t>(1, std::min<int64_t>((max_len + kC - 1) / kC, kMost / chunk));
-  return {static_cast<int>(span), span * chunk};
+// As many chunks of all requests as `most_bytes` have room for; where not even one fits, one chunk of equal groups of requests.  The
+// least is a chunk of one request.  (Groups that fill the GPU once, with longer spans, leave the scan's last CTAs of every group
+// alone: 32 x 1024 tokens 1467 us instead of 1388 with 512 MB.  128 MB instead of 512: 4 x 2000 tokens 450 us instead of 432,
+// 32 x 1024 1651.)
+GdnPrefillPlan gdn_prefill_plan(const GdnRuleParams& p, int max_len, int64_t most_bytes) {
+  const int64_t chunk = slot_bytes(p.dv) * p.heads, slots = std::max<int64_t>(1, most_bytes / chunk);
+  const int64_t batch = std::max(1, p.batch), groups = (batch + slots - 1) / slots, group = (batch + groups - 1) / groups;
+  const int64_t span = std::max<int64_t>(1, std::min<int64_t>((max_len + kC - 1) / kC, slots / group));
+  return {static_cast<int>(group), static_cast<int>(span), group * span * chunk};
 }
 
-int launch_gdn_prefill(const GdnRuleParams& p, void* ws, int span, int max_len, int num_sms, cudaStream_t s) {
+int launch_gdn_prefill(const GdnRuleParams& p, void* ws, const GdnPrefillPlan& plan, int max_len, int num_sms, cudaStream_t s) {
   if (p.batch <= 0 || max_len <= 0) return 0;
   if (!gdn_prefill_covers(p) || p.heads % p.k_heads != 0 || p.g == nullptr || (reinterpret_cast<uintptr_t>(p.out) & 3) != 0) return -1;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(gdn_prepare_kernel), kPrepareSmem) != cudaSuccess) return -3;
@@ -571,7 +574,7 @@ int launch_gdn_prefill(const GdnRuleParams& p, void* ws, int span, int max_len, 
   int best = 64, least = 1 << 30;
   const int widths[3] = {16, 32, 64}, times[3] = {12, 17, 29};
   for (int i = 0; i < 3; ++i) {
-    const int64_t ctas = static_cast<int64_t>(p.batch) * p.heads * ((p.dv + widths[i] - 1) / widths[i]);
+    const int64_t ctas = static_cast<int64_t>(plan.group) * p.heads * ((p.dv + widths[i] - 1) / widths[i]);
     const int64_t cost = (ctas + num_sms - 1) / num_sms * times[i];
     if (cost < least) {
       least = static_cast<int>(std::min<int64_t>(cost, 1 << 30));
@@ -579,13 +582,21 @@ int launch_gdn_prefill(const GdnRuleParams& p, void* ws, int span, int max_len, 
     }
   }
   const int chunks = (max_len + kC - 1) / kC;
-  for (int c0 = 0; c0 < chunks; c0 += span) {
-    PrefillParams pp{p, static_cast<uint8_t*>(ws), c0, span};
-    const cudaError_t err = launch_pdl(gdn_prepare_kernel, dim3(std::min(span, chunks - c0), p.heads, p.batch), dim3(kThreads), kPrepareSmem, s, pp);
-    note_launch();      // the pair counts as one: the rule over a span
-    if (err != cudaSuccess) return -4;
-    const int rc = best == 16 ? launch_scan<16>(pp, s) : best == 32 ? launch_scan<32>(pp, s) : launch_scan<64>(pp, s);
-    if (rc != 0) return rc;
+  for (int b0 = 0; b0 < p.batch; b0 += plan.group) {
+    GdnRuleParams r = p;
+    r.batch = std::min(plan.group, p.batch - b0);
+    r.slots += b0;
+    r.lens += b0;
+    r.has_state += b0;
+    r.q_start += b0;
+    for (int c0 = 0; c0 < chunks; c0 += plan.span) {
+      PrefillParams pp{r, static_cast<uint8_t*>(ws), c0, plan.span};
+      const cudaError_t err = launch_pdl(gdn_prepare_kernel, dim3(std::min(plan.span, chunks - c0), r.heads, r.batch), dim3(kThreads), kPrepareSmem, s, pp);
+      note_launch();      // the pair counts as one: the rule over a span
+      if (err != cudaSuccess) return -4;
+      const int rc = best == 16 ? launch_scan<16>(pp, s) : best == 32 ? launch_scan<32>(pp, s) : launch_scan<64>(pp, s);
+      if (rc != 0) return rc;
+    }
   }
   return 0;
 }

@@ -578,15 +578,15 @@ int launch_gdn_recurrent(const GdnRuleParams& p, cudaStream_t s);
 // the same rule evaluated 64 tokens at a time with tensor-core products (prefill; fp16, or split_tf32); dk up to 128, multiples of 8
 int launch_gdn_chunk(const GdnRuleParams& p, int num_sms, cudaStream_t s);
 bool gdn_chunk_covers(const GdnRuleParams& p);
-// prefill of bf16 inputs without split_tf32, where gdn_chunk_covers (gdn_prefill.cu).  The workspace holds `span` chunks of every
-// request; longer runs loop over spans
+// prefill of bf16 inputs without split_tf32, where gdn_chunk_covers (gdn_prefill.cu).  The workspace holds `span` chunks of `group`
+// requests; longer runs and larger batches loop over it
 struct GdnPrefillPlan {
-  int span;
+  int group, span;
   int64_t ws_bytes;
 };
 bool gdn_prefill_covers(const GdnRuleParams& p);
-GdnPrefillPlan gdn_prefill_plan(const GdnRuleParams& p, int max_len);
-int launch_gdn_prefill(const GdnRuleParams& p, void* ws, int span, int max_len, int num_sms, cudaStream_t s);
+GdnPrefillPlan gdn_prefill_plan(const GdnRuleParams& p, int max_len, int64_t most_bytes);
+int launch_gdn_prefill(const GdnRuleParams& p, void* ws, const GdnPrefillPlan& plan, int max_len, int num_sms, cudaStream_t s);
 // decays per key channel, 16 tokens at a time (prefill); dk up to 128, multiples of 8, gates formed inside.  The workspace
 // holds `span` chunks of every request; longer runs loop over spans
 struct GdnChannelPlan {

@@ -474,6 +474,8 @@ class ModelRunner:
         frac = self.server_config.mem_fraction_static or 0.85
         avail = get_available_gpu_memory(self.device.type, self.gpu_id)
         rest = avail - self._pre_load_avail_gib * (1.0 - frac)
+        if self.device.type == "cuda":      # what a step keeps between its kernels comes out of the same memory
+            rest -= getattr(self.model, "step_workspace_bytes", 0) / (1 << 30)
         cell = self.cell_bytes()
         tokens = int(rest * (1 << 30) // cell)
         return MemoryProfileResult(max_total_num_tokens=tokens, cell_bytes=cell, rest_gib=rest)

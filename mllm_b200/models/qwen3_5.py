@@ -303,6 +303,9 @@ class Qwen3_5ForCausalLM(nn.Module):
                 loaded.add(h)
         return {n for n in loaded if not n.endswith((':gate', ':up'))}
 
+    # beside the caches, for the prefill of the delta rule
+    step_workspace_bytes = ops.GDN_WORKSPACE_BYTES
+
     def post_load(self) -> None:
         for m in self.modules():
             if isinstance(m, (GatedDeltaNet, Qwen3_5Attention)):

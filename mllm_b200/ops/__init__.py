@@ -1155,6 +1155,8 @@ def set_gdn_extend_backend(name: str) -> None:
 
 
 _GDN_MAX_DK = 512       # key features the sequential kernel holds
+# most bytes that the delta rule's prefill keeps between its kernels; a server leaves them free beside the caches
+GDN_WORKSPACE_BYTES = 512 << 20
 
 
 def _heads_like(t: torch.Tensor, heads: int) -> torch.Tensor:
@@ -1185,7 +1187,7 @@ def gated_delta_rule(q, k, v, g, beta, state, state_indices, seq_lens, has_state
                 g, beta = gdn_gates(*raw_gates)
                 raw_gates = None
             g, beta = g.float().contiguous(), beta.float().contiguous()
-            if ext().gdn_chunk(q, k, v, g, beta, *meta, split_tf32, int(max_len)) == 0:
+            if ext().gdn_chunk(q, k, v, g, beta, *meta, split_tf32, int(max_len), GDN_WORKSPACE_BYTES) == 0:
                 return out
         if raw_gates is not None:
             ext().gdn_recurrent_raw(q, k, v, *raw_gates, *meta)

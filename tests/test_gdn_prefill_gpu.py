@@ -67,6 +67,32 @@ def test_decays(decay):
     _check([200], 2, 2, 128, 128, decay=decay)
 
 
-def test_spans_of_the_workspace():
-    """Enough heads that the 512 MB of the workspace hold two chunks at a time."""
+@pytest.mark.parametrize("chunks", [2, 3, 5])
+@pytest.mark.parametrize("lens", [[330, 129], [64 * 7 + 1], [1, 0, 640, 65, 200]], ids=str)
+def test_spans_of_the_workspace(lens, chunks, monkeypatch):
+    """Room for one to five chunks at a time: spans of several chunks, the last one in part, that take the state up where the span before
+    left it; fewer chunks than requests, which then come in groups."""
+    heads, slot = 6, 2 * 64 * 128 * 2 + 2 * 64 * 64 * 2 + 160 * 4 + 64 * 128 * 4      # of a (chunk, head): W and P in two terms, scalars, U0
+    monkeypatch.setattr(ops, "GDN_WORKSPACE_BYTES", chunks * heads * slot)
+    _check(lens, heads, 3, 128, 128)
+
+
+def test_workspace_of_many_requests(monkeypatch):
+    """One chunk of all requests is more than the workspace may have."""
+    monkeypatch.setattr(ops, "GDN_WORKSPACE_BYTES", 1 << 20)
+    lens = [40 + 7 * (i % 5) for i in range(24)]
+    _check(lens, 2, 2, 128, 128)
+    T = sum(lens)
+    q, k, v = (torch.randn(T, 2, 128, device="cuda").bfloat16() for _ in range(3))
+    g, beta, state = -torch.rand(T, 2, device="cuda"), torch.rand(T, 2, device="cuda"), torch.zeros(24, 2, 128, 128, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+    index = (torch.arange(24, **i32), torch.tensor(lens, **i32), torch.zeros(24, **i32))
+    torch.cuda.reset_peak_memory_stats()
+    inputs = torch.cuda.memory_allocated()
+    ops.gated_delta_rule(q, k, v, g, beta, state, *index, max_len=max(lens))
+    assert torch.cuda.max_memory_allocated() - inputs < (1 << 20) + v.numel() * 2 + (64 << 10)
+
+
+def test_spans_of_many_heads():
+    """Heads that leave room for one chunk at a time in 512 MB, the longest run not known."""
     _check([330, 129], 1700, 100, 8, 128, max_len=0)
