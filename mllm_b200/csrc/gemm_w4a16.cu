@@ -180,7 +180,8 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_holder;
-  pdl_wait();
+  // activations come by TMA; scales, zero points and bias by ordinary loads
+  pdl_wait_loads();
 
   const int split = blockIdx.y;
   const int kb0 = split * p.kb_per_split;

@@ -67,6 +67,10 @@ def test_read_only_loads_without_a_fence_are_of_parameters(source):
     """Loads through the read-only path are not ordered by the stream-order wait: where it stands without its fence they may return
     what was in a buffer before the kernel in front wrote it."""
     text = re.sub(r"//[^\n]*|/\*.*?\*/", "", (CSRC / source).read_text(), flags=re.S)
+    for name, body in _kernels(CSRC / source):
+        if "pdl_wait_loads()" in body and "pdl_wait()" not in body:
+            for m in re.finditer(r"__ldg\(", body):
+                assert any(p in body[m.end():m.end() + 70] for p in PARAMETERS), (name, body[m.start():m.end() + 70])
     if "pdl_wait_loads()" in text and "pdl_wait()" not in text:
         for m in re.finditer(r"__ldg\(", text):
             assert any(name in text[m.end():m.end() + 70] for name in PARAMETERS), text[m.start():m.end() + 70]
