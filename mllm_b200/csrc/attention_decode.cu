@@ -379,6 +379,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
     const bool whole = t0 == 0 && n == n_all;
     const int64_t part = (static_cast<int64_t>(blockIdx.x) * 2 + (at_run_begin ? 0 : 1)) * g;
     const float* parts = reinterpret_cast<const float*>(ring - warp * C::kRingBytes);
+    // a sum of 0: no key to be seen.  A NaN or infinite score makes it NaN, and that the result
     for (int i = threadIdx.x; i < g * HD; i += kThreads) {
       const int h = i / HD, d = i % HD;
       float top = part_m[0][h];
@@ -393,10 +394,10 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
       }
       if (whole) {
         if (p.sink != nullptr) den += exp2f(p.sink[hk * g + h] * kLog2e - top);
-        static_cast<T*>(p.out)[b * p.out_stride + static_cast<int64_t>(hk * g + h) * HD + d] = from_f32<T>(den > 0.f ? acc / den : 0.f);
+        static_cast<T*>(p.out)[b * p.out_stride + static_cast<int64_t>(hk * g + h) * HD + d] = from_f32<T>(den == 0.f ? 0.f : acc / den);
       } else {
-        p.part_o[(part + h) * HD + d] = den > 0.f ? acc / den : 0.f;
-        if (d == 0) p.part_lse[part + h] = den > 0.f ? top + log2f(den) : -INFINITY;
+        p.part_o[(part + h) * HD + d] = den == 0.f ? 0.f : acc / den;
+        if (d == 0) p.part_lse[part + h] = den == 0.f ? -INFINITY : top + log2f(den);
       }
     }
     __syncthreads();
@@ -472,7 +473,7 @@ __global__ void __launch_bounds__(kThreads) attn_decode_join_kernel(const Decode
 #pragma unroll
   for (int k = 0; k < kPer; ++k) {
     const int d = threadIdx.x + k * kThreads;
-    if (d < HD) out[d] = from_f32<T>(den > 0.f ? acc[k] / den : 0.f);
+    if (d < HD) out[d] = from_f32<T>(den == 0.f ? 0.f : acc[k] / den);
   }
 }
 

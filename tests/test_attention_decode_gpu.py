@@ -67,3 +67,23 @@ def test_sink_joins_whole_and_divided_contexts():
 def test_fp16_and_slot_major():
     _run(LENGTHS["edges"], 16, 4, 128, dtype=torch.float16)
     _run(LENGTHS["edges"], 16, 4, 128, head_major=False)
+
+
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("hq,hkv,hd", [(8, 2, 64), (16, 4, 128), (8, 2, 256)])
+def test_scores_that_are_no_numbers(hq, hkv, hd, value):
+    """A key of NaN or infinity makes the softmax of its head NaN, whether the context lies in one thread block or in many; it leaves the
+    other heads and requests alone."""
+    lens = [3, 70, 5000, 40]
+    g = torch.Generator(device="cuda").manual_seed(hd)
+    table = torch.arange(sum(lens), dtype=torch.int32, device="cuda")
+    table = torch.nn.utils.rnn.pad_sequence(table.split(lens), batch_first=True).contiguous()
+    k, v = (torch.randn((sum(lens), hkv, hd), generator=g, device="cuda").bfloat16() for _ in range(2))
+    q = torch.randn((len(lens), hq, hd), generator=g, device="cuda").abs().bfloat16()
+    for b in (0, 2):
+        k[table[b, 2].item(), 1] = value
+    req, seq = torch.arange(len(lens), dtype=torch.int32, device="cuda"), torch.tensor(lens, dtype=torch.int32, device="cuda")
+    got = ops.attention_decode(q, k, v, table, req, seq, hd ** -0.5, max_seq_len=max(lens)).view(len(lens), hkv, -1, hd)
+    hit = torch.zeros_like(got, dtype=torch.bool)
+    hit[0, 1] = hit[2, 1] = True
+    assert torch.equal(got.isnan(), hit)
