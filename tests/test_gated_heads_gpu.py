@@ -12,8 +12,9 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("dim,half", [(64, 8), (64, 32), (128, 16), (256, 32), (256, 128)])
 @pytest.mark.parametrize("tokens", [1, 9, 5000])
 @pytest.mark.parametrize("axes", [False, True])
-def test_prologue_and_epilogue(dim, half, tokens, axes):
-    hq, hkv, eps, dt = 6, 2, 1e-6, torch.bfloat16
+@pytest.mark.parametrize("dt", [torch.bfloat16, torch.float16])
+def test_prologue_and_epilogue(dim, half, tokens, axes, dt):
+    hq, hkv, eps = 6, 2, 1e-6
     g = torch.Generator(device="cuda").manual_seed(dim + tokens)
     row = torch.randn((tokens, (2 * hq + 2 * hkv) * dim), generator=g, device="cuda").to(dt)
     qw, kw = (1 + 0.1 * torch.randn((dim,), generator=g, device="cuda").to(dt) for _ in range(2))
