@@ -1060,7 +1060,7 @@ int launch_attention(const AttnArgs& a, cudaStream_t s) {
     p.kv_row_add = static_cast<int>(a.num_slots);
     p.kv_runs = 1;
   } else if (a.is_decode && specialised && g <= 32) {
-    return -1;                   // decode at this head size is for the two layouts that the pools have
+    return -1;                   // refused: no pool has another layout (the decode kernel itself takes any strides)
   }
   if (a.is_decode && decode_streams(hd, g, a.kv_fmt)) {
     if ((reinterpret_cast<uintptr_t>(a.k_cache) | reinterpret_cast<uintptr_t>(a.v_cache)) & 15) return -2;

@@ -257,8 +257,8 @@ size_t gemm_workspace_bytes(int m, int n, int k, int num_sms);
 // products whose tiles fit one wave of two CTAs per SM, more than 8 rows (gemm_tile.cu).  Returns 0 when launched, 1 when the
 // product is not for it.
 int launch_gemm_tile(const GemmArgs& args, cudaStream_t s);
-// m <= 8, 16-bit operands: the weight matrix streamed through registers and warp-level MMAs (no tensor memory, no
-// shared-memory ring, no split of k between CTAs).  Returns 0 when launched, 1 when the shape is not for it.
+// m <= 8, 16-bit operands: the weight matrix streamed through per-lane copy queues and warp-level MMAs, long k cut over a cluster
+// (gemm_stream.cuh).  Returns 0 when launched, 1 when the shape is not for it.
 int launch_gemm_smallm(const GemmArgs& args, cudaStream_t s);
 
 // ----- W4A16 GEMM (4-bit weights expanded in shared memory, tcgen05) ----------------------------

@@ -503,7 +503,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor, block: int = SWIGLU_BLO
 
 
 def linear_relu_squared(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """``max(x W^T, 0)^2``, the activation inside the GEMM where its kernel has it (up to 8 rows, more than 256)."""
+    """``max(x W^T, 0)^2``, the activation inside the GEMM for up to 8 rows and for more than 256, in place behind it in between."""
     x2 = _2d(x)
     if use_kernels(x) and _gemm_shape_ok(x2, weight):
         if x2.stride(-1) != 1 or (x2.stride(0) * x2.element_size()) % 16:
