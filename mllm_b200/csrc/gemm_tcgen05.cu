@@ -1117,19 +1117,32 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
     int tr, tc;
     constexpr int kOutCols = kGated<SWIGLU> ? kPairBN / 2 : kPairBN;
     const int n_out = kGated<SWIGLU> ? p.n / 2 : p.n;
+    float* col_scale = reinterpret_cast<float*>(epi_staging + ew * (32 * kStageRowBytes));     // of this warp; 8-bit only
     for (int idx = 0; ok && get_tile(idx, tr, tc); ++idx) {
       const int acc = idx & 1;
       const uint32_t acc_phase = (idx >> 1) & 1;
+      const int64_t row = static_cast<int64_t>(tr) * 2 * kBM + static_cast<int64_t>(rank) * kBM + row_in_tile;
+      const bool row_ok = row < p.m;
+      const int64_t col0 = static_cast<int64_t>(tc) * kOutCols;
+      float sa = 1.f;
+      if (p.is_int8) {
+        // The tile's scales come while its products are formed, the weights' by way of shared memory.  Loaded where they are used, one
+        // by one between two stores, they held a tile's end up for 15 us, twice as long as the products of k = 2048 take: 2048 rows of
+        // 12288 x 2048 89.0 us and now 52.5, of 4096 x 2048 32.2 and 20.0, of 12288 x 8192 150.6 and 140.7
+        if (row_ok) sa = p.a_scale[row];
+        if (p.rs_tp == 0) {
+          __syncwarp();        // every lane has used the scales of the tile before
+#pragma unroll
+          for (int i = 0; i < kPairBN / 32; ++i) col_scale[i * 32 + lane] = p.b_scale[static_cast<int64_t>(tc) * kPairBN + i * 32 + lane];
+          __syncwarp();
+        }
+      }
       if (*abort_flag || !mbar_wait(&acc_full[acc], acc_phase, abort_flag)) {
         ok = false;
         break;
       }
       tc_fence_after_sync();
       const uint32_t t_base = tmem_base + (static_cast<uint32_t>(ew * 32) << 16) + acc * kPairBN;
-      const int64_t row = static_cast<int64_t>(tr) * 2 * kBM + static_cast<int64_t>(rank) * kBM + row_in_tile;
-      const bool row_ok = row < p.m;
-      const int64_t col0 = static_cast<int64_t>(tc) * kOutCols;
-      const float sa = (p.is_int8 && row_ok) ? p.a_scale[row] : 1.f;
       if constexpr (!kGated<SWIGLU>) {
         if (p.rs_tp > 0) {
           // reduce-scatter: 64 output columns at a time are rounded, parked in shared memory and written so that
@@ -1187,60 +1200,67 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
           continue;
         }
       }
+      auto store_tile = [&](auto int8_tag) {
+        constexpr bool kInt8 = decltype(int8_tag)::value;
 #pragma unroll 1
-      for (int c = 0; c < kOutCols; c += 32) {
-        uint32_t r0[32], r1[32];
-        tmem_ld_32x32(t_base + c, r0);
-        if constexpr (kGated<SWIGLU>) tmem_ld_32x32(t_base + kPairBN / 2 + c, r1);
-        tmem_ld_wait();
-        if (!row_ok) continue;
+        for (int c = 0; c < kOutCols; c += 32) {
+          uint32_t r0[32], r1[32];
+          tmem_ld_32x32(t_base + c, r0);
+          if constexpr (kGated<SWIGLU>) tmem_ld_32x32(t_base + kPairBN / 2 + c, r1);
+          tmem_ld_wait();
+          if (!row_ok) continue;
 #pragma unroll
-        for (int v8 = 0; v8 < 4; ++v8) {
-          const int64_t col = col0 + c + v8 * 8;
-          if (col >= n_out) break;
-          float f[8], xb[8], ub[8];
-          load_gate_bias8<SWIGLU>(p, static_cast<int64_t>(tc) * kPairBN + c + v8 * 8, xb, ub);
+          for (int v8 = 0; v8 < 4; ++v8) {
+            const int64_t col = col0 + c + v8 * 8;
+            if (col >= n_out) break;
+            float f[8], xb[8], ub[8];
+            load_gate_bias8<SWIGLU>(p, static_cast<int64_t>(tc) * kPairBN + c + v8 * 8, xb, ub);
 #pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            float x = acc_to_float(r0[v8 * 8 + j], p.is_int8);
-            if constexpr (kGated<SWIGLU>) {
-              float u = acc_to_float(r1[v8 * 8 + j], p.is_int8);
-              if (p.is_int8) {
-                x *= sa * p.b_scale[tc * kPairBN + c + v8 * 8 + j];
-                u *= sa * p.b_scale[tc * kPairBN + kPairBN / 2 + c + v8 * 8 + j];
-              }
-              x = gated_unit<SWIGLU>(p, x, u, xb[j], ub[j]);
-            } else {
-              if (p.is_int8) x *= sa * p.b_scale[col + j];
-              if (p.bias != nullptr) x += load_out1(p.bias, col + j, p.out_f16);
-              x = plain_act<SWIGLU>(x);
-            }
-            f[j] = x;
-          }
-          if (!kGated<SWIGLU> && p.residual != nullptr) {
-            const uint4 rv = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.residual) +
-                                                             row * p.ld_res + col);
-            const uint32_t* ru = reinterpret_cast<const uint32_t*>(&rv);
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              float2 q;
-              if (p.out_f16) {
-                q = __half22float2(*reinterpret_cast<const __half2*>(&ru[j]));
+            for (int j = 0; j < 8; ++j) {
+              float x = acc_to_float(r0[v8 * 8 + j], kInt8);
+              if constexpr (kGated<SWIGLU>) {
+                float u = acc_to_float(r1[v8 * 8 + j], kInt8);
+                if constexpr (kInt8) {
+                  x *= sa * col_scale[c + v8 * 8 + j];
+                  u *= sa * col_scale[kPairBN / 2 + c + v8 * 8 + j];
+                }
+                x = gated_unit<SWIGLU>(p, x, u, xb[j], ub[j]);
               } else {
-                q = unpack_bf16x2(ru[j]);
+                if constexpr (kInt8) x *= sa * col_scale[c + v8 * 8 + j];
+                if (p.bias != nullptr) x += load_out1(p.bias, col + j, p.out_f16);
+                x = plain_act<SWIGLU>(x);
               }
-              f[2 * j] += q.x;
-              f[2 * j + 1] += q.y;
+              f[j] = x;
             }
+            if (!kGated<SWIGLU> && p.residual != nullptr) {
+              const uint4 rv = *reinterpret_cast<const uint4*>(static_cast<const uint16_t*>(p.residual) +
+                                                               row * p.ld_res + col);
+              const uint32_t* ru = reinterpret_cast<const uint32_t*>(&rv);
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                float2 q;
+                if (p.out_f16) {
+                  q = __half22float2(*reinterpret_cast<const __half2*>(&ru[j]));
+                } else {
+                  q = unpack_bf16x2(ru[j]);
+                }
+                f[2 * j] += q.x;
+                f[2 * j + 1] += q.y;
+              }
+            }
+            uint4 o;
+            o.x = pack_out2(f[0], f[1], p.out_f16);
+            o.y = pack_out2(f[2], f[3], p.out_f16);
+            o.z = pack_out2(f[4], f[5], p.out_f16);
+            o.w = pack_out2(f[6], f[7], p.out_f16);
+            *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + row * p.ldc + col) = o;
           }
-          uint4 o;
-          o.x = pack_out2(f[0], f[1], p.out_f16);
-          o.y = pack_out2(f[2], f[3], p.out_f16);
-          o.z = pack_out2(f[4], f[5], p.out_f16);
-          o.w = pack_out2(f[6], f[7], p.out_f16);
-          *reinterpret_cast<uint4*>(static_cast<uint16_t*>(p.out) + row * p.ldc + col) = o;
         }
-      }
+      };
+      if (p.is_int8)
+        store_tile(std::true_type{});
+      else
+        store_tile(std::false_type{});
       tc_fence_before_sync();
       mbar_arrive_cluster(mapa_smem(smem_u32(&acc_empty[acc]), 0));
     }
