@@ -519,47 +519,80 @@ __device__ __forceinline__ void tma_gather4(void* smem_dst, const CUtensorMap* m
 }
 
 // ---------------------------------------------------------------------------------------------
-// Prefill kernel, warp-specialised.  A CTA owns one request, one KV head and TWO tiles of 128 rows (a row is a
-// (query token, query head of the GQA group) pair, as above), so every K/V tile that reaches shared memory
-// serves both; KV tiles hold 128 tokens.  The CTA's roles meet only at mbarriers:
-//   warps 0-3  softmax of row tile A      warps 4-7  softmax of row tile B
-//   warp  8    producer: moves rows by slot with the TMA engine (2 KB boxes over runs of 16 consecutive slots, else
-//              gather4 by row index) into a two-slot K ring and a single V slot
-//   warp  9    one thread issues the MMAs.  Tensor memory holds S_A, S_B (128 columns each) and O_A, O_B.
-// A softmax thread pulls its whole S row (128 scores) into registers with four tcgen05.ld and releases the S
-// buffer at once, so the scores of tile t+1 are computed while the exponentials of tile t are; P*V of tile t
-// runs under the softmax of tile t+1.  K is fetched two tiles ahead, V one.  The running maximum and the row
-// sum are kept in several independent chains (a single chain of 128 dependent operations would cost more than
-// the exponentials).  Tiles that need no causal / window mask and no soft cap take one FMA and one exponential
-// per score.
+// Prefill kernel, warp-specialised.  A CTA owns one request, one KV head and a tile of 128 rows (a row is a (query token, query head of
+// the GQA group) pair, as above); KV tiles hold 128 tokens.  What bounds it is the exponentials (16 a cycle and SM: 1024 cycles per
+// tile) and the tensor pipe (1024 as well), and beside them a chain that no tile can leave: scores, maximum, exponentials, product, next
+// scores.  So two CTAs share an SM and each works while the other waits, be it inside a tile, at its start (table, copies, first
+// scores) or at its end (rows to memory):
+//   warps 0-3  softmax, a thread per row
+//   warp  4    producer: moves rows by slot with the TMA engine (2 KB boxes over runs of 16 consecutive slots, else gather4 by row
+//              index) into five slots of 16 KB: half a K tile (64 features) or half a V tile (64 tokens) each
+//   warp  5    one thread issues the MMAs
+// Tensor memory of a CTA (256 columns): S, whose first 64 columns the probabilities overwrite, and O.  P is the left operand from
+// there: nothing passes through shared memory, and the product of its first half runs under the exponentials of the second.  S of the
+// next tile is queued behind P V, so a full S barrier says that O is complete too.  Scale and sums take two columns per
+// instruction, the maximum three scores; a masked tile's columns that no row of the warp sees cost nothing.
+// Before, one CTA per SM with two row tiles that shared K and V and kept P in shared memory: 1 x 128 tokens (16 query heads, 8 kv heads)
+// 11.6 us, now 7.9; 1 x 500 18.1, 14.2; 2 x 517 (32, 8) 21.8, 21.1; 8 x 2048 464, 448.  A tile takes 4400 - 5700 cycles, two side by
+// side: 2100 - 2500 from the last probabilities to the next scores (the product's second half, the scores, two handovers), 500 for the
+// maximum, 1600 - 2400 for the exponentials, which two CTAs share.
 // ---------------------------------------------------------------------------------------------
-constexpr int kPfThreads = 320;
+constexpr int kPfThreads = 256;
 constexpr int kPfTile = 128;                    // KV tokens per tile
-constexpr int kPfHalf = 128 * 128;              // 16 KB: 128 rows of one 128-byte swizzle span
-constexpr int kPfTileBytes = 2 * kPfHalf;       // 32 KB: a Q tile, a K or V tile, or one group's P tile
-constexpr int kPfSmem = (2 + 2 + 3) * kPfTileBytes + 1024 + 256;
+constexpr int kPfSlot = 128 * 128;              // 16 KB
+constexpr int kPfSlots = 5;
+constexpr int kPfQBytes = kRows * kD * 2;       // 32 KB; at the end the output rows
+constexpr int kPfHalf = kRows * 128;            // of Q: 64 features
+constexpr int kPfSmem = kPfQBytes + kPfSlots * kPfSlot + 1024;    // 113 KB: two CTAs per SM
+constexpr int kPfSoftmaxRegs = 192, kPfOtherRegs = 56;            // of the 128 x 256 that a CTA is launched with
+static_assert(128 * (kPfSoftmaxRegs + kPfOtherRegs) <= kPfThreads * 124, "register split");
 
-__global__ void __launch_bounds__(kPfThreads, 1)
+__device__ __forceinline__ uint64_t pair_of(float a, float b) {
+  uint64_t r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+  return r;
+}
+__device__ __forceinline__ float2 halves_of(uint64_t v) {
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(v));
+  return r;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+__device__ __forceinline__ uint64_t add2(uint64_t a, uint64_t b) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ float max3(float a, float b, float c) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(a), "f"(b), "f"(c));
+  return r;
+}
+__device__ __forceinline__ float ex2(float x) {       // as fast_exp2, for the compiler to move
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+
+__global__ void __launch_bounds__(kPfThreads, 2)
 attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v,
                        const __grid_constant__ CUtensorMap tm_k_run, const __grid_constant__ CUtensorMap tm_v_run,
                        const AttnParams p) {
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  uint8_t* sQ = smem;                             // two row tiles
-  uint8_t* sP = sQ + 2 * kPfTileBytes;            // two row tiles of probabilities
-  uint8_t* sK = sP + 2 * kPfTileBytes;            // two K tiles
-  uint8_t* sV = sK + 2 * kPfTileBytes;            // one V tile
-  uint64_t* bars = reinterpret_cast<uint64_t*>(sV + kPfTileBytes);
-  uint64_t* k_full = bars;             // [2] TMA transaction bytes
-  uint64_t* k_empty = bars + 2;        // [2] tcgen05.commit
-  uint64_t* v_full = bars + 4;         // TMA transaction bytes
-  uint64_t* v_empty = bars + 5;        // tcgen05.commit
-  uint64_t* s_full = bars + 6;         // [2] tcgen05.commit: scores of a group are in tensor memory
-  uint64_t* s_free = bars + 8;         // [2] 128 threads: the group holds its scores in registers
-  uint64_t* p_full = bars + 10;        // [2] 128 threads: the group has written P (and rescaled O)
-  uint64_t* o_done = bars + 12;        // [2] tcgen05.commit: the group's P*V has finished
-  uint64_t* q_full = bars + 14;        // 256 threads: both Q tiles are in shared memory
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(bars + 15);
+  extern __shared__ __align__(1024) uint8_t pf_smem[];
+  uint8_t* sQ = pf_smem;
+  uint8_t* ring = sQ + kPfQBytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(ring + kPfSlots * kPfSlot);
+  uint64_t* full = bars;                    // [slot] TMA transaction bytes
+  uint64_t* empty = full + kPfSlots;        // [slot] tcgen05.commit
+  uint64_t* s_full = empty + kPfSlots;      // tcgen05.commit: scores of a tile, and O of the tiles before
+  uint64_t* p_full = s_full + 1;            // [half] 128 threads: P of 64 tokens is in tensor memory (and O rescaled)
+  uint64_t* o_done = p_full + 2;            // tcgen05.commit: the last product
+  uint64_t* q_full = o_done + 1;            // 128 threads
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(q_full + 1);
   int* fail_flag = reinterpret_cast<int*>(tmem_holder + 1);
 
   const int tid = threadIdx.x;
@@ -575,25 +608,27 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
   const int seq_len = p.seq_lens[b];
   const int prefix = p.prefix_lens[b];
   const int q_len = seq_len - prefix;
-  const int q0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * 2 * tpt;   // long rows first
+  const int q0 = (static_cast<int>(gridDim.x) - 1 - static_cast<int>(blockIdx.x)) * tpt;   // long rows first
   if (q0 >= q_len) return;
+  if ((smem_u32(pf_smem) & 1023) != 0) {         // the swizzle counts from 1 KB boundaries
+    if (tid == 0 && p.status != nullptr) atomicExch(p.status, kStatusPipelineTimeout);
+    return;
+  }
   const int q_row0 = p.q_start[b];
   const int kv_begin = p.non_causal ? 0 : first_key(p, prefix + q0) / kPfTile * kPfTile;
-  const int kv_end = p.non_causal ? seq_len : min(seq_len, prefix + min(q_len, q0 + 2 * tpt));
+  const int kv_end = p.non_causal ? seq_len : min(seq_len, prefix + min(q_len, q0 + tpt));
   const int n_tiles = (kv_end - kv_begin + kPfTile - 1) / kPfTile;   // >= 1: the tile's first row sees itself
 
   if (tid == 0) {
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(&k_full[i], 1);
-      mbar_init(&k_empty[i], 1);
-      mbar_init(&s_full[i], 1);
-      mbar_init(&s_free[i], 128);
-      mbar_init(&p_full[i], 128);
-      mbar_init(&o_done[i], 1);
+    for (int i = 0; i < kPfSlots; ++i) {
+      mbar_init(&full[i], 1);
+      mbar_init(&empty[i], 1);
     }
-    mbar_init(v_full, 1);
-    mbar_init(v_empty, 1);
-    mbar_init(q_full, 256);
+    mbar_init(s_full, 1);
+    mbar_init(&p_full[0], 128);
+    mbar_init(&p_full[1], 128);
+    mbar_init(o_done, 1);
+    mbar_init(q_full, 128);
     *fail_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tm_k);
@@ -601,159 +636,167 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     tma_prefetch_desc(&tm_k_run);
     tma_prefetch_desc(&tm_v_run);
   }
-  __syncthreads();
-  if (warp == 9) {
-    tmem_alloc(tmem_holder, 512);
+  if (warp == 5) {
+    tmem_alloc(tmem_holder, 256);
     tmem_relinquish();
   }
   tc_fence_before_sync();
   __syncthreads();
   tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_holder;
+  const uint32_t tmem_s0 = tmem_base, tmem_o0 = tmem_base + 128;
+  // behind the allocation: a CTA of the next kernel that took the columns first would hold them until this kernel ends
+  pdl_launch_dependents();
 
-  if (warp == 8) {
-    // =============================== producer warp ===============================
-    // Order of the copies: K0, K1, V0, K2, V1, K3, V2, ...  (K two tiles ahead of the tile being multiplied, V one)
-    const int* rtt = p.req_to_token + static_cast<int64_t>(req) * p.rtt_stride;
-    bool ok_all = true, bad = false;
-    // lane = four consecutive tokens; a quad = 16 tokens, one 2 KB box per 64-feature half when their slots
-    // are consecutive
-    const int grp = lane >> 2, sub = lane & 3;
-    auto load_tile = [&](int t, bool is_v) {
-      int cur[4];
+  if (warp >= 4) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kPfOtherRegs));
+    if (warp == 4) {
+      // =============================== producer warp ===============================
+      const int* rtt = p.req_to_token + static_cast<int64_t>(req) * p.rtt_stride;
+      bool ok_all = true, bad = false;
+      // lane = four consecutive tokens; a quad = 16 tokens, one 2 KB box per 64-feature half when their slots
+      // are consecutive
+      const int grp = lane >> 2, sub = lane & 3;
+      int next[4];
+      auto look_up = [&](int t) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int tk = min(kv_begin + t * kPfTile + grp * 16 + sub * 4 + j, kv_end - 1);
-        cur[j] = __ldg(rtt + tk);
-        if (cur[j] < 0 || cur[j] >= p.num_slots) {
-          bad = true;
-          cur[j] = 0;
+        for (int j = 0; j < 4; ++j) next[j] = __ldg(rtt + min(kv_begin + t * kPfTile + lane * 4 + j, kv_end - 1));
+      };
+      look_up(0);
+      int slot = 0;
+      uint32_t phase = 0;
+      for (int t = 0; t < n_tiles && ok_all; ++t) {
+        int cur[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          cur[j] = next[j];
+          if (cur[j] < 0 || cur[j] >= p.num_slots) {
+            bad = true;
+            cur[j] = 0;
+          }
         }
-      }
-      bool run = p.kv_runs != 0;
-      const int first = __shfl_sync(0xffffffffu, cur[0], lane & ~3);
+        if (t + 1 < n_tiles) look_up(t + 1);
+        bool run = p.kv_runs != 0;
+        const int first = __shfl_sync(0xffffffffu, cur[0], lane & ~3);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int tk = kv_begin + t * kPfTile + grp * 16 + sub * 4 + j;
-        run = run && (tk >= kv_end || cur[j] == first + sub * 4 + j);   // tokens past the end are masked
-      }
-      const uint32_t votes = __ballot_sync(0xffffffffu, run);
-      run = ((votes >> (lane & ~3)) & 0xFu) == 0xFu && first + 16 <= p.num_slots;
-      uint64_t* full = is_v ? v_full : &k_full[t & 1];
-      uint64_t* empty = is_v ? v_empty : &k_empty[t & 1];
-      const uint32_t ph = is_v ? (t & 1) : ((t >> 1) & 1);
-      if (!mbar_wait(empty, ph ^ 1, fail_flag)) ok_all = false;
-      if (!__all_sync(0xffffffffu, ok_all)) {
-        ok_all = false;
-        return;
-      }
-      if (lane == 0) mbar_arrive_expect_tx(full, kPfTileBytes);
-      __syncwarp();
-      uint8_t* tile = is_v ? sV : sK + (t & 1) * kPfTileBytes;
-      if (run) {
+        for (int j = 0; j < 4; ++j) {
+          const int tk = kv_begin + t * kPfTile + lane * 4 + j;
+          run = run && (tk >= kv_end || cur[j] == first + sub * 4 + j);   // tokens past the end are masked
+        }
+        const uint32_t votes = __ballot_sync(0xffffffffu, run);
+        run = ((votes >> (lane & ~3)) & 0xFu) == 0xFu && first + 16 <= p.num_slots;
         const int row0 = first * p.kv_row_mul + hk * p.kv_row_add;
-        if (sub < 2)
-          tma_load_2d(tile + sub * kPfHalf + grp * 16 * 128, is_v ? &tm_v_run : &tm_k_run, full, sub * 64, row0);
-      } else {
         int rows[4];
 #pragma unroll
         for (int j = 0; j < 4; ++j) rows[j] = cur[j] * p.kv_row_mul + hk * p.kv_row_add;
-        const int off = (grp * 16 + sub * 4) * 128;
-        tma_gather4(tile + off, is_v ? &tm_v : &tm_k, full, 0, rows);
-        tma_gather4(tile + kPfHalf + off, is_v ? &tm_v : &tm_k, full, 64, rows);
+        // K features 0 - 63, 64 - 127, V tokens 0 - 63, 64 - 127
+#pragma unroll 1
+        for (int part = 0; part < 4; ++part) {
+          if (!mbar_wait(&empty[slot], phase ^ 1, fail_flag)) ok_all = false;
+          if (!__all_sync(0xffffffffu, ok_all)) {
+            ok_all = false;
+            break;
+          }
+          if (lane == 0) mbar_arrive_expect_tx(&full[slot], kPfSlot);
+          __syncwarp();
+          uint8_t* to = ring + slot * kPfSlot;
+          if (part < 2) {
+            if (run) {
+              if (sub == 0) tma_load_2d(to + grp * 16 * 128, &tm_k_run, &full[slot], part * 64, row0);
+            } else {
+              tma_gather4(to + lane * 4 * 128, &tm_k, &full[slot], part * 64, rows);
+            }
+          } else if ((grp >> 2) == part - 2) {
+            const int at = lane & 15;                 // four tokens of this half
+            if (run) {
+              if (sub < 2) tma_load_2d(to + sub * (kPfSlot / 2) + (at & ~3) * 4 * 128, &tm_v_run, &full[slot], sub * 64, row0);
+            } else {
+              tma_gather4(to + at * 4 * 128, &tm_v, &full[slot], 0, rows);
+              tma_gather4(to + kPfSlot / 2 + at * 4 * 128, &tm_v, &full[slot], 64, rows);
+            }
+          }
+          if (++slot == kPfSlots) {
+            slot = 0;
+            phase ^= 1;
+          }
+        }
       }
-    };
-    load_tile(0, false);
-    if (ok_all && n_tiles > 1) load_tile(1, false);
-    for (int t = 0; t < n_tiles && ok_all; ++t) {
-      load_tile(t, true);
-      if (ok_all && t + 2 < n_tiles) load_tile(t + 2, false);
-    }
-    if (bad && p.status != nullptr) atomicExch(p.status, kStatusBadIndex);
-    if (!ok_all) *fail_flag = 1;
-  } else if (warp == 9) {
-    // =============================== MMA issuer ===============================
-    if (lane == 0) {
+      if (bad && p.status != nullptr) atomicExch(p.status, kStatusBadIndex);
+      if (!ok_all) *fail_flag = 1;
+    } else if (warp == 5 && lane == 0) {
+      // =============================== MMA issuer ===============================
       bool ok_all = mbar_wait(q_full, 0, fail_flag);
       auto wait_on = [&](uint64_t* bar, uint32_t parity) {
         if (ok_all && !mbar_wait(bar, parity, fail_flag)) ok_all = false;
         if (ok_all) tc_fence_after_sync();
       };
-      auto issue_s = [&](int grp_i, int t) {        // S = Q K^T of group grp_i and KV tile t
-        const uint32_t qa = smem_u32(sQ + grp_i * kPfTileBytes);
-        const uint32_t ka = smem_u32(sK + (t & 1) * kPfTileBytes);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t a_desc = umma_desc_k_sw128(qa + (kk >> 2) * kPfHalf + (kk & 3) * 32);
-          const uint64_t b_desc = umma_desc_k_sw128(ka + (kk >> 2) * kPfHalf + (kk & 3) * 32);
-          umma_f16(tmem_base + grp_i * 128, a_desc, b_desc, p.idesc_s, kk > 0 ? 1u : 0u);
+      // One thread issues all products of the CTA: descriptors are made once, and moved by additions to their address field.
+      const uint64_t q_desc = umma_desc_k_sw128(smem_u32(sQ)), k_desc0 = umma_desc_k_sw128(smem_u32(ring));
+      const uint64_t v_desc0 = umma_desc_mn_sw128(smem_u32(ring), kPfSlot / 2, 1024);
+      const uint32_t idesc_s = p.idesc_s, idesc_o = p.idesc_o;
+      int slot = 0;
+      uint32_t phase = 0;
+      auto done_with = [&]() {
+        umma_commit(&empty[slot]);
+        if (++slot == kPfSlots) {
+          slot = 0;
+          phase ^= 1;
         }
-        umma_commit(&s_full[grp_i]);
       };
-      auto issue_pv = [&](int grp_i, int t) {       // O += P V
-        const uint32_t pa = smem_u32(sP + grp_i * kPfTileBytes);
-        const uint32_t va = smem_u32(sV);
-#pragma unroll
-        for (int kk = 0; kk < 8; ++kk) {
-          const uint64_t a_desc = umma_desc_k_sw128(pa + (kk >> 2) * kPfHalf + (kk & 3) * 32);
-          const uint64_t b_desc = umma_desc_mn_sw128(va + kk * 2048, kPfHalf, 1024);
-          umma_f16(tmem_base + 256 + grp_i * 128, a_desc, b_desc, p.idesc_o, (t > 0 || kk > 0) ? 1u : 0u);
-        }
-        umma_commit(&o_done[grp_i]);
-      };
-      wait_on(&k_full[0], 0);
-      if (ok_all) {
-        issue_s(0, 0);
-        issue_s(1, 0);
-        umma_commit(&k_empty[0]);
-      }
       for (int t = 0; t < n_tiles && ok_all; ++t) {
-        if (t + 1 < n_tiles) {
-          // scores of the next tile, as soon as the groups hold the current ones in registers
-          wait_on(&k_full[(t + 1) & 1], ((t + 1) >> 1) & 1);
-          wait_on(&s_free[0], t & 1);
-          if (ok_all) issue_s(0, t + 1);
-          wait_on(&s_free[1], t & 1);
-          if (ok_all) {
-            issue_s(1, t + 1);
-            umma_commit(&k_empty[(t + 1) & 1]);
-          }
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {        // S = Q K^T, 64 features at a time
+          wait_on(&full[slot], phase);
+          if (!ok_all) break;
+          const uint64_t k_desc = k_desc0 + static_cast<uint32_t>(slot) * (kPfSlot >> 4);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            umma_f16(tmem_s0, q_desc + half * (kPfHalf >> 4) + kk * 2, k_desc + kk * 2, idesc_s, half > 0 || kk > 0 ? 1u : 0u);
+          done_with();
         }
-        wait_on(v_full, t & 1);
-        wait_on(&p_full[0], t & 1);
-        if (ok_all) issue_pv(0, t);
-        wait_on(&p_full[1], t & 1);
-        if (ok_all) {
-          issue_pv(1, t);
-          umma_commit(v_empty);
+        if (!ok_all) break;
+        umma_commit(s_full);
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {        // O += P V, 64 tokens at a time
+          wait_on(&full[slot], phase);
+          wait_on(&p_full[half], t & 1);
+          if (!ok_all) break;
+          const uint64_t v_desc = v_desc0 + static_cast<uint32_t>(slot) * (kPfSlot >> 4);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk)
+            umma_f16_ts(tmem_o0, tmem_s0 + half * 32 + kk * 8, v_desc + kk * (2048 >> 4), idesc_o, t > 0 || half > 0 || kk > 0 ? 1u : 0u);
+          done_with();
         }
       }
+      if (ok_all) umma_commit(o_done);
       if (!ok_all) *fail_flag = 1;
     }
   } else {
-    // =============================== softmax groups ===============================
-    const int grp_i = warp >> 2;                    // 0 = row tile A, 1 = row tile B
-    const int row = tid & 127;
-    const uint32_t lane_base = static_cast<uint32_t>((warp & 3) * 32) << 16;
-    const uint32_t tmem_s = tmem_base + grp_i * 128 + lane_base;
-    const uint32_t tmem_o = tmem_base + 256 + grp_i * 128 + lane_base;
-    const int tile_q0 = q0 + grp_i * tpt;           // first query token of this group's row tile
-    const int row_tok = row / g;
-    const int row_head = hk * g + row % g;
-    const bool row_valid = (row_tok < tpt) && (tile_q0 + row_tok < q_len);
-    const int kv_limit = p.non_causal ? seq_len - 1 : (row_valid ? prefix + tile_q0 + row_tok : prefix + q0);
+    // =============================== softmax ===============================
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kPfSoftmaxRegs));
+    const int row = tid;
+    const uint32_t lane_base = static_cast<uint32_t>(warp * 32) << 16;
+    const uint32_t tmem_s = tmem_s0 + lane_base, tmem_o = tmem_o0 + lane_base;
+    // token of a row: rows are below 128 and g is not above, where 16 bits of the reciprocal give the quotient exactly
+    const uint32_t inv_g = (65536u + g - 1) / g;
+    auto token_of = [&](int r) { return static_cast<int>((r * inv_g) >> 16); };
+    const int row_tok = token_of(row);
+    const bool row_valid = (row_tok < tpt) && (q0 + row_tok < q_len);
+    const int kv_limit = p.non_causal ? seq_len - 1 : (row_valid ? prefix + q0 + row_tok : prefix + q0);
+    const int first_of_row = p.non_causal ? -(1 << 30) : first_key(p, kv_limit);
 
-    // ---- Q tile of this group: 128 rows x 256 B ----
+    // ---- the Q tile: 128 rows x 256 B ----
     {
       const uint16_t* qbase = static_cast<const uint16_t*>(p.q);
-      const uint32_t sq = smem_u32(sQ + grp_i * kPfTileBytes);
-      for (int c = row; c < kRows * 16; c += 128) {
-        const int r = c >> 4, ch = c & 15;
-        const int tok = r / g;
-        const bool ok = (tok < tpt) && (tile_q0 + tok < q_len);
-        const int head = hk * g + r % g;
-        const uint16_t* src = qbase + static_cast<int64_t>(q_row0 + (ok ? tile_q0 + tok : 0)) * p.q_stride +
-                              static_cast<int64_t>(head) * kD + ch * 8;
+      const uint32_t sq = smem_u32(sQ);
+      const int ch = row & 15;
+#pragma unroll 4
+      for (int i = 0; i < 16; ++i) {
+        const int r = (row >> 4) + i * 8;
+        const int tok = token_of(r);
+        const bool ok = (tok < tpt) && (q0 + tok < q_len);
+        const uint16_t* src = qbase + static_cast<int64_t>(q_row0 + (ok ? q0 + tok : 0)) * p.q_stride +
+                              static_cast<int64_t>(hk * g + (ok ? r - tok * g : 0)) * kD + ch * 8;
         cp_async16(sq + swz_off(r, ch, kPfHalf), src, ok);
       }
       cp_async_commit();
@@ -763,13 +806,12 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     }
 
     float m_used = -INFINITY;   // running maximum in use for the exponent (log2 domain)
-    float l_sum = 0.f;
+    uint64_t sums[4] = {0, 0, 0, 0};      // pairs of fp32
     bool ok_all = true;
-    const uint32_t sp = smem_u32(sP + grp_i * kPfTileBytes) + row * 128;
     const bool plain_scores = p.logit_cap <= 0.f;
 
     for (int t = 0; t < n_tiles; ++t) {
-      if (!mbar_wait(&s_full[grp_i], t & 1, fail_flag)) {
+      if (!mbar_wait(s_full, t & 1, fail_flag)) {
         ok_all = false;
         break;
       }
@@ -779,16 +821,16 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       for (int c0 = 0; c0 < kPfTile; c0 += 32)
         tmem_ld_32x32(tmem_s + c0, *reinterpret_cast<uint32_t(*)[32]>(&raw[c0]));
       tmem_ld_wait();
-      tc_fence_before_sync();
-      mbar_arrive(&s_free[grp_i]);   // the scores of the next tile may overwrite the buffer
 
       const int col0 = kv_begin + t * kPfTile;
       const int visible = min(kv_limit, kv_end - 1) - col0;      // columns 0..visible are allowed
-      const int first_vis = p.non_causal ? -(1 << 30) : first_key(p, kv_limit) - col0;
+      const int first_vis = first_of_row - col0;
       const bool fast = __all_sync(0xffffffffu, plain_scores && visible >= kPfTile - 1 && first_vis <= 0);
       float mul = p.scale_log2;
+      int last_vis = kPfTile - 1;           // of the warp
       if (!fast) {
         // masked / capped tile: turn the raw products into final scores in place
+        last_vis = __reduce_max_sync(0xffffffffu, visible);
         if (plain_scores) {
 #pragma unroll
           for (int c = 0; c < kPfTile; ++c) raw[c] = __float_as_uint(__uint_as_float(raw[c]) * p.scale_log2);
@@ -802,16 +844,17 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           raw[c] = (c <= visible && c >= first_vis) ? raw[c] : __float_as_uint(-INFINITY);
         mul = 1.f;
       }
-      float mx[8];
+      float mx[4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) mx[i] = __uint_as_float(raw[i]);
+      for (int i = 0; i < 4; ++i) mx[i] = __uint_as_float(raw[i]);
 #pragma unroll
-      for (int c = 8; c < kPfTile; c += 8) {
+      for (int c = 4; c + 8 <= kPfTile; c += 8) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) mx[i] = fmaxf(mx[i], __uint_as_float(raw[c + i]));
+        for (int i = 0; i < 4; ++i) mx[i] = max3(mx[i], __uint_as_float(raw[c + 2 * i]), __uint_as_float(raw[c + 2 * i + 1]));
       }
-      const float m_tile = fmaxf(fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])),
-                                 fmaxf(fmaxf(mx[4], mx[5]), fmaxf(mx[6], mx[7]))) * mul;   // mul > 0
+#pragma unroll
+      for (int i = 0; i < 4; ++i) mx[i] = fmaxf(mx[i], __uint_as_float(raw[kPfTile - 4 + i]));
+      const float m_tile = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * mul;   // mul > 0
       float factor = 1.f;
       bool need = false;
       if (m_used == -INFINITY) {
@@ -822,65 +865,64 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
         need = true;
       }
       const float m_exp = (m_used == -INFINITY) ? 0.f : m_used;
-      // The group's previous P*V must have finished before P is overwritten and O is rescaled.  It was queued a
-      // whole softmax ago, so this wait is short; taking it here lets the exponentials go to shared memory as
-      // they are computed instead of waiting in 64 registers.
-      if (t > 0) {
-        if (!mbar_wait(&o_done[grp_i], (t - 1) & 1, fail_flag)) {
-          ok_all = false;
-          break;
-        }
-        tc_fence_after_sync();
-      }
-      if (__any_sync(0xffffffffu, need)) {
-        l_sum *= factor;
+      if (__any_sync(0xffffffffu, need)) {      // the products before this tile's scores are complete
+#pragma unroll
+        for (int i = 0; i < 4; ++i) sums[i] = fma2(sums[i], pair_of(factor, factor), 0);
 #pragma unroll 1
-        for (int c = 0; c < kD; c += 32) {
-          uint32_t o[32];
-          tmem_ld_32x32(tmem_o + c, o);
+        for (int c = 0; c < kD; c += 16) {
+          uint32_t o[16];
+          tmem_ld_32x16(tmem_o + c, o);
           tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-          tmem_st_32x32(tmem_o + c, o);
+          for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+          tmem_st_32x16(tmem_o + c, o);
         }
-        tmem_st_wait();
       }
-      // exponentials -> P in the operand layout: two 64-token halves of 128-byte rows, 16-byte chunks swizzled
-      // by the row
-      float ps[4] = {0.f, 0.f, 0.f, 0.f};
+      // exponentials -> P, two tokens to a column
+      const uint64_t mul2 = pair_of(mul, mul), neg2 = pair_of(-m_exp, -m_exp);
 #pragma unroll
-      for (int q16 = 0; q16 < 16; ++q16) {
-        uint32_t w4[4];
+      for (int half = 0; half < 2; ++half) {
+        uint32_t w[32];
 #pragma unroll
-        for (int k4 = 0; k4 < 4; ++k4) {
-          const int i = q16 * 4 + k4;
-          const float p0 = fast_exp2(fmaf(__uint_as_float(raw[2 * i]), mul, -m_exp));
-          const float p1 = fast_exp2(fmaf(__uint_as_float(raw[2 * i + 1]), mul, -m_exp));
-          ps[k4] += p0 + p1;
-          if (p.out_f16) {
-            __half2 h = __floats2half2_rn(p0, p1);
-            w4[k4] = *reinterpret_cast<uint32_t*>(&h);
+        for (int q = 0; q < 4; ++q) {                  // 16 tokens each
+          if (half * 64 + q * 16 > last_vis) {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) w[q * 8 + i] = 0u;
           } else {
-            w4[k4] = pack_bf16x2(p0, p1);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int c = half * 64 + q * 16 + 2 * i;
+              const float2 x = halves_of(fma2(pair_of(__uint_as_float(raw[c]), __uint_as_float(raw[c + 1])), mul2, neg2));
+              const float p0 = ex2(x.x), p1 = ex2(x.y);
+              sums[i & 3] = add2(sums[i & 3], pair_of(p0, p1));
+              if (p.out_f16) {
+                __half2 h = __floats2half2_rn(p0, p1);
+                w[q * 8 + i] = *reinterpret_cast<uint32_t*>(&h);
+              } else {
+                w[q * 8 + i] = pack_bf16x2(p0, p1);
+              }
+            }
           }
         }
-        const uint32_t dst = sp + (q16 >> 3) * kPfHalf + (((q16 & 7) ^ (row & 7)) << 4);
-        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(w4[0]), "r"(w4[1]), "r"(w4[2]), "r"(w4[3])
-                     : "memory");
+        tmem_st_32x32(tmem_s + half * 32, w);
+        tmem_st_wait();
+        tc_fence_before_sync();
+        mbar_arrive(&p_full[half]);
       }
-      l_sum += (ps[0] + ps[1]) + (ps[2] + ps[3]);
-      fence_proxy_async_smem();
-      tc_fence_before_sync();
-      mbar_arrive(&p_full[grp_i]);
     }
-    if (ok_all && !mbar_wait(&o_done[grp_i], (n_tiles - 1) & 1, fail_flag)) ok_all = false;
+    if (ok_all && !mbar_wait(o_done, 0, fail_flag)) ok_all = false;
     tc_fence_after_sync();
     if (!ok_all) *fail_flag = 1;
 
-    // ---- epilogue: normalise, park the group's 128 rows x 256 B in its P buffer (free now), then store them
-    // row by row: 16 lanes cover one output row, and the g rows of a token are adjacent in memory ----
-    if (p.sink != nullptr) l_sum += sink_term(p.sink, hk * g + row % g, m_used);
-    const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
+    // ---- epilogue: normalise, park the 128 rows x 256 B where Q was, then store them row by row: 16 lanes cover one output row, and
+    // the g rows of a token are adjacent in memory ----
+    float l_sum;
+    {
+      const float2 v = halves_of(add2(add2(sums[0], sums[1]), add2(sums[2], sums[3])));
+      l_sum = v.x + v.y;
+    }
+    if (p.sink != nullptr) l_sum += sink_term(p.sink, hk * g + row - row_tok * g, m_used);
+    const float inv_l = l_sum == 0.f ? 0.f : 1.f / l_sum;       // 0: no key to be seen.  A sum that is no number shows
 #pragma unroll 1
     for (int c = 0; c < kD; c += 32) {
       uint32_t o[32];
@@ -901,26 +943,22 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
           }
         }
         const int chunk = (c + i) >> 3;   // 16-byte chunk of the 256-byte row
-        const uint32_t dst = smem_u32(sP + grp_i * kPfTileBytes) + row * 256 + ((chunk ^ (row & 7)) << 4);
+        const uint32_t dst = smem_u32(sQ) + row * 256 + ((chunk ^ (row & 7)) << 4);
         asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(vv[0]), "r"(vv[1]), "r"(vv[2]), "r"(vv[3])
                      : "memory");
       }
     }
-    if (grp_i == 0)
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-    else
-      asm volatile("bar.sync 2, 128;" ::: "memory");
+    asm volatile("bar.sync 1, 128;" ::: "memory");
     if (ok_all) {
-      const int w4 = warp & 3;
       const int chunk = lane & 15;
 #pragma unroll 4
       for (int it = 0; it < 16; ++it) {
-        const int r = it * 8 + w4 * 2 + (lane >> 4);
-        const int tok = r / g;
-        if (tok < tpt && tile_q0 + tok < q_len) {
-          const uint4 v = *reinterpret_cast<const uint4*>(sP + grp_i * kPfTileBytes + r * 256 + ((chunk ^ (r & 7)) << 4));
+        const int r = it * 8 + warp * 2 + (lane >> 4);
+        const int tok = token_of(r);
+        if (tok < tpt && q0 + tok < q_len) {
+          const uint4 v = *reinterpret_cast<const uint4*>(sQ + r * 256 + ((chunk ^ (r & 7)) << 4));
           uint16_t* dst = static_cast<uint16_t*>(p.out) +
-                          static_cast<int64_t>(q_row0 + tile_q0 + tok) * p.out_stride + (hk * g + r % g) * kD + chunk * 8;
+                          static_cast<int64_t>(q_row0 + q0 + tok) * p.out_stride + (hk * g + r - tok * g) * kD + chunk * 8;
           *reinterpret_cast<uint4*>(dst) = v;
         }
       }
@@ -935,9 +973,9 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
     __syncthreads();
   }
-  if (warp == 9) {
+  if (warp == 5) {
     tc_fence_after_sync();
-    tmem_dealloc(tmem_base, 512);
+    tmem_dealloc(tmem_base, 256);
   }
 }
 
@@ -1014,8 +1052,17 @@ int launch_prefill_ws(AttnParams p, const AttnArgs& a, cudaStream_t s) {
   const uint32_t fmt = a.dt == kF16 ? 0u : 1u;
   p.idesc_s = umma_idesc(kRows, kPfTile, 1, fmt, fmt, 0, 0);
   p.idesc_o = umma_idesc(kRows, kD, 1, fmt, fmt, 0, 1);
-  const int q_tiles = (a.max_q_len + 2 * p.tokens_per_tile - 1) / (2 * p.tokens_per_tile);
+  const int q_tiles = (a.max_q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
   if (q_tiles <= 0) return 0;
+  {
+    // the softmax warps take registers that the others give back: together no more than the kernel is launched with
+    static const int regs = [] {
+      cudaFuncAttributes at{};
+      return cudaFuncGetAttributes(&at, reinterpret_cast<const void*>(attn_prefill_ws_kernel)) == cudaSuccess ? at.numRegs : 0;
+    }();
+    if (regs * kPfThreads < 128 * (kPfSoftmaxRegs + kPfOtherRegs)) return -3;
+  }
+  ensure_max_carveout(reinterpret_cast<const void*>(attn_prefill_ws_kernel));
   const cudaError_t err = launch_pdl(attn_prefill_ws_kernel, dim3(q_tiles, a.hkv, a.batch), dim3(kPfThreads), kPfSmem, s,
                                      tm_k, tm_v, tm_k_run, tm_v_run, p);
   note_launch();

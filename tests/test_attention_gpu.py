@@ -228,3 +228,29 @@ def test_decode_sliding_window_and_soft_cap(window, cap, seq_lens):
     want = ref.attention_decode(s["q"], s["kc"], s["vc"], s["rtt"], s["req"], s["seq"], scale, window=window or None,
                                 logit_cap=cap)
     assert _err(got, want) < 3e-2
+
+
+@pytest.mark.parametrize("hq,hkv", [(12, 2), (7, 1), (5, 5), (64, 1)])
+@pytest.mark.parametrize("seq_lens,prefix_lens", [([21, 22, 43], [0, 0, 1]), ([128, 129, 257], [0, 127, 128]), ([150], [20])])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_prefill_row_tiles(hq, hkv, seq_lens, prefix_lens, dtype):
+    """Groups that do not divide a tile's 128 rows, tiles that end inside a request, keys on both sides of a tile's edge."""
+    s = _setup(seq_lens, prefix_lens, hq, hkv, dtype=dtype, seed=hq)
+    got = ops.attention_prefill(s["q"], s["kc"], s["vc"], s["rtt"], s["req"], s["seq"], s["pre"], s["q_start"], D ** -0.5, max_q_len=s["max_q"])
+    ops.check_status()
+    want = ref.attention_prefill(s["q"], s["kc"], s["vc"], s["rtt"], s["req"], s["seq"], s["pre"], s["q_start"], D ** -0.5)
+    assert _err(got, want) < 3e-2
+
+
+def test_prefill_scores_that_are_no_numbers():
+    """A query without a number makes its own row none, and no other."""
+    s = _setup([140, 60], [0, 0], 8, 2, seed=5)
+    want = ops.attention_prefill(s["q"], s["kc"], s["vc"], s["rtt"], s["req"], s["seq"], s["pre"], s["q_start"], D ** -0.5, max_q_len=s["max_q"])
+    q = s["q"].clone()
+    q[70, 3] = float("nan")
+    q[150, 6, 5] = float("inf")
+    got = ops.attention_prefill(q, s["kc"], s["vc"], s["rtt"], s["req"], s["seq"], s["pre"], s["q_start"], D ** -0.5, max_q_len=s["max_q"])
+    ops.check_status()
+    assert got[70, 3].isnan().all() and got[150, 6].isnan().all()
+    got[70, 3], got[150, 6] = want[70, 3], want[150, 6]
+    assert torch.equal(got, want)
