@@ -183,10 +183,10 @@ int64_t gdn_chunk(const Tensor& q, const Tensor& k, const Tensor& v, const Tenso
   c10::cuda::CUDAGuard gd(q.device());
   if (mb200::gdn_prefill_covers(p)) {
     const int longest = static_cast<int>(max_len > 0 ? std::min<int64_t>(max_len, q.size(0)) : q.size(0));
-    const int sms = device_state(q.get_device()).num_sms;
+    int* status = device_state(q.get_device()).status.data_ptr<int>();
     const mb200::GdnPrefillPlan plan = mb200::gdn_prefill_plan(p, longest, workspace);
     Tensor ws = torch::empty({plan.ws_bytes}, state.options().dtype(torch::kUInt8));
-    const int rc = mb200::launch_gdn_prefill(p, ws.data_ptr(), plan, longest, sms, stream_of(q));
+    const int rc = mb200::launch_gdn_prefill(p, ws.data_ptr(), plan, longest, status, stream_of(q));
     TORCH_CHECK(rc == 0, "gdn_chunk: launch failed (code ", rc, ")");
     return 0;
   }

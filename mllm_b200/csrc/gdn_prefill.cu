@@ -8,15 +8,14 @@
 //   * gdn_prepare_kernel takes every (chunk, head) by itself, all of them side by side: unit norms, decays, K K^T and Q K^T, the
 //     inverse T (16 x 16 blocks by substitution, joined by products, in fp32), and from it -W = -T diag(beta exp(G)) K and
 //     U0 = T diag(beta) V.
-//   * gdn_scan_kernel walks the chunks with the state in its accumulators: U = U0 - W S0, then O and the next S; two barriers a
-//     chunk, the next chunk's operands on their way meanwhile.  A CTA owns a block of the value features, whose columns of the
+//   * gdn_scan_kernel walks the chunks with the state in registers.  A CTA owns a block of 64 value features, whose columns of the
 //     state never mix.
-// Products are warp-level MMAs.  K, Q and V are bf16 and enter as they are; every fp32 operand (T, W, the state, U, the decayed
-// scores) enters as two bf16 terms, its rounding and the remainder: 16 bits of it, against the 11 of a tf32 operand, for as many
-// instructions.  Sums and the state are fp32.
+// Products enter the tensor cores in 16 bits.  K, Q and V are bf16 and enter as they are; every fp32 operand (T, W, the state, U, the
+// decayed scores) enters as two bf16 terms, its rounding and the remainder: 16 bits of it, against the 11 of a tf32 operand, for as many
+// instructions.  Sums and the state are fp32.  The first kernel's products are warp-level MMAs, chained through element-wise steps; the
+// scan's are tcgen05 with accumulators in tensor memory: what bounds the scan is the chain from one chunk's state to the next, and of a
+// chunk's 2032 warp-level MMAs, their fragment loads and the addresses of its copies it made 12300 cycles.
 //
-// Measured (16 heads of 128 x 128; one kernel with tf32 operands, then these two): 4 x 2000 tokens
-// 1274 -> 433 us, 1 x 2048 582 -> 126, 8 x 2048 1612 -> 732, 32 x 1024 2849 -> 1388; the state's error against 64 bits 2e-4 -> 4e-6.
 #include <algorithm>
 
 #include "common.cuh"
@@ -30,31 +29,36 @@ constexpr int kC = 64;                 // tokens of a chunk
 constexpr int kD = 128;                // key features, zero-padded
 constexpr int kThreads = 256;
 constexpr int kLd = kC + 4;            // row stride (floats) of chunk x chunk matrices
-constexpr int kRow = kD * 2;           // bytes of a K, Q, V or W row in shared memory
-constexpr int kTileBytes = kC * kRow;  // 16 KB
-constexpr int kPBytes = kC * kC * 2;   // 8 KB
+constexpr int kXLd = 18;               // of 16 x 16 blocks
+constexpr int kTileBytes = kC * kD * 2;  // 16 KB: a chunk of K, Q or V, two planes
 constexpr int kScalars = 160;          // floats: exp(G) / |q|, exp(G_C - G) / |k|, exp(G_C)
+constexpr int kBV = 64;                // value features of a scan CTA
+constexpr int kPlane = kC * 128;       // 8 KB: 64 rows of 64 16-bit values, one swizzle span each
 
-// what the first kernel leaves for a (chunk, head)
+// What the first kernel leaves for a (chunk, head): the scan's operands as they lie in its shared memory (planes of 64 rows with the
+// 128-byte swizzle, so that one bulk copy moves them all), the scalars behind them, and U0 in the order in which the scan's threads
+// take it, [block of 64 value features][four features][token][4].
 struct Slot {
-  static constexpr int64_t kW = 0, kP = 2 * kTileBytes, kScal = kP + 2 * kPBytes, kU = kScal + kScalars * 4;
+  // for each half of the key features W (rounding), Q, W (remainder): rows 0 - 127 of the left operand are W and Q together
+  static constexpr int kWhi = 0, kQ = kPlane, kWlo = 2 * kPlane, kHalf = 3 * kPlane;
+  static constexpr int kK = 2 * kHalf, kP = kK + 2 * kPlane;       // K: two halves; decayed scores: rounding, remainder
+  static constexpr int kScal = kP + 2 * kPlane, kBulk = kScal + kScalars * 4;
+  static constexpr int64_t kU = kBulk;
 };
-__host__ __device__ inline int64_t slot_bytes(int dv) { return Slot::kU + static_cast<int64_t>(kC) * ((dv + 15) / 16 * 16) * 4; }
+static_assert(Slot::kBulk % 16 == 0, "bulk copies move multiples of 16 bytes");
+__host__ __device__ inline int value_blocks(int dv) { return (dv + kBV - 1) / kBV; }
+__host__ __device__ inline int64_t slot_bytes(int dv) { return Slot::kU + static_cast<int64_t>(value_blocks(dv)) * kBV * kC * 4; }
 
 struct PrefillParams {
   GdnRuleParams r;
   uint8_t* ws;
+  int* status;
   int chunk0, span;      // chunks chunk0 .. chunk0 + span of every request are in the workspace
+  int wide;              // state and outputs may be moved 16 bytes at a time
 };
 
-__device__ __forceinline__ uint32_t at128(int row, int chunk) { return row * kRow + ((chunk ^ (row & 7)) << 4); }   // 256-byte rows
-__device__ __forceinline__ uint32_t at64(int row, int chunk) { return row * (kC * 2) + ((chunk ^ (row & 7)) << 4); }  // 128-byte rows
-// rows of BV 16-bit values: eight rows of a fragment load fall on different 16-byte groups of the banks
-template <int BV>
-__device__ __forceinline__ uint32_t at_v(int row, int chunk) {
-  constexpr int kCh = BV / 8, kPer = 8 / kCh;
-  return row * (BV * 2) + ((chunk ^ ((row / kPer) & (kCh - 1))) << 4);
-}
+// 16-byte piece of a row of 128 values in two planes: eight neighbouring rows lie in different banks
+__device__ __forceinline__ uint32_t at128(int row, int chunk) { return (chunk >> 3) * kPlane + row * 128 + (((chunk & 7) ^ (row & 7)) << 4); }
 // (a, b) as the pair of their roundings and the pair of the remainders
 __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t& lo) {
   hi = pack_bf16x2(a, b);
@@ -62,6 +66,15 @@ __device__ __forceinline__ void split2(float a, float b, uint32_t& hi, uint32_t&
   lo = pack_bf16x2(a - r.x, b - r.y);
 }
 using BF = __nv_bfloat16;
+
+// fragments of four 8 x 8 tiles to their rows, whose addresses the lanes give (8 lanes a tile)
+__device__ __forceinline__ void stsm4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void bulk_store(void* dst, uint32_t src, uint32_t bytes) {
+  asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(src), "r"(bytes) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 
 __global__ void __launch_bounds__(kThreads, 2) gdn_prepare_kernel(const PrefillParams pp) {
   const GdnRuleParams& p = pp.r;
@@ -72,12 +85,15 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prepare_kernel(const PrefillP
   uint8_t* sV = sQ + kTileBytes;
   float* sA = reinterpret_cast<float*>(sV + kTileBytes);
   float* sT = sA + kC * kLd;
-  float* sX = sT + kC * kLd;             // [3][16][17]
-  float* sG = sX + 3 * 16 * 17;
+  float* sX = sT + kC * kLd;             // [3][16][kXLd]
+  float* sG = sX + 3 * 16 * kXLd;
   float* sB = sG + kC;
   float* sRk = sB + kC;
   float* sRq = sRk + kC;
   float* sE = sRq + kC;
+  uint8_t* sP = reinterpret_cast<uint8_t*>(sE + kC);       // the decayed scores, two planes
+  // -W, planes as they lie in the slot: where A was, and Q
+  auto w_plane = [&](int half) { return half == 0 ? reinterpret_cast<uint8_t*>(sA) : sQ; };
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   const int h = blockIdx.y, b = blockIdx.z;
@@ -116,23 +132,36 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prepare_kernel(const PrefillP
     sB[tid] = tid < nv ? p.beta[at] : 0.f;
   }
   cp_wait<0>();
+  fence_proxy_async_smem();
   __syncthreads();
 
-  // ---- norms of the rows (a warp takes eight), running sum of the log decays ----
+  // ---- Q and K as the scan takes them ----
+  if (tid == 0) {
+    bulk_store(slot + Slot::kK, smem_u32(sK), 2 * kPlane);
+    bulk_store(slot + Slot::kQ, smem_u32(sQ), kPlane);
+    bulk_store(slot + Slot::kHalf + Slot::kQ, smem_u32(sQ) + kPlane, kPlane);
+    bulk_commit();
+  }
+  // ---- norms of the rows, two threads to a row of K or of Q (in an order that keeps their pieces in different banks) ----
   const float qscale = 1.f / sqrtf(static_cast<float>(p.dk));
+  {
+    const int r = (tid >> 1) & (kC - 1), half = tid & 1;
+    const uint8_t* from = tid < 2 * kC ? sK : sQ;
+    float ss = 0.f;
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int r = warp * 8 + i;
-    float s[2];
+    for (int i = 0; i < 8; ++i) {
+      const uint4 v = *reinterpret_cast<const uint4*>(from + at128(r, half * 8 + (i ^ (half * 4))));
+      const uint32_t w[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-    for (int w = 0; w < 2; ++w) {
-      const uint2 v = *reinterpret_cast<const uint2*>((w ? sQ : sK) + at128(r, lane >> 1) + (lane & 1) * 8);
-      const float2 a = unpack_bf16x2(v.x), c = unpack_bf16x2(v.y);
-      s[w] = warp_sum(a.x * a.x + a.y * a.y + c.x * c.x + c.y * c.y);
+      for (int j = 0; j < 4; ++j) {
+        const float2 a = unpack_bf16x2(w[j]);
+        ss = fmaf(a.x, a.x, fmaf(a.y, a.y, ss));
+      }
     }
-    if (lane == 0) {
-      sRk[r] = 1.f / sqrtf(s[0] + 1e-6f);
-      sRq[r] = qscale / sqrtf(s[1] + 1e-6f);
+    ss += __shfl_xor_sync(0xffffffffu, ss, 1);
+    if (half == 0) {
+      if (tid < 2 * kC) sRk[r] = 1.f / sqrtf(ss + 1e-6f);
+      else sRq[r] = qscale / sqrtf(ss + 1e-6f);
     }
   }
   __syncthreads();
@@ -184,10 +213,12 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prepare_kernel(const PrefillP
       }
     }
 #pragma unroll
-    for (int nt = 0; nt < 8; ++nt) {
-      if (nt >= 2 * (ti + 1)) continue;
+    for (int np = 0; np < 4; ++np) {
+      if (np > ti && !is_q) continue;            // (the scores' tiles above the diagonal are written too: zero)
+      uint32_t hi[4], lo[4];
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
+      for (int e = 0; e < 4; ++e) {
+        const int nt = 2 * np + (e >> 1), half = e & 1;
         const int i = ti * 16 + g + half * 8, j = nt * 8 + 2 * t;
         float v[2];
 #pragma unroll
@@ -196,19 +227,22 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prepare_kernel(const PrefillP
           const float f = (is_q ? sRq[i] : sB[i] * sRk[i]) * sRk[j + c];
           v[c] = in ? __expf(sG[i] - sG[j + c]) * (f * acc[nt][half * 2 + c]) : 0.f;
         }
-        if (is_q) {
-          uint32_t hi, lo;
-          split2(v[0], v[1], hi, lo);
-          uint8_t* dst = slot + Slot::kP + i * (kC * 2) + j * 2;
-          *reinterpret_cast<uint32_t*>(dst) = hi;
-          *reinterpret_cast<uint32_t*>(dst + kPBytes) = lo;
-        } else {
-          *reinterpret_cast<float2*>(sA + i * kLd + j) = make_float2(v[0], v[1]);
-        }
+        if (is_q) split2(v[0], v[1], hi[e], lo[e]);
+        else *reinterpret_cast<float2*>(sA + i * kLd + j) = make_float2(v[0], v[1]);
+      }
+      if (is_q) {
+        const uint32_t at = smem_u32(sP) + at128(ti * 16 + (lane & 15), 2 * np + (lane >> 4));
+        stsm4(at, hi[0], hi[1], hi[2], hi[3]);
+        stsm4(at + kPlane, lo[0], lo[1], lo[2], lo[3]);
       }
     }
   }
+  fence_proxy_async_smem();
   __syncthreads();
+  if (tid == 0) {
+    bulk_store(slot + Slot::kP, smem_u32(sP), 2 * kPlane);
+    bulk_commit();
+  }
 
   // ---- T = (I + A)^-1: the diagonal blocks by substitution, a thread per column ----
   if (tid < kC) {
@@ -225,23 +259,45 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prepare_kernel(const PrefillP
     for (int i = 0; i < 16; ++i) sT[(blk + i) * kLd + blk + col] = x[i];
   }
   __syncthreads();
-  // ---- the blocks below, diagonal by diagonal: T_ij = -T_ii sum_k A_ik T_kj ----
+  // ---- the blocks below, diagonal by diagonal: T_ij = -T_ii sum_k A_ik T_kj.  Half the threads to a block, two neighbouring columns each,
+  // so that a load serves two to four products (one value at a time the block products were bound by shared memory) ----
   {
-    const int r = tid >> 4, c = tid & 15;
+    const int grp = tid >> 7, r = (tid >> 3) & 15, c = (tid & 7) * 2;
     for (int d = 1; d < 4; ++d) {
-      for (int bi = d; bi < 4; ++bi) {
+      for (int bi = d + grp; bi < 4; bi += 2) {
         const int bj = bi - d;
-        float s = 0.f;
-        for (int m = bj * 16; m < bi * 16; ++m) s = fmaf(sA[(bi * 16 + r) * kLd + m], sT[m * kLd + bj * 16 + c], s);
-        sX[((bi - d) * 16 + r) * 17 + c] = s;
+        float s0 = 0.f, s1 = 0.f;
+        for (int m = bj * 16; m < bi * 16; m += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(sA + (bi * 16 + r) * kLd + m);
+          const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 x = *reinterpret_cast<const float2*>(sT + (m + e) * kLd + bj * 16 + c);
+            s0 = fmaf(av[e], x.x, s0);
+            s1 = fmaf(av[e], x.y, s1);
+          }
+        }
+        *reinterpret_cast<float2*>(sX + (bj * 16 + r) * kXLd + c) = make_float2(s0, s1);
       }
       __syncthreads();
-      for (int bi = d; bi < 4; ++bi) {
-        float s = 0.f;
+      for (int bi = d + grp; bi < 4; bi += 2) {
+        const int bj = bi - d;
+        float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-        for (int m = 0; m < 16; ++m) s = fmaf(sT[(bi * 16 + r) * kLd + bi * 16 + m], sX[((bi - d) * 16 + m) * 17 + c], s);
-        sT[(bi * 16 + r) * kLd + (bi - d) * 16 + c] = -s;
+        for (int m = 0; m < 16; m += 4) {
+          const float4 a = *reinterpret_cast<const float4*>(sT + (bi * 16 + r) * kLd + bi * 16 + m);
+          const float av[4] = {a.x, a.y, a.z, a.w};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const float2 x = *reinterpret_cast<const float2*>(sX + (bj * 16 + m + e) * kXLd + c);
+            s0 = fmaf(av[e], x.x, s0);
+            s1 = fmaf(av[e], x.y, s1);
+          }
+        }
+        *reinterpret_cast<float2*>(sT + (bi * 16 + r) * kLd + bj * 16 + c) = make_float2(-s0, -s1);
       }
+      // the copies have read Q, whose place W takes
+      if (d == 3 && tid == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
       __syncthreads();
     }
   }
@@ -250,7 +306,7 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prepare_kernel(const PrefillP
   {
     const int ti = warp & 3;
     const bool is_u = warp >= 4;
-    const int dv16 = (p.dv + 15) / 16 * 16;
+    const int blocks = value_blocks(p.dv);
     for (int v0 = 0; v0 < p.dv; v0 += kD) {
       if (v0 > 0) {
         __syncthreads();
@@ -287,268 +343,321 @@ __global__ void __launch_bounds__(kThreads, 2) gdn_prepare_kernel(const PrefillP
           }
         }
       }
+      if (is_u) {
 #pragma unroll
-      for (int nt = 0; nt < 16; ++nt) {
+        for (int nt = 0; nt < 16; ++nt) {
 #pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const int row = ti * 16 + g + half * 8, col = nt * 8 + 2 * t;
-          const float a = acc[nt][half * 2], c = acc[nt][half * 2 + 1];
-          if (is_u) {
-            if (v0 + col < dv16)
-              *reinterpret_cast<float2*>(slot + Slot::kU + (static_cast<int64_t>(row) * dv16 + v0 + col) * 4) = make_float2(a, c);
-          } else {
-            uint32_t hi, lo;
-            split2(-a, -c, hi, lo);
-            uint8_t* dst = slot + Slot::kW + row * kRow + col * 2;
-            *reinterpret_cast<uint32_t*>(dst) = hi;
-            *reinterpret_cast<uint32_t*>(dst + kTileBytes) = lo;
+          for (int half = 0; half < 2; ++half) {
+            const int row = ti * 16 + g + half * 8, vc = v0 + nt * 8 + 2 * t, vb = vc / kBV;
+            if (vb < blocks)
+              *reinterpret_cast<float2*>(slot + Slot::kU + (static_cast<int64_t>(vb * (kBV / 4) + (vc % kBV) / 4) * kC + row) * 16 + (vc & 3) * 4) =
+                  make_float2(acc[nt][half * 2], acc[nt][half * 2 + 1]);
           }
+        }
+      } else {
+#pragma unroll
+        for (int np = 0; np < 8; ++np) {
+          uint32_t hi[4], lo[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int nt = 2 * np + (e >> 1), half = e & 1;
+            split2(-acc[nt][half * 2], -acc[nt][half * 2 + 1], hi[e], lo[e]);
+          }
+          const uint32_t at = smem_u32(w_plane(np >> 2)) + at128(ti * 16 + (lane & 15), 2 * (np & 3) + (lane >> 4));
+          stsm4(at, hi[0], hi[1], hi[2], hi[3]);
+          stsm4(at + kPlane, lo[0], lo[1], lo[2], lo[3]);
+        }
+        fence_proxy_async_smem();
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        if (tid == 0) {
+#pragma unroll
+          for (int half = 0; half < 2; ++half) {
+            bulk_store(slot + half * Slot::kHalf + Slot::kWhi, smem_u32(w_plane(half)), kPlane);
+            bulk_store(slot + half * Slot::kHalf + Slot::kWlo, smem_u32(w_plane(half)) + kPlane, kPlane);
+          }
+          bulk_commit();
         }
       }
     }
   }
+  if (tid == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
 }
 
-template <int BV>
-struct ScanCfg {
-  static constexpr int kStage = 4 * kTileBytes + 2 * kPBytes + kScalars * 4;   // W (two terms), Q, K, P (two terms), scalars
-  static constexpr int kS = kD * BV * 2, kU = kC * BV * 2;                     // one term of the state, of U
-  static constexpr int kSmem = 2 * kStage + 2 * kS + 4 * kU + 128;
-  static_assert(kSmem <= 232448, "shared memory");
-};
+// ---------------------------------------------------------------------------------------------------------------------
+// The scan.  Warps 0 - 15 hold the state (a thread has 16 value features of one key feature) and form the operands; one thread of warp
+// 16 moves the chunks and issues the products:
+//   D1 = [W; Q] [S_hi | S_lo] and D2 = W_lo S_hi (rows 0 - 63 of D1 and D2 make W S, rows 64 - 127 of D1 are Q S),
+//   dS = K^T [U'_hi | U'_lo],   D3 = P_hi [U_hi | U_lo] + P_lo U_hi  (rows 64 - 127; what stands in the other rows is not read).
+// The two terms of a right operand are side by side, so that one instruction takes both.  What bounds it is the chain of a chunk: state ->
+// operands -> D1, D2 (1000 cycles) -> U -> operands -> dS (300) -> state, with four handovers; D3, the outputs, the next chunk's copy
+// and U0 lie beside it.  (Eight warps with 32 value features a thread: the element-wise parts of the chain took twice as long, and a
+// chunk 7500 cycles.)
+// Tensor memory: D1 0 - 127, D2 128 - 191, dS 256 - 383, D3 384 - 511.
+// ---------------------------------------------------------------------------------------------------------------------
+constexpr int kScanWarps = 16, kScanCols = kBV / (kScanWarps / 4), kScanThreads = 32 * (kScanWarps + 1);
+constexpr int kOperand = kD * 128;                                   // 16 KB: one term of the state, [128][64]
+constexpr int kScanSmem = 1024 + 2 * Slot::kScal + 2 * kOperand + 4 * kPlane + 2 * kScalars * 4 + 256;
+static_assert(kScanSmem <= 232448, "shared memory");
 
-template <int BV>
-__global__ void __launch_bounds__(kThreads, 1) gdn_scan_kernel(const PrefillParams pp) {
-  using C = ScanCfg<BV>;
-  constexpr int NT = BV / 8;
+__device__ __forceinline__ void bulk_load(uint32_t dst, const void* src, uint32_t bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes),
+               "r"(smem_u32(bar))
+               : "memory");
+}
+
+__global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_kernel(const PrefillParams pp) {
   const GdnRuleParams& p = pp.r;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127));
-  const uint32_t base = smem_u32(smem);
-  const uint32_t sS = base + 2 * C::kStage;          // two terms of the state [128][BV]
-  const uint32_t sU = sS + 2 * C::kS;                // two terms of U, then of exp(G_C - G) / |k| U, [64][BV]
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* stages = smem;                                  // two chunks' operands
+  uint8_t* sS = stages + 2 * Slot::kScal;                  // two terms of the state, [key feature][64]
+  uint8_t* sU = sS + 2 * kOperand;                         // two terms of U, then of exp(G_C - G) / |k| U, [token][64]
+  float* scalars = reinterpret_cast<float*>(sU + 4 * kPlane);
+  uint64_t* loaded = reinterpret_cast<uint64_t*>(scalars + 2 * kScalars);      // [stage] bytes of the copies
+  uint64_t* left = loaded + 2;               // [stage] commit: the chunk's products are complete (and its D3)
+  uint64_t* state_ready = left + 2;          // all threads of the state
+  uint64_t* u_ready = state_ready + 1;       // the same
+  uint64_t* d_full = u_ready + 1;            // commit: D1, D2
+  uint64_t* ds_full = d_full + 1;            // commit: dS
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(ds_full + 1);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_holder + 1);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int g = lane >> 2, t = lane & 3, ti = warp & 3;
-  const bool upper = warp >= 4;                      // warps 4 - 7 form the outputs, 0 - 3 U
   const int vb = blockIdx.x, h = blockIdx.y, b = blockIdx.z;
   pdl_wait_loads();
   const int n = p.lens[b];
   const int chunks = (n + kC - 1) / kC;
   const int c_end = min(pp.chunk0 + pp.span, chunks);
   if (pp.chunk0 >= c_end) return;
-  const int hk = h / (p.heads / p.k_heads);
-  const int cols = min(BV, p.dv - vb * BV), dv16 = (p.dv + 15) / 16 * 16;
-  const int64_t row0 = p.q_start[b];
-  float* S = p.state + (static_cast<int64_t>(p.slots[b]) * p.heads + h) * p.dk * p.dv + vb * BV;
-  const BF* q = static_cast<const BF*>(p.q) + static_cast<int64_t>(hk) * p.dk;
-  const BF* k = static_cast<const BF*>(p.k) + static_cast<int64_t>(hk) * p.dk;
+  if (tid == 0) {
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&loaded[i], 1);
+      mbar_init(&left[i], 1);
+    }
+    mbar_init(state_ready, 32 * kScanWarps);
+    mbar_init(u_ready, 32 * kScanWarps);
+    mbar_init(d_full, 1);
+    mbar_init(ds_full, 1);
+    *abort_flag = 0;
+    fence_barrier_init();
+  }
+  if (warp == kScanWarps) {
+    tmem_alloc(tmem_holder, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before_sync();
+  __syncthreads();
+  tc_fence_after_sync();
+  const uint32_t tmem = *tmem_holder;
+  const uint32_t t_d1 = tmem, t_d2 = tmem + 128, t_ds = tmem + 256, t_d3 = tmem + 384;
+  pdl_launch_dependents();
 
   auto slot_of = [&](int c) {
     return pp.ws + ((static_cast<int64_t>(b) * pp.span + (c - pp.chunk0)) * p.heads + h) * slot_bytes(p.dv);
   };
-  auto load_stage = [&](int c) {
-    const uint32_t to = base + ((c - pp.chunk0) & 1) * C::kStage;
-    const uint8_t* slot = slot_of(c);
-    for (int i = tid; i < 2 * kC * 16; i += kThreads) {          // both terms of W
-      const int r = (i >> 4) & (kC - 1), ch = i & 15, term = i >> 10;
-      cp16_zfill(to + term * kTileBytes + at128(r, ch), slot + Slot::kW + term * kTileBytes + r * kRow + ch * 16, true);
-    }
-    const int nv = min(kC, n - c * kC);
-    for (int i = tid; i < kC * 16; i += kThreads) {
-      const int r = i >> 4, ch = i & 15;
-      const bool ok = r < nv && ch * 8 < p.dk;
-      const int64_t row = row0 + static_cast<int64_t>(c) * kC + (ok ? r : 0);
-      cp16_zfill(to + 2 * kTileBytes + at128(r, ch), q + row * p.q_ld + (ok ? ch * 8 : 0), ok);
-      cp16_zfill(to + 3 * kTileBytes + at128(r, ch), k + row * p.k_ld + (ok ? ch * 8 : 0), ok);
-    }
-    for (int i = tid; i < 2 * kC * 8; i += kThreads) {           // both terms of P, tiles on and below the diagonal
-      const int r = (i >> 3) & (kC - 1), ch = i & 7, term = i >> 9;
-      if ((ch >> 1) <= (r >> 4))
-        cp16_zfill(to + 4 * kTileBytes + term * kPBytes + at64(r, ch), slot + Slot::kP + term * kPBytes + r * (kC * 2) + ch * 16, true);
-    }
-    if (tid < kScalars / 4) cp16_zfill(to + 4 * kTileBytes + 2 * kPBytes + tid * 16, slot + Slot::kScal + tid * 16, true);
-    cp_commit();
-  };
-  float u0[NT][4];
-  auto load_u0 = [&](int c) {
-    if (upper) return;
-    const float* src = reinterpret_cast<const float*>(slot_of(c) + Slot::kU) + vb * BV;
+  if (warp == kScanWarps) {
+    if (lane == 0) {
+      auto load = [&](int c) {
+        const int st = (c - pp.chunk0) & 1;
+        const uint8_t* src = slot_of(c);
+        mbar_arrive_expect_tx(&loaded[st], Slot::kBulk);
+        bulk_load(smem_u32(stages) + st * Slot::kScal, src, Slot::kScal, &loaded[st]);
+        bulk_load(smem_u32(scalars) + st * (kScalars * 4), src + Slot::kScal, kScalars * 4, &loaded[st]);
+      };
+      const uint32_t fmt = 1;                              // bf16 operands, fp32 sums
+      const uint32_t id_128 = umma_idesc(128, 128, 1, fmt, fmt, 0, 1), id_64 = umma_idesc(128, 64, 1, fmt, fmt, 0, 1);
+      const uint32_t id_kt = umma_idesc(128, 128, 1, fmt, fmt, 1, 1);
+      const uint64_t st0 = umma_desc_k_sw128(smem_u32(stages));
+      const uint64_t k0 = umma_desc_mn_sw128(smem_u32(stages + Slot::kK), kPlane, 1024);
+      const uint64_t s_desc = umma_desc_mn_sw128(smem_u32(sS), kOperand, 1024);
+      const uint64_t u_desc = umma_desc_mn_sw128(smem_u32(sU), kPlane, 1024);
+      bool ok = true;
+      auto wait_on = [&](uint64_t* bar, uint32_t parity) {
+        if (ok && !mbar_wait(bar, parity, abort_flag)) ok = false;
+        if (ok) tc_fence_after_sync();
+      };
+      load(pp.chunk0);
+      if (pp.chunk0 + 1 < c_end) load(pp.chunk0 + 1);
+      for (int c = pp.chunk0; c < c_end && ok; ++c) {
+        const int i = c - pp.chunk0, st = i & 1;
+        const uint32_t ph = i & 1, ph_stage = (i >> 1) & 1;
+        const uint32_t off = st * (Slot::kScal >> 4);
+        wait_on(&loaded[st], ph_stage);
+        wait_on(state_ready, ph);
+        if (!ok) break;
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int col = nt * 8 + 2 * t;
-        const float2 v = vb * BV + col < dv16 ? __ldcg(reinterpret_cast<const float2*>(src + static_cast<int64_t>(ti * 16 + g + half * 8) * dv16 + col))
-                                              : make_float2(0.f, 0.f);
-        u0[nt][half * 2] = v.x;
-        u0[nt][half * 2 + 1] = v.y;
-      }
-  };
-
-  load_stage(pp.chunk0);
-  load_u0(pp.chunk0);
-  // the state: this warp has key features 16 warp .. 16 warp + 15
-  float s[NT][4];
-  const bool resume = p.has_state[b] != 0 || pp.chunk0 > 0;
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = warp * 16 + g + (i >> 1) * 8, col = nt * 8 + 2 * t + (i & 1);
-      s[nt][i] = resume && row < p.dk && col < cols ? S[static_cast<int64_t>(row) * p.dv + col] : 0.f;
-    }
-
-  for (int c = pp.chunk0; c < c_end; ++c) {
-    const uint32_t st = base + ((c - pp.chunk0) & 1) * C::kStage;
-    const float* scal = reinterpret_cast<const float*>(smem + (st - base) + 4 * kTileBytes + 2 * kPBytes);
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        uint32_t hi, lo;
-        split2(s[nt][half * 2], s[nt][half * 2 + 1], hi, lo);
-        const uint32_t to = sS + at_v<BV>(warp * 16 + g + half * 8, nt) + t * 4;
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(to), "r"(hi) : "memory");
-        asm volatile("st.shared.u32 [%0], %1;" ::"r"(to + C::kS), "r"(lo) : "memory");
-      }
-    cp_wait<0>();
-    __syncthreads();
-    if (c + 1 < c_end) load_stage(c + 1);      // into the buffer that the chunk before has left
-
-    // ---- U = U0 - W S0 (warps 0 - 3), Q S0 (4 - 7) ----
-    float acc[NT][4];
-#pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) acc[nt][i] = upper ? 0.f : u0[nt][i];
-    {
-      const uint32_t left = upper ? st + 2 * kTileBytes : st;
-#pragma unroll
-      for (int kk = 0; kk < kD / 16; ++kk) {
-        uint32_t a[4], al[4];
-        const uint32_t off = at128(ti * 16 + (lane & 15), kk * 2 + (lane >> 4));
-        ldsm4(a, left + off);
-        if (!upper) ldsm4(al, left + kTileBytes + off);
-#pragma unroll
-        for (int np = 0; np < NT / 2; ++np) {
-          uint32_t w[4], wl[4];
-          const uint32_t at = sS + at_v<BV>(kk * 16 + (lane & 15), np * 2 + (lane >> 4));
-          ldsm4_t(w, at);
-          ldsm4_t(wl, at + C::kS);
-          mma_16816<BF>(acc[2 * np], a[0], a[1], a[2], a[3], w[0], w[1]);
-          mma_16816<BF>(acc[2 * np + 1], a[0], a[1], a[2], a[3], w[2], w[3]);
-          mma_16816<BF>(acc[2 * np], a[0], a[1], a[2], a[3], wl[0], wl[1]);
-          mma_16816<BF>(acc[2 * np + 1], a[0], a[1], a[2], a[3], wl[2], wl[3]);
-          if (!upper) {
-            mma_16816<BF>(acc[2 * np], al[0], al[1], al[2], al[3], w[0], w[1]);
-            mma_16816<BF>(acc[2 * np + 1], al[0], al[1], al[2], al[3], w[2], w[3]);
-          }
+        for (int kk = 0; kk < 8; ++kk) {
+          const uint64_t a = st0 + off + (kk >> 2) * (Slot::kHalf >> 4) + (kk & 3) * 2;
+          umma_f16(t_d1, a, s_desc + kk * (2048 >> 4), id_128, kk > 0 ? 1u : 0u);
         }
+#pragma unroll
+        for (int kk = 0; kk < 8; ++kk) {
+          const uint64_t a = st0 + off + ((Slot::kWlo + (kk >> 2) * Slot::kHalf) >> 4) + (kk & 3) * 2;
+          umma_f16(t_d2, a, s_desc + kk * (2048 >> 4), id_64, kk > 0 ? 1u : 0u);
+        }
+        umma_commit(d_full);
+        // every thread has left the chunk before, and its products were complete before these began: its stage is free
+        if (i >= 1 && c + 1 < c_end) {
+          wait_on(&left[st ^ 1], ((i - 1) >> 1) & 1);
+          if (ok) load(c + 1);
+        }
+        wait_on(u_ready, ph);
+        if (!ok) break;
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          umma_f16(t_ds, k0 + off + kk * (2048 >> 4), u_desc + ((2 * kPlane + kk * 2048) >> 4), id_kt, kk > 0 ? 1u : 0u);
+        umma_commit(ds_full);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)      // rows 64 - 127 of the left operand are the scores; the plane in front fills the others
+          umma_f16(t_d3, st0 + off + ((Slot::kP - kPlane) >> 4) + kk * 2, u_desc + kk * (2048 >> 4), id_128, kk > 0 ? 1u : 0u);
+#pragma unroll
+        for (int kk = 0; kk < 4; ++kk)
+          umma_f16(t_d3, st0 + off + (Slot::kP >> 4) + kk * 2, u_desc + kk * (2048 >> 4), id_64, 1u);
+        umma_commit(&left[st]);
       }
+      if (!ok) *abort_flag = 1;
     }
-    if (c + 1 < c_end) load_u0(c + 1);
+  } else {
+    constexpr int N = kScanCols;
+    const int quad = warp & 3, col0 = (warp >> 2) * N;           // this warp's lanes of tensor memory, and its value features
+    const uint32_t lanes = static_cast<uint32_t>(quad * 32) << 16;
+    const int key = quad * 32 + lane, tok = (quad & 1) * 32 + lane;
+    const bool is_o = quad >= 2;                                 // rows 64 - 127: outputs; rows 0 - 63: U
+    const int cols = min(N, p.dv - vb * kBV - col0);             // may be negative
+    float* S = p.state + ((static_cast<int64_t>(p.slots[b]) * p.heads + h) * p.dk + min(key, p.dk - 1)) * p.dv + vb * kBV + col0;
+    const bool resume = p.has_state[b] != 0 || pp.chunk0 > 0;
+    float s[N];
 #pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int row = ti * 16 + g + half * 8;
-      const float f = scal[upper ? row : kC + row];
+    for (int j = 0; j < N; j += 4) {
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (resume && key < p.dk && j < cols) v = pp.wide ? *reinterpret_cast<const float4*>(S + j) : make_float4(S[j], S[j + 1], S[j + 2], S[j + 3]);
+      s[j] = v.x;
+      s[j + 1] = v.y;
+      s[j + 2] = v.z;
+      s[j + 3] = v.w;
+    }
+    float u0[N];
+    auto load_u0 = [&](int c) {
+      if (is_o) return;
+      const float4* src = reinterpret_cast<const float4*>(slot_of(c) + Slot::kU) + static_cast<int64_t>(vb * (kBV / 4) + col0 / 4) * kC + tok;
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        float& a = acc[nt][half * 2];
-        float& d = acc[nt][half * 2 + 1];
-        if (upper) {
-          a *= f;
-          d *= f;
+      for (int j = 0; j < N / 4; ++j) {
+        const float4 v = __ldcg(src + j * kC);
+        u0[4 * j] = v.x;
+        u0[4 * j + 1] = v.y;
+        u0[4 * j + 2] = v.z;
+        u0[4 * j + 3] = v.w;
+      }
+    };
+    // values of a row as two terms into planes of 128-byte rows, `second` bytes apart
+    auto put = [&](uint8_t* plane, int row, const float (&v)[N], float f, uint32_t second) {
+#pragma unroll
+      for (int q = 0; q < N / 8; ++q) {
+        uint32_t hi[4], lo[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) split2(v[q * 8 + 2 * j] * f, v[q * 8 + 2 * j + 1] * f, hi[j], lo[j]);
+        uint8_t* to = plane + row * 128 + (((col0 / 8 + q) ^ (row & 7)) << 4);
+        *reinterpret_cast<uint4*>(to) = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        *reinterpret_cast<uint4*>(to + second) = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+      }
+    };
+    // v += f * (the columns at `at` and, where there are two terms, those 64 on)
+    auto add_columns = [&](uint32_t at, float (&v)[N], float f, bool two) {
+      uint32_t r[N], r2[N];
+      tmem_ld_32x16(at + lanes + col0, r);
+      if (two) tmem_ld_32x16(at + 64 + lanes + col0, r2);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < N; ++j) {
+        v[j] = fmaf(__uint_as_float(r[j]), f, v[j]);
+        if (two) v[j] = fmaf(__uint_as_float(r2[j]), f, v[j]);
+      }
+    };
+    static_assert(N == 16, "loads of tensor memory");
+    bool ok = true;
+    auto wait_on = [&](uint64_t* bar, uint32_t parity) {
+      if (ok && !mbar_wait(bar, parity, abort_flag)) ok = false;
+      tc_fence_after_sync();
+    };
+    float v[N];
+    auto finish_outputs = [&](int c) {       // v: exp(G) Q S of the chunk
+      const int i = c - pp.chunk0;
+      wait_on(&left[i & 1], (i >> 1) & 1);
+      add_columns(t_d3, v, 1.f, true);
+      if (!ok || c * kC + tok >= n) return;
+      BF* out = static_cast<BF*>(p.out) + ((static_cast<int64_t>(p.q_start[b]) + static_cast<int64_t>(c) * kC + tok) * p.heads + h) * p.dv + vb * kBV + col0;
+      if (cols == N && pp.wide) {
+#pragma unroll
+        for (int q = 0; q < N / 8; ++q)
+          reinterpret_cast<uint4*>(out)[q] = make_uint4(pack_bf16x2(v[q * 8], v[q * 8 + 1]), pack_bf16x2(v[q * 8 + 2], v[q * 8 + 3]),
+                                                        pack_bf16x2(v[q * 8 + 4], v[q * 8 + 5]), pack_bf16x2(v[q * 8 + 6], v[q * 8 + 7]));
+      } else {
+#pragma unroll
+        for (int j = 0; j < N; j += 2)
+          if (j < cols) *reinterpret_cast<uint32_t*>(out + j) = pack_bf16x2(v[j], v[j + 1]);
+      }
+    };
+    load_u0(pp.chunk0);
+    for (int c = pp.chunk0; c < c_end && ok; ++c) {
+      const int i = c - pp.chunk0, st = i & 1;
+      const uint32_t ph = i & 1, ph_stage = (i >> 1) & 1;
+      put(sS, key, s, 1.f, kOperand);
+      fence_proxy_async_smem();
+      tc_fence_before_sync();
+      mbar_arrive(state_ready);
+      if (is_o && i > 0) finish_outputs(c - 1);
+      wait_on(&loaded[st], ph_stage);
+      const float* scal = scalars + st * kScalars;
+      const float f = scal[is_o ? tok : kC + tok], carry = scal[2 * kC];
+#pragma unroll
+      for (int j = 0; j < N; ++j) v[j] = is_o ? 0.f : u0[j];
+      wait_on(d_full, ph);
+      if (is_o) {
+        add_columns(t_d1, v, f, true);
+      } else {
+        add_columns(t_d1, v, 1.f, true);
+        add_columns(t_d2, v, 1.f, false);
+        put(sU + 2 * kPlane, tok, v, f, kPlane);
+        put(sU, tok, v, 1.f, kPlane);
+        fence_proxy_async_smem();
+      }
+      tc_fence_before_sync();
+      mbar_arrive(u_ready);
+      if (c + 1 < c_end) load_u0(c + 1);
+#pragma unroll
+      for (int j = 0; j < N; ++j) s[j] *= carry;
+      wait_on(ds_full, ph);
+      add_columns(t_ds, s, 1.f, true);
+    }
+    if (is_o && ok) finish_outputs(c_end - 1);
+    if (!ok) *abort_flag = 1;
+    if (key < p.dk && ok) {
+#pragma unroll
+      for (int j = 0; j < N; j += 4) {
+        if (j >= cols) continue;
+        if (pp.wide) {
+          *reinterpret_cast<float4*>(S + j) = make_float4(s[j], s[j + 1], s[j + 2], s[j + 3]);
         } else {
-          uint32_t hi, lo;
-          const uint32_t to = sU + at_v<BV>(row, nt) + t * 4;
-          split2(a, d, hi, lo);
-          asm volatile("st.shared.u32 [%0], %1;" ::"r"(to), "r"(hi) : "memory");
-          asm volatile("st.shared.u32 [%0], %1;" ::"r"(to + C::kU), "r"(lo) : "memory");
-          split2(a * f, d * f, hi, lo);
-          asm volatile("st.shared.u32 [%0], %1;" ::"r"(to + 2 * C::kU), "r"(hi) : "memory");
-          asm volatile("st.shared.u32 [%0], %1;" ::"r"(to + 3 * C::kU), "r"(lo) : "memory");
-        }
-      }
-    }
-    __syncthreads();
-
-    // ---- S = exp(G_C) S0 + K^T U' (all warps) ----
-    const float carry = scal[2 * kC];
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-      for (int i = 0; i < 4; ++i) s[nt][i] *= carry;
-#pragma unroll
-    for (int ks = 0; ks < kC / 16; ++ks) {
-      uint32_t a[4];
-      ldsm4_t(a, st + 3 * kTileBytes + at128(ks * 16 + (lane & 7) + ((lane >> 4) << 3), warp * 2 + ((lane >> 3) & 1)));
-#pragma unroll
-      for (int np = 0; np < NT / 2; ++np) {
-        uint32_t w[4], wl[4];
-        const uint32_t at = sU + 2 * C::kU + at_v<BV>(ks * 16 + (lane & 15), np * 2 + (lane >> 4));
-        ldsm4_t(w, at);
-        ldsm4_t(wl, at + C::kU);
-        mma_16816<BF>(s[2 * np], a[0], a[1], a[2], a[3], w[0], w[1]);
-        mma_16816<BF>(s[2 * np + 1], a[0], a[1], a[2], a[3], w[2], w[3]);
-        mma_16816<BF>(s[2 * np], a[0], a[1], a[2], a[3], wl[0], wl[1]);
-        mma_16816<BF>(s[2 * np + 1], a[0], a[1], a[2], a[3], wl[2], wl[3]);
-      }
-    }
-    // ---- O = exp(G) (Q S0) + P U (warps 4 - 7) ----
-    if (upper) {
-#pragma unroll
-      for (int ks = 0; ks < kC / 16; ++ks) {
-        if (ks <= ti) {
-          uint32_t a[4], al[4];
-          const uint32_t off = st + 4 * kTileBytes + at64(ti * 16 + (lane & 15), ks * 2 + (lane >> 4));
-          ldsm4(a, off);
-          ldsm4(al, off + kPBytes);
-#pragma unroll
-          for (int np = 0; np < NT / 2; ++np) {
-            uint32_t w[4], wl[4];
-            const uint32_t at = sU + at_v<BV>(ks * 16 + (lane & 15), np * 2 + (lane >> 4));
-            ldsm4_t(w, at);
-            ldsm4_t(wl, at + C::kU);
-            mma_16816<BF>(acc[2 * np], a[0], a[1], a[2], a[3], w[0], w[1]);
-            mma_16816<BF>(acc[2 * np + 1], a[0], a[1], a[2], a[3], w[2], w[3]);
-            mma_16816<BF>(acc[2 * np], a[0], a[1], a[2], a[3], wl[0], wl[1]);
-            mma_16816<BF>(acc[2 * np + 1], a[0], a[1], a[2], a[3], wl[2], wl[3]);
-            mma_16816<BF>(acc[2 * np], al[0], al[1], al[2], al[3], w[0], w[1]);
-            mma_16816<BF>(acc[2 * np + 1], al[0], al[1], al[2], al[3], w[2], w[3]);
-          }
-        }
-      }
-      const int nv = min(kC, n - c * kC);
-#pragma unroll
-      for (int half = 0; half < 2; ++half) {
-        const int row = ti * 16 + g + half * 8;
-        BF* out = static_cast<BF*>(p.out) + ((row0 + static_cast<int64_t>(c) * kC + row) * p.heads + h) * p.dv + vb * BV;
-#pragma unroll
-        for (int nt = 0; nt < NT; ++nt) {
-          const int col = nt * 8 + 2 * t;
-          if (row < nv && col < cols) *reinterpret_cast<uint32_t*>(out + col) = pack_bf16x2(acc[nt][half * 2], acc[nt][half * 2 + 1]);
+          for (int e = 0; e < 4; ++e) S[j + e] = s[j + e];
         }
       }
     }
   }
-#pragma unroll
-  for (int nt = 0; nt < NT; ++nt)
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const int row = warp * 16 + g + (i >> 1) * 8, col = nt * 8 + 2 * t + (i & 1);
-      if (row < p.dk && col < cols) S[static_cast<int64_t>(row) * p.dv + col] = s[nt][i];
-    }
+  tc_fence_before_sync();
+  __syncthreads();
+  if (*abort_flag) {
+    if (tid == 0 && pp.status != nullptr) atomicExch(pp.status, kStatusPipelineTimeout);
+    // copies may still be in flight: give them time to land before the CTA's memory is reused
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+  }
+  if (warp == kScanWarps) {
+    tc_fence_after_sync();
+    tmem_dealloc(tmem, 512);
+  }
 }
 
-constexpr int kPrepareSmem = 3 * kTileBytes + (2 * kC * kLd + 3 * 16 * 17 + 5 * kC) * 4 + 128;
-
-template <int BV>
-int launch_scan(const PrefillParams& pp, cudaStream_t s) {
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(gdn_scan_kernel<BV>), ScanCfg<BV>::kSmem) != cudaSuccess) return -3;
-  const cudaError_t err = launch_pdl(gdn_scan_kernel<BV>, dim3((pp.r.dv + BV - 1) / BV, pp.r.heads, pp.r.batch), dim3(kThreads),
-                                     ScanCfg<BV>::kSmem, s, pp);
-  return err == cudaSuccess ? 0 : -4;
-}
+constexpr int kPrepareSmem = 3 * kTileBytes + (2 * kC * kLd + 3 * 16 * kXLd + 5 * kC) * 4 + 2 * kPlane + 128;
+static_assert(2 * (kPrepareSmem + 1024) <= 228 * 1024, "two CTAs of the first kernel per SM");
 
 }  // namespace
 
@@ -565,22 +674,12 @@ GdnPrefillPlan gdn_prefill_plan(const GdnRuleParams& p, int max_len, int64_t mos
   return {static_cast<int>(group), static_cast<int>(span), group * span * chunk};
 }
 
-int launch_gdn_prefill(const GdnRuleParams& p, void* ws, const GdnPrefillPlan& plan, int max_len, int num_sms, cudaStream_t s) {
+int launch_gdn_prefill(const GdnRuleParams& p, void* ws, const GdnPrefillPlan& plan, int max_len, int* status, cudaStream_t s) {
   if (p.batch <= 0 || max_len <= 0) return 0;
   if (!gdn_prefill_covers(p) || p.heads % p.k_heads != 0 || p.g == nullptr || (reinterpret_cast<uintptr_t>(p.out) & 3) != 0) return -1;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(gdn_prepare_kernel), kPrepareSmem) != cudaSuccess) return -3;
-  // a wider block of value features takes a chunk's operands in fewer times and leaves fewer CTAs: the width with the least
-  // waves x time of a chunk (in tenths of us)
-  int best = 64, least = 1 << 30;
-  const int widths[3] = {16, 32, 64}, times[3] = {12, 17, 29};
-  for (int i = 0; i < 3; ++i) {
-    const int64_t ctas = static_cast<int64_t>(plan.group) * p.heads * ((p.dv + widths[i] - 1) / widths[i]);
-    const int64_t cost = (ctas + num_sms - 1) / num_sms * times[i];
-    if (cost < least) {
-      least = static_cast<int>(std::min<int64_t>(cost, 1 << 30));
-      best = widths[i];
-    }
-  }
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(gdn_scan_kernel), kScanSmem) != cudaSuccess) return -3;
+  const int wide = ((reinterpret_cast<uintptr_t>(p.state) | reinterpret_cast<uintptr_t>(p.out)) & 15) == 0;
   const int chunks = (max_len + kC - 1) / kC;
   for (int b0 = 0; b0 < p.batch; b0 += plan.group) {
     GdnRuleParams r = p;
@@ -590,12 +689,12 @@ int launch_gdn_prefill(const GdnRuleParams& p, void* ws, const GdnPrefillPlan& p
     r.has_state += b0;
     r.q_start += b0;
     for (int c0 = 0; c0 < chunks; c0 += plan.span) {
-      PrefillParams pp{r, static_cast<uint8_t*>(ws), c0, plan.span};
-      const cudaError_t err = launch_pdl(gdn_prepare_kernel, dim3(std::min(plan.span, chunks - c0), r.heads, r.batch), dim3(kThreads), kPrepareSmem, s, pp);
+      PrefillParams pp{r, static_cast<uint8_t*>(ws), status, c0, plan.span, wide};
+      cudaError_t err = launch_pdl(gdn_prepare_kernel, dim3(std::min(plan.span, chunks - c0), r.heads, r.batch), dim3(kThreads), kPrepareSmem, s, pp);
       note_launch();      // the pair counts as one: the rule over a span
       if (err != cudaSuccess) return -4;
-      const int rc = best == 16 ? launch_scan<16>(pp, s) : best == 32 ? launch_scan<32>(pp, s) : launch_scan<64>(pp, s);
-      if (rc != 0) return rc;
+      err = launch_pdl(gdn_scan_kernel, dim3(value_blocks(r.dv), r.heads, r.batch), dim3(kScanThreads), kScanSmem, s, pp);
+      if (err != cudaSuccess) return -4;
     }
   }
   return 0;

@@ -586,7 +586,7 @@ struct GdnPrefillPlan {
 };
 bool gdn_prefill_covers(const GdnRuleParams& p);
 GdnPrefillPlan gdn_prefill_plan(const GdnRuleParams& p, int max_len, int64_t most_bytes);
-int launch_gdn_prefill(const GdnRuleParams& p, void* ws, const GdnPrefillPlan& plan, int max_len, int num_sms, cudaStream_t s);
+int launch_gdn_prefill(const GdnRuleParams& p, void* ws, const GdnPrefillPlan& plan, int max_len, int* status, cudaStream_t s);
 // decays per key channel, 16 tokens at a time (prefill); dk up to 128, multiples of 8, gates formed inside.  The workspace
 // holds `span` chunks of every request; longer runs loop over spans
 struct GdnChannelPlan {

@@ -96,3 +96,20 @@ def test_workspace_of_many_requests(monkeypatch):
 def test_spans_of_many_heads():
     """Heads that leave room for one chunk at a time in 512 MB, the longest run not known."""
     _check([330, 129], 1700, 100, 8, 128, max_len=0)
+
+
+def test_state_between_other_values():
+    """A state that does not start on a 16-byte boundary is moved value by value, and nothing beside it is touched."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+    lens, heads, dk, dv = [70, 5], 2, 128, 96
+    q, k, v = (torch.randn((75, heads, d), generator=gen, device="cuda").bfloat16() for d in (dk, dk, dv))
+    g, beta = -torch.rand((75, heads), generator=gen, device="cuda") * 0.1, torch.rand((75, heads), generator=gen, device="cuda")
+    room = torch.randn(2 * heads * dk * dv + 6, generator=gen, device="cuda") * 0.1
+    plain = room[1:-5].clone().view(2, heads, dk, dv)
+    odd = room[1:-5].view(2, heads, dk, dv)
+    before = room.clone()
+    i32 = dict(dtype=torch.int32, device="cuda")
+    got = [ops.gated_delta_rule(q, k, v, g, beta, s, torch.arange(2, **i32), torch.tensor(lens, **i32), torch.ones(2, **i32), max_len=70) for s in (plain, odd)]
+    ops.check_status()
+    assert torch.equal(got[0], got[1]) and torch.equal(plain, odd)
+    assert torch.equal(room[:1], before[:1]) and torch.equal(room[-5:], before[-5:])
