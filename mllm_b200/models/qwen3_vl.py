@@ -259,33 +259,38 @@ def get_rope_index(input_ids: torch.Tensor, image_grid_thw, image_token_id: int,
     (a cached prefix of text).  ``t_scales`` holds one factor per grid for the temporal axis: a video clip
     of Qwen2.5-VL advances ``seconds per temporal patch x tokens per second`` positions per temporal patch
     (truncated to an integer per patch); 1 everywhere else."""
-    ids = input_ids.tolist()
+    ids = input_ids.cpu().numpy()
     T = len(ids)
     grids = [] if image_grid_thw is None else (image_grid_thw.tolist() if isinstance(image_grid_thw, torch.Tensor)
                                                else [list(g) for g in image_grid_thw])
     pos = np.zeros((3, T), dtype=np.int64)
     cur, img, i = start, 0, 0
-    while i < T:
-        if ids[i] == vision_start_token_id and img < len(grids):
-            pos[:, i] = cur
-            cur += 1
-            i += 1
-            t, h, w = int(grids[img][0]), int(grids[img][1]) // spatial_merge_size, int(grids[img][2]) // spatial_merge_size
-            n = min(t * h * w, T - i)
-            steps = np.arange(t)
-            if t_scales is not None and float(t_scales[img]) != 1.0:
-                steps = (steps * float(t_scales[img])).astype(np.int64)
-            tt, hh, ww = np.meshgrid(steps, np.arange(h), np.arange(w), indexing="ij")
-            pos[0, i:i + n] = tt.flatten()[:n] + cur
-            pos[1, i:i + n] = hh.flatten()[:n] + cur
-            pos[2, i:i + n] = ww.flatten()[:n] + cur
-            cur += max(int(steps[-1]) + 1, h, w)
-            i += n
-            img += 1
-        else:
-            pos[:, i] = cur
-            cur += 1
-            i += 1
+
+    def text(end: int) -> None:
+        nonlocal cur, i
+        pos[:, i:end] = np.arange(cur, cur + end - i)
+        cur += end - i
+        i = end
+
+    for at in np.flatnonzero(ids == vision_start_token_id) if grids else ():
+        if at < i:                      # inside an image block
+            continue
+        if img == len(grids):
+            break
+        text(int(at) + 1)
+        t, h, w = int(grids[img][0]), int(grids[img][1]) // spatial_merge_size, int(grids[img][2]) // spatial_merge_size
+        n = min(t * h * w, T - i)
+        steps = np.arange(t)
+        if t_scales is not None and float(t_scales[img]) != 1.0:
+            steps = (steps * float(t_scales[img])).astype(np.int64)
+        tt, hh, ww = np.meshgrid(steps, np.arange(h), np.arange(w), indexing="ij")
+        pos[0, i:i + n] = tt.flatten()[:n] + cur
+        pos[1, i:i + n] = hh.flatten()[:n] + cur
+        pos[2, i:i + n] = ww.flatten()[:n] + cur
+        cur += max(int(steps[-1]) + 1, h, w)
+        i += n
+        img += 1
+    text(T)
     return torch.from_numpy(pos).to(input_ids.device), cur - start - T
 
 
@@ -329,15 +334,19 @@ class VisionLanguageMixin:
         if sync:
             torch.cuda.synchronize()
         fb.vit_prefill_ms = (time.perf_counter() - t0) * 1e3
-        mask = input_ids == self.image_token_id
+        # the rows are found on the host, in the ids that the positions were made from: asking the device for them would wait for the tower
+        ids = fb.extra.get("input_ids_cpu")
+        ids = (input_ids.cpu() if ids is None else ids).numpy()
+        mask = ids == self.image_token_id
         if self.video_token_id is not None:
-            mask = mask | (input_ids == self.video_token_id)
-        n_tok = int(mask.sum())
+            mask |= ids == self.video_token_id
+        rows = np.flatnonzero(mask)
+        n_tok = len(rows)
         fb.vit_prefill_tokens = n_tok
         if n_tok != feats.shape[0]:
             raise ValueError(f"Image features and image tokens do not match, tokens: {n_tok}, features: {feats.shape[0]}")
         input_embeds = self.model.embed_tokens(input_ids)
-        where = mask.nonzero(as_tuple=True)[0]
+        where = torch.from_numpy(rows).to(input_ids.device)
         input_embeds.index_copy_(0, where, feats[:, : self.hidden_size].to(input_embeds.dtype))
         deepstack = None
         if self.num_deepstack:
@@ -380,7 +389,7 @@ class VisionLanguageMixin:
         known = fb.mrope_position_deltas.tolist() if fb.mrope_position_deltas is not None else [0] * len(lens)
         grids = None if fb.image_grid_thw is None else fb.image_grid_thw.tolist()
         scales = None if getattr(fb, "mrope_t_scale", None) is None else fb.mrope_t_scale.tolist()
-        ids_cpu = input_ids.cpu()
+        ids_cpu = fb.extra["input_ids_cpu"] = input_ids.cpu()
         out, deltas, off, img = [], [], 0, 0
         for i, n in enumerate(lens):
             seq = ids_cpu[off:off + n]

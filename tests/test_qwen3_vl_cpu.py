@@ -189,3 +189,28 @@ def test_builtin_image_preprocessing_matches_the_hf_processor():
     pv, grid = preprocess_image(torch.from_numpy(odd))
     assert grid.tolist() == want["image_grid_thw"].tolist() and pv.shape == want["pixel_values"].shape
     assert (pv - want["pixel_values"]).abs().mean().item() < 0.05
+
+
+def test_get_rope_index_walks_like_a_counter():
+    """Against a counter that takes the tokens one by one: blocks that the end cuts off, start tokens inside a block, more start tokens
+    than grids, a block at the very end."""
+    rng = np.random.default_rng(0)
+    for _ in range(300):
+        ids = rng.choice([1, 2, 3, IMG, VSTART], size=int(rng.integers(0, 60)), p=[0.3, 0.2, 0.2, 0.2, 0.1])
+        grids = [[int(rng.integers(1, 3)), 2 * int(rng.integers(1, 4)), 2 * int(rng.integers(1, 4))] for _ in range(int(rng.integers(0, 4)))]
+        start, want, cur, img, i = int(rng.integers(0, 9)), np.zeros((3, len(ids)), dtype=np.int64), 0, 0, 0
+        cur = start
+        while i < len(ids):
+            want[:, i] = cur
+            cur, i = cur + 1, i + 1
+            if ids[i - 1] == VSTART and img < len(grids):
+                t, h, w = grids[img][0], grids[img][1] // 2, grids[img][2] // 2
+                for a in range(t):
+                    for b in range(h):
+                        for c in range(w):
+                            if i < len(ids):
+                                want[:, i] = cur + a, cur + b, cur + c
+                                i += 1
+                cur, img = cur + max(t, h, w), img + 1
+        pos, delta = get_rope_index(torch.tensor(ids), grids, IMG, VSTART, 2, start=start)
+        assert (pos.numpy() == want).all() and delta == cur - start - len(ids)
