@@ -20,33 +20,48 @@ namespace {
 
 constexpr int kMaxConvK = 16;
 
-// SiLU of a value that is rounded to T next: the fast exponential and division for 16-bit results
+// Sigmoid and SiLU of a value that is rounded to 16 bits next: an exponential and a reciprocal that flush subnormal numbers, 2 units in
+// the last place in all.  (The fast exponential and division of the library keep subnormal numbers, for some ten instructions more.)
+__device__ __forceinline__ float fast_sigmoid(float v) {
+  float e, r;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(v * -1.4426950408889634f));
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+  return r;
+}
 template <typename T>
 __device__ __forceinline__ float silu(float v) {
-  if constexpr (sizeof(T) == 2) return __fdividef(v, 1.f + __expf(-v));
+  if constexpr (sizeof(T) == 2) return v * fast_sigmoid(v);
   return v / (1.f + expf(-v));
 }
 
 // V neighbouring elements (V * sizeof(T) a power of two, aligned) as floats, and back.  The load is from the L2, so that a CTA
 // that was resident before its inputs were written sees them without a fence that empties the SM's L1.
 template <typename T, int V>
-__device__ __forceinline__ void load_v(const T* p, float (&f)[V]) {
-  struct alignas(sizeof(T) * V) Pack { T e[V]; };
+struct alignas(sizeof(T) * V) Pack {
+  T e[V];
+};
+template <typename T, int V>
+__device__ __forceinline__ Pack<T, V> load_pack(const T* p) {
+  using Pack = Pack<T, V>;
   Pack r;
   if constexpr (sizeof(Pack) == 16) *reinterpret_cast<uint4*>(&r) = __ldcg(reinterpret_cast<const uint4*>(p));
   else if constexpr (sizeof(Pack) == 8) *reinterpret_cast<uint2*>(&r) = __ldcg(reinterpret_cast<const uint2*>(p));
   else if constexpr (sizeof(Pack) == 4) *reinterpret_cast<uint32_t*>(&r) = __ldcg(reinterpret_cast<const uint32_t*>(p));
   else *reinterpret_cast<uint16_t*>(&r) = __ldcg(reinterpret_cast<const uint16_t*>(p));
+  return r;
+}
+template <typename T, int V>
+__device__ __forceinline__ void load_v(const T* p, float (&f)[V]) {
+  const Pack<T, V> r = load_pack<T, V>(p);
 #pragma unroll
   for (int i = 0; i < V; ++i) f[i] = to_f32(r.e[i]);
 }
 template <typename T, int V>
 __device__ __forceinline__ void store_v(T* p, const float (&f)[V]) {
-  struct alignas(sizeof(T) * V) Pack { T e[V]; };
-  Pack r;
+  Pack<T, V> r;
 #pragma unroll
   for (int i = 0; i < V; ++i) r.e[i] = from_f32<T>(f[i]);
-  *reinterpret_cast<Pack*>(p) = r;
+  *reinterpret_cast<Pack<T, V>*>(p) = r;
 }
 
 // grid (ceil(C / 256 V), chunks, B); a thread handles V neighbouring channels of a run of tokens of one request.  KT:
@@ -91,38 +106,56 @@ __global__ void gdn_conv1d_silu_kernel(const T* __restrict__ x, int64_t x_ld, co
       }
     }
   }
-  // eight tokens are in flight while eight are worked on: a thread's loads, not its arithmetic, set the rate
+  // eight tokens are in flight while eight are worked on: a thread's loads, not its arithmetic, set the rate.  They stay as they come
+  // until they are used: widened on arrival they had to be waited for in front of the work.
+  // Beside them, instructions set it: 16 an output, where pointers and ends of the run were worked out per token 33.
   constexpr int kAhead = 8;
-  float nxt[kAhead][V];
-  auto fetch = [&](int t) {
+  Pack<T, V> nxt[kAhead];
+  const T* from = x + (row0 + t0) * x_ld + c;
+  T* to = out + (row0 + t0) * channels + c;
+  auto one = [&](const Pack<T, V>& in) {
+    float acc[V], cur[V];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u)
-      if (t + u < t1) load_v<T, V>(x + (row0 + t + u) * x_ld + c, nxt[u]);
+    for (int i = 0; i < V; ++i) cur[i] = to_f32(in.e[i]);
+#pragma unroll
+    for (int i = 0; i < V; ++i) {
+      acc[i] = bv[i];
+#pragma unroll
+      for (int j = 0; j < kCap; ++j)
+        if (j < K) acc[i] = fmaf(wv[j][i], j == K - 1 ? cur[i] : win[j][i], acc[i]);
+      acc[i] = add_input ? cur[i] + acc[i] : silu<T>(acc[i]);
+#pragma unroll
+      for (int j = 0; j < kCap - 1; ++j)
+        if (j < K - 1) win[j][i] = j == K - 2 ? cur[i] : win[j + 1][i];
+    }
+    store_v<T, V>(to, acc);
+    to += channels;
+  };
+  auto fetch = [&](int t) {
+    const T* at = from;
+    if (t + kAhead <= t1) {
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u, at += x_ld) nxt[u] = load_pack<T, V>(at);
+    } else {
+#pragma unroll
+      for (int u = 0; u < kAhead; ++u, at += x_ld)
+        if (t + u < t1) nxt[u] = load_pack<T, V>(at);
+    }
+    from = at;
   };
   fetch(t0);
   for (int t = t0; t < t1; t += kAhead) {
-    float cur[kAhead][V];
+    Pack<T, V> now[kAhead];
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u)
-#pragma unroll
-      for (int i = 0; i < V; ++i) cur[u][i] = nxt[u][i];
+    for (int u = 0; u < kAhead; ++u) now[u] = nxt[u];
     fetch(t + kAhead);
+    if (t + kAhead <= t1) {
 #pragma unroll
-    for (int u = 0; u < kAhead; ++u) {
-      if (t + u >= t1) break;
-      float acc[V];
+      for (int u = 0; u < kAhead; ++u) one(now[u]);
+    } else {
 #pragma unroll
-      for (int i = 0; i < V; ++i) {
-        acc[i] = bv[i];
-#pragma unroll
-        for (int j = 0; j < kCap; ++j)
-          if (j < K) acc[i] = fmaf(wv[j][i], j == K - 1 ? cur[u][i] : win[j][i], acc[i]);
-        acc[i] = add_input ? cur[u][i] + acc[i] : silu<T>(acc[i]);
-#pragma unroll
-        for (int j = 0; j < kCap - 1; ++j)
-          if (j < K - 1) win[j][i] = j == K - 2 ? cur[u][i] : win[j + 1][i];
-      }
-      store_v<T, V>(out + (row0 + t + u) * channels + c, acc);
+      for (int u = 0; u < kAhead; ++u)
+        if (t + u < t1) one(now[u]);
     }
   }
   if (own_state) {
@@ -379,10 +412,60 @@ __global__ void rmsnorm_gated_kernel(const T* __restrict__ x, const T* __restric
     for (int i = 0; i < V; ++i) {
       float nrm = f[i] * rstd;
       if (round_norm) nrm = to_f32(from_f32<T>(nrm));
-      if constexpr (SIG) f[i] = wv[i] * nrm * (sizeof(T) == 2 ? __fdividef(1.f, 1.f + __expf(-g[i])) : 1.f / (1.f + expf(-g[i])));
+      if constexpr (SIG) f[i] = wv[i] * nrm * (sizeof(T) == 2 ? fast_sigmoid(g[i]) : 1.f / (1.f + expf(-g[i])));
       else f[i] = wv[i] * nrm * silu<T>(g[i]);
     }
     store_v<T, V>(out + r * width + c, f);
+  }
+}
+
+// The same for 16-bit rows of up to 128 values and many of them: half a warp has a row, 16 bytes a lane, and R rows on their way.  A copy
+// of two inputs and an output in all, if the loads are wide and many.
+template <typename T, bool SIG, int R>
+__global__ void __launch_bounds__(256, 5) rmsnorm_gated_rows_kernel(const T* x, const T* gate, int64_t gate_ld, const T* w, T* out, int rows,
+                                                                 int heads, int width, float eps, int round_norm) {
+  pdl_wait_loads();
+  const int lane = threadIdx.x & 31, at = (lane & 15) * 8;
+  const int first = (blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * 2 * R + (lane >> 4);
+  const bool mine = at < width;
+  float wv[8];
+  Pack<T, 8> f[R], g[R];
+  int token = first / heads, head = first - token * heads;
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int r = first + 2 * i;
+    if (mine && r < rows) {
+      f[i] = load_pack<T, 8>(x + static_cast<int64_t>(r) * width + at);
+      g[i] = load_pack<T, 8>(gate + token * gate_ld + head * width + at);
+      for (head += 2; head >= heads; head -= heads) ++token;
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[i].e[j] = g[i].e[j] = from_f32<T>(0.f);
+    }
+  }
+  if (mine) load_v<T, 8>(w + at, wv);
+#pragma unroll
+  for (int i = 0; i < R; ++i) {
+    const int r = first + 2 * i;
+    float v[8], ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = to_f32(f[i].e[j]);
+      ss = fmaf(v[j], v[j], ss);
+    }
+#pragma unroll
+    for (int d = 8; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+    const float rstd = 1.f / sqrtf(ss / static_cast<float>(width) + eps);
+    if (!mine || r >= rows) continue;
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float gate_v = to_f32(g[i].e[j]);
+      float nrm = v[j] * rstd;
+      if (round_norm) nrm = to_f32(from_f32<T>(nrm));
+      if constexpr (SIG) v[j] = wv[j] * nrm * fast_sigmoid(gate_v);
+      else v[j] = wv[j] * nrm * silu<T>(gate_v);
+    }
+    store_v<T, 8>(out + static_cast<int64_t>(r) * width + at, v);
   }
 }
 
@@ -476,6 +559,25 @@ void launch_rmsnorm_gated(const void* x, const void* gate, int64_t gate_ld, cons
     launch_pdl(kernel, grid, block, 0, s, static_cast<const T*>(x), static_cast<const T*>(gate), gate_ld, static_cast<const T*>(w),
                static_cast<T*>(out), rows, heads, width, eps, round_norm);
   };
+  // Half a warp to a row from 4096 rows on; a step's few rows get a warp each and reach more SMs that way
+  constexpr int kRowsInFlight = 2;
+  if (dt != kF32 && width % 8 == 0 && width <= 128 && gate_ld % 8 == 0 && align % 16 == 0 && rows >= 4096 && rows < (int64_t(1) << 30)) {
+    const unsigned blocks = static_cast<unsigned>((rows + 16 * kRowsInFlight - 1) / (16 * kRowsInFlight));
+    auto go_rows = [&](auto typed, auto kernel) {
+      using T = decltype(typed);
+      launch_pdl(kernel, dim3(blocks), dim3(256), 0, s, static_cast<const T*>(x), static_cast<const T*>(gate), gate_ld,
+                 static_cast<const T*>(w), static_cast<T*>(out), static_cast<int>(rows), heads, width, eps, round_norm);
+    };
+    if (dt == kF16) {
+      if (sigmoid) go_rows(__half{}, rmsnorm_gated_rows_kernel<__half, true, kRowsInFlight>);
+      else go_rows(__half{}, rmsnorm_gated_rows_kernel<__half, false, kRowsInFlight>);
+    } else {
+      if (sigmoid) go_rows(__nv_bfloat16{}, rmsnorm_gated_rows_kernel<__nv_bfloat16, true, kRowsInFlight>);
+      else go_rows(__nv_bfloat16{}, rmsnorm_gated_rows_kernel<__nv_bfloat16, false, kRowsInFlight>);
+    }
+    note_launch();
+    return;
+  }
   const bool vec = width % 4 == 0 && gate_ld % 4 == 0 && align % (dt == kF32 ? 16 : 8) == 0;
   MB200_DISPATCH_FLOAT(dt, {
     if (sigmoid) {

@@ -113,3 +113,18 @@ def test_state_between_other_values():
     ops.check_status()
     assert torch.equal(got[0], got[1]) and torch.equal(plain, odd)
     assert torch.equal(room[:1], before[:1]) and torch.equal(room[-5:], before[-5:])
+
+
+@pytest.mark.parametrize("tokens,heads,width", [(256, 16, 128), (819, 5, 128), (1025, 4, 64), (4097, 1, 8), (700, 6, 120), (4100, 3, 256)])
+@pytest.mark.parametrize("sigmoid", [False, True])
+def test_gated_norm_of_many_rows(tokens, heads, width, sigmoid):
+    """Rows at the edges of a warp's and a block's share, widths that leave lanes idle, a gate inside wider rows: the output's rounding
+    to 8 bits (at most 2^-8 of it) is the largest error of a row, beside 2^-18 for the fast exponential and division."""
+    gen = torch.Generator(device="cuda").manual_seed(tokens)
+    x = torch.randn((tokens, heads, width), generator=gen, device="cuda").bfloat16()
+    rows = torch.randn((tokens, 16 + heads * width), generator=gen, device="cuda").bfloat16()
+    gate, w = rows[:, 8:8 + heads * width], torch.randn(width, generator=gen, device="cuda").bfloat16()
+    got = ops.rmsnorm_gated(x.flatten(1), gate, w, 1e-6, round_norm=False, sigmoid=sigmoid).double().reshape(tokens, heads, width)
+    g = gate.double().reshape(tokens, heads, width)
+    want = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6) * w.double() * (torch.sigmoid(g) if sigmoid else g * torch.sigmoid(g))
+    assert ((got - want).abs() <= (2 ** -8 + 2 ** -18) * want.abs() + 1e-30).all()
