@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(kAttnThreads, FwdCfg<NH>::kCtasPerSm) attn_fwd
     tc_fence_before_sync();
     __syncthreads();  // tile j (and Q) visible to the tensor core
 
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
       const uint32_t qa = smem_u32(sQ);
       const uint32_t ka = smem_u32(sK + buf * kSmemKVBuf);
@@ -426,7 +426,7 @@ __global__ void __launch_bounds__(kAttnThreads, FwdCfg<NH>::kCtasPerSm) attn_fwd
     fence_proxy_async_smem();
     __syncthreads();  // P written by all rows, O rescaled
 
-    if (tid == 0) {
+    if (warp == 0 && elect_one()) {
       tc_fence_after_sync();
       const uint32_t pa = smem_u32(sP);
       const uint32_t va = smem_u32(sV + buf * kSmemKVBuf);
@@ -533,9 +533,7 @@ __device__ __forceinline__ void tma_gather4(void* smem_dst, const CUtensorMap* m
 // next tile is queued behind P V, so a full S barrier says that O is complete too.  Scale and sums take two columns per
 // instruction, the maximum three scores; a masked tile's columns that no row of the warp sees cost nothing.
 // Before, one CTA per SM with two row tiles that shared K and V and kept P in shared memory: 1 x 128 tokens (16 query heads, 8 kv heads)
-// 11.6 us, now 7.9; 1 x 500 18.1, 14.2; 2 x 517 (32, 8) 21.8, 21.1; 8 x 2048 464, 448.  A tile takes 4400 - 5700 cycles, two side by
-// side: 2100 - 2500 from the last probabilities to the next scores (the product's second half, the scores, two handovers), 500 for the
-// maximum, 1600 - 2400 for the exponentials, which two CTAs share.
+// 11.8 us, now 7.5; 1 x 500 18.1, 13.8; 2 x 517 (32, 8) 21.6, 19.6; 8 x 2048 465, 395.
 // ---------------------------------------------------------------------------------------------
 constexpr int kPfThreads = 256;
 constexpr int kPfTile = 128;                    // KV tokens per tile
@@ -723,7 +721,7 @@ attn_prefill_ws_kernel(const __grid_constant__ CUtensorMap tm_k, const __grid_co
       }
       if (bad && p.status != nullptr) atomicExch(p.status, kStatusBadIndex);
       if (!ok_all) *fail_flag = 1;
-    } else if (warp == 5 && lane == 0) {
+    } else if (warp == 5 && elect_one()) {
       // =============================== MMA issuer ===============================
       bool ok_all = mbar_wait(q_full, 0, fail_flag);
       auto wait_on = [&](uint64_t* bar, uint32_t parity) {

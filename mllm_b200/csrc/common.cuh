@@ -51,6 +51,9 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31; }
 
+// One lane of a whole warp.  A role of one thread begins with this and not with a comparison of the lane: behind it the compiler knows
+// that one thread runs, keeps the operands of the tensor instructions in uniform registers and issues them as they are.  Behind
+// `lane == 0` four products with their wait and commit take 580 cycles, behind this 270 (16 stages of 128 x 32 x 64 in a loop).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred = 0;
   asm volatile(

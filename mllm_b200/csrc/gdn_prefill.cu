@@ -457,7 +457,7 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_kernel(const Prefill
     return pp.ws + ((static_cast<int64_t>(b) * pp.span + (c - pp.chunk0)) * p.heads + h) * slot_bytes(p.dv);
   };
   if (warp == kScanWarps) {
-    if (lane == 0) {
+    if (elect_one()) {
       auto load = [&](int c) {
         const int st = (c - pp.chunk0) & 1;
         const uint8_t* src = slot_of(c);

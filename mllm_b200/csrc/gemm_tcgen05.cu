@@ -332,7 +332,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_con
     return static_cast<int>(min(static_cast<int64_t>(gridDim.x) - 1, ((x + 1) * gridDim.x - 1) / total_iters));
   };
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     // ------------------------------ TMA producer ------------------------------
     int stage = 0;
     uint32_t phase = 0;
@@ -400,7 +400,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_con
       *abort_flag = 1;
       if (p.status != nullptr) atomicExch(p.status, kStatusPipelineTimeout);
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1 && elect_one()) {
     // ------------------------------ MMA issuer --------------------------------
     int stage = 0;
     uint32_t phase = 0;
@@ -984,7 +984,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
     if (p.status != nullptr) atomicExch(p.status, code);
   };
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     // ------------------------------ TMA producer (both CTAs) ------------------------------
     const int k_elems_per_block = p.is_int8 ? kRowBytes : kRowBytes / 2;
     const uint32_t full_leader0 = mapa_smem(smem_u32(&full_bar[0]), 0);   // barriers are 8 bytes apart
@@ -1021,7 +1021,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
       }
     }
     if (!ok) give_up(kStatusPipelineTimeout);
-  } else if (warp == 1 && lane == 0 && leader) {
+  } else if (warp == 1 && leader && elect_one()) {
     // ------------------------------ MMA issuer (leader CTA) -------------------------------
     int stage = 0;
     uint32_t phase = 0;

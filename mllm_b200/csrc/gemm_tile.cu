@@ -117,7 +117,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   // Only the producer runs ahead of the stream-order wait.  The roles that wait for its copies begin behind it, so that their limits
   // cover this kernel's own work and not the kernels in front.
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       auto load_w = [&](int s, int kb) {
         uint8_t* at = smem + static_cast<size_t>(s) * kStageBytes;
         mbar_arrive_expect_tx(&full_bar[s], kStageBytes);
@@ -152,11 +152,11 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
     }
   } else if (warp == 1) {
     pdl_wait_loads();
-    if (lane == 0) {
+    if (elect_one()) {
       const uint64_t desc0 = umma_desc_k_sw128(smem_u32(smem));
       bool ok = true;
-      // One thread issues everything: what stands between two products is paid 4 times a stage.  (With the choice of the type between
-      // them and descriptors from 64-bit sums a stage took 880 cycles, of which the products are 250.)
+      // One thread issues everything: what stands between two products is paid four times a stage, so the type is chosen outside and
+      // descriptors are moved, not made
       auto multiply = [&](auto int8_tag) {
         constexpr bool kInt8 = decltype(int8_tag)::value;
         const uint32_t idesc = p.idesc;

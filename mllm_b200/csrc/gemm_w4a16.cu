@@ -192,7 +192,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
     if (p.status != nullptr) atomicExch(p.status, kStatusPipelineTimeout);
   };
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     // ---------------- TMA producer: activations and packed weights ----------------
     int stage = 0, rstage = 0;
     uint32_t phase = 0, rphase = 0;
@@ -226,7 +226,7 @@ w4a16_gemm_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constan
       }
     }
     if (!ok) fail();
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1 && elect_one()) {
     // ---------------- MMA issuer ----------------
     int stage = 0;
     uint32_t phase = 0;

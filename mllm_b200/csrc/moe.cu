@@ -602,7 +602,7 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
     valid = min(BN, o1 - row0);
   };
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -611,7 +611,7 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
       get_item(item, e, row0, valid, tile);
       const int wrow = e * p.n + tile * kBM * C::R;
       for (int kb = 0; kb < p.k_blocks; ++kb) {
-        if (*abort_flag || !mbar_wait(&empty_bar[stage], phase ^ 1)) {
+        if (!mbar_wait(&empty_bar[stage], phase ^ 1, abort_flag)) {
           ok = false;
           break;
         }
@@ -629,7 +629,7 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
       *abort_flag = 1;
       if (p.status != nullptr) atomicExch(p.status, kStatusPipelineTimeout);
     }
-  } else if (warp == 1 && lane == 0) {
+  } else if (warp == 1 && elect_one()) {
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -644,7 +644,7 @@ moe_grouped_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_c
       tc_fence_after_sync();
       const uint32_t d_base = tmem_base + acc * C::kAccCols;
       for (int kb = 0; kb < p.k_blocks; ++kb) {
-        if (*abort_flag || !mbar_wait(&full_bar[stage], phase)) {
+        if (!mbar_wait(&full_bar[stage], phase, abort_flag)) {
           ok = false;
           break;
         }

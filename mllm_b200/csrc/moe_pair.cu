@@ -152,7 +152,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
   };
   int row0, row_end, wrow, tc;
 
-  if (warp == 0 && lane == 0) {
+  if (warp == 0 && elect_one()) {
     const uint32_t full_leader0 = mapa_smem(smem_u32(&full_bar[0]), 0);
     int stage = 0;
     uint32_t phase = 0;
@@ -175,7 +175,7 @@ moe_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant_
       }
     }
     if (!ok) give_up();
-  } else if (warp == 1 && lane == 0 && leader) {
+  } else if (warp == 1 && leader && elect_one()) {
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
