@@ -58,6 +58,7 @@ struct KParams {
   int is_int8;
   int row_static;        // swap tiling: the row operand (weights) is not written by earlier kernels of the stream
   int cluster_k;         // swap tiling: > 1 = the k range of a tile is split over the CTAs of a cluster of this size
+  int pair_bn;           // two-CTA tiling: columns of a tile
   int early_trigger;     // swap tiling: let the kernels behind this one start their set-up as soon as this one runs
   uint32_t idesc;
   // ---- tensor-parallel fusion (normal tiling only) ----
@@ -933,6 +934,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
   const uint32_t rank = cluster_ctarank();
+  const int bn = kGated<SWIGLU> ? kPairBN : p.pair_bn;      // a gated tile holds a block of gate rows and one of up rows
   const bool leader = rank == 0;
 
   if (threadIdx.x == 0) {
@@ -994,7 +996,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
     int tr, tc;
     for (int idx = 0; ok && get_tile(idx, tr, tc); ++idx) {
       const int row0 = tr * 2 * kBM + static_cast<int>(rank) * kBM;       // this CTA's 128 activation rows
-      const int col0 = tc * kPairBN + static_cast<int>(rank) * (kPairBN / 2);  // this CTA's 128 weight rows
+      const int col0 = tc * bn + static_cast<int>(rank) * (bn / 2);       // this CTA's weight rows
       if (p.gate_flags != nullptr && row0 < p.m) {
         if (!wait_flag_ge(p.gate_flags + (row0 >> 7), p.gate_epoch, p.status)) {
           give_up(kStatusPeerTimeout);
@@ -1010,7 +1012,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
         }
         uint8_t* stage_base = smem + static_cast<size_t>(stage) * kPairStageBytes;
         const uint32_t full_leader = full_leader0 + static_cast<uint32_t>(stage) * 8u;
-        if (leader) mbar_arrive_expect_tx(&full_bar[stage], 2 * kPairStageBytes);
+        if (leader) mbar_arrive_expect_tx(&full_bar[stage], (2 * kBM + bn) * kRowBytes);
         const int x = kb * k_elems_per_block;
         tma_load_2d_pair(stage_base, &tm_row, full_leader, x, row0);
         tma_load_2d_pair(stage_base + kBM * kRowBytes, &tm_col, full_leader, x, col0);
@@ -1115,7 +1117,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
     const int row_in_tile = ew * 32 + lane;
     bool ok = true;
     int tr, tc;
-    constexpr int kOutCols = kGated<SWIGLU> ? kPairBN / 2 : kPairBN;
+    const int out_cols = kGated<SWIGLU> ? kPairBN / 2 : bn;
     const int n_out = kGated<SWIGLU> ? p.n / 2 : p.n;
     float* col_scale = reinterpret_cast<float*>(epi_staging + ew * (32 * kStageRowBytes));     // of this warp; 8-bit only
     for (int idx = 0; ok && get_tile(idx, tr, tc); ++idx) {
@@ -1123,7 +1125,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
       const uint32_t acc_phase = (idx >> 1) & 1;
       const int64_t row = static_cast<int64_t>(tr) * 2 * kBM + static_cast<int64_t>(rank) * kBM + row_in_tile;
       const bool row_ok = row < p.m;
-      const int64_t col0 = static_cast<int64_t>(tc) * kOutCols;
+      const int64_t col0 = static_cast<int64_t>(tc) * out_cols;
       float sa = 1.f;
       if (p.is_int8) {
         // The tile's scales come while its products are formed, the weights' by way of shared memory.  Loaded where they are used, one
@@ -1133,7 +1135,10 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
         if (p.rs_tp == 0) {
           __syncwarp();        // every lane has used the scales of the tile before
 #pragma unroll
-          for (int i = 0; i < kPairBN / 32; ++i) col_scale[i * 32 + lane] = p.b_scale[static_cast<int64_t>(tc) * kPairBN + i * 32 + lane];
+          for (int i = 0; i < kPairBN / 32; ++i) {
+            const int64_t at = static_cast<int64_t>(tc) * bn + i * 32 + lane;
+            if (i * 32 < bn) col_scale[i * 32 + lane] = at < p.n ? p.b_scale[at] : 0.f;
+          }
           __syncwarp();
         }
       }
@@ -1155,7 +1160,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
           const int64_t dst_row0 = static_cast<int64_t>(local_tile) * kBM + ew * 32;
           const int64_t tile_row0 = static_cast<int64_t>(tr128) * kBM + ew * 32;
 #pragma unroll 1
-          for (int c = 0; c < kOutCols; c += 64) {
+          for (int c = 0; c < out_cols; c += 64) {
             uint32_t packed[32];
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
@@ -1203,7 +1208,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
       auto store_tile = [&](auto int8_tag) {
         constexpr bool kInt8 = decltype(int8_tag)::value;
 #pragma unroll 1
-        for (int c = 0; c < kOutCols; c += 32) {
+        for (int c = 0; c < out_cols; c += 32) {
           uint32_t r0[32], r1[32];
           tmem_ld_32x32(t_base + c, r0);
           if constexpr (kGated<SWIGLU>) tmem_ld_32x32(t_base + kPairBN / 2 + c, r1);
@@ -1441,11 +1446,24 @@ int launch_gemm(const GemmArgs& a, cudaStream_t s) {
     if (pair_knob && a.n % 256 == 0 && tiles_pair >= num_sms / 2 && pair_rs_ok) {
       if (a.rs_tp > 0) p.rs_shift = rs_first_owner * (p.rs_tiles_per_rank / 2);
       p.tiles_r = (a.m + 2 * kBM - 1) / (2 * kBM);
-      p.tiles_c = (a.n + kPairBN - 1) / kPairBN;
-      p.idesc = umma_idesc(2 * kBM, kPairBN, c_fmt, ab_fmt, ab_fmt);
+      p.pair_bn = kPairBN;
+      if (!gated && a.rs_tp == 0) {
+        // A last round of few tiles takes as long as a full one.  Narrower tiles where they make the rounds times the width of a tile
+        // less, beside what a tile costs at any width (some four k blocks of 256 columns).  1551 rows, 7 row tiles on 74 pairs of SMs, with
+        // 256 and with 224 columns: 6144 x 4096 67.5 and 64.4 us, 4096 x 4096 45.4 and 43.3, 4096 x 12288 131 and 127
+        const int64_t pairs_all = num_sms / 2;
+        auto cost = [&](int bn) {
+          const int64_t tiles = static_cast<int64_t>(p.tiles_r) * ((a.n + bn - 1) / bn);
+          return (tiles + pairs_all - 1) / pairs_all * (static_cast<int64_t>(p.k_blocks) * bn + 4 * kPairBN);
+        };
+        for (const int bn : {224, 192})
+          if (cost(bn) * 100 < cost(p.pair_bn) * 98) p.pair_bn = bn;
+      }
+      p.tiles_c = (a.n + p.pair_bn - 1) / p.pair_bn;
+      p.idesc = umma_idesc(2 * kBM, p.pair_bn, c_fmt, ab_fmt, ab_fmt);
       if (!make_operand_map(&tm_row, a.a, a.m, a.k, a.lda, eb, type, kBM)) return -2;
-      if (!make_operand_map(&tm_col, a.b, a.n, a.k, a.ldb, eb, type, kPairBN / 2)) return -2;
-      const int pairs = static_cast<int>(std::min<int64_t>(tiles_pair, num_sms / 2));
+      if (!make_operand_map(&tm_col, a.b, a.n, a.k, a.ldb, eb, type, p.pair_bn / 2)) return -2;
+      const int pairs = static_cast<int>(std::min<int64_t>(static_cast<int64_t>(p.tiles_r) * p.tiles_c, num_sms / 2));
       if (relu2) return launch_pair_cfg<3>(tm_row, tm_col, p, pairs, s);
       if (a.swiglu == 2) return launch_pair_cfg<2>(tm_row, tm_col, p, pairs, s);
       if (clamped) return launch_pair_cfg<4>(tm_row, tm_col, p, pairs, s);

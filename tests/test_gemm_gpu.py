@@ -196,3 +196,26 @@ def test_add_rmsnorm_fused_into_the_streaming_gemm(monkeypatch, m, n, k, swiglu,
     h9 = (s9_want.float() * torch.rsqrt(s9_want.float().pow(2).mean(-1, keepdim=True) + 1e-6) * nw.float()).to(dt)
     want9 = ref.linear_swiglu(h9.float(), w.float(), 0) if swiglu else ref.linear(h9, w, out_dtype=torch.float32)
     assert _rel_err(y9, want9) < 8e-3
+
+
+@pytest.mark.parametrize("m,n,k", [(1551, 4096, 512), (1100, 5120, 512), (1100, 5120, 2048), (1300, 4352, 256)])
+@pytest.mark.parametrize("kind", ["bf16", "fp16", "int8"])
+def test_gemm_pair_tiles_of_other_widths(m, n, k, kind):
+    """Tiles of 224 and 192 columns of the two-CTA tiling, whose last tile ends inside the matrix.  Products of 16-bit values are exact in
+    fp32; beside the output's rounding the sums' order shows, below 2^-20 of the sum of the magnitudes at these k."""
+    g = torch.Generator(device=DEV).manual_seed(m + n)
+    if kind == "int8":
+        x, w = (torch.randint(-127, 128, (r, k), generator=g, device=DEV, dtype=torch.int8) for r in (m, n))
+        sx, sw = torch.rand(m, generator=g, device=DEV), torch.rand(n, generator=g, device=DEV)
+        got = ops.int8_scaled_mm(x, w, sx, sw, torch.bfloat16).double()
+        want = (x.double() @ w.double().t()) * sx.double()[:, None] * sw.double()
+        assert ((got - want).abs() <= (2 ** -8 + 2 ** -20) * want.abs()).all()
+        return
+    dtype, u = (torch.bfloat16, 2 ** -8) if kind == "bf16" else (torch.float16, 2 ** -11)
+    x, w = (torch.randn((r, k), generator=g, device=DEV).to(dtype) for r in (m, n))
+    b, r = torch.randn(n, generator=g, device=DEV).to(dtype), torch.randn((m, n), generator=g, device=DEV).to(dtype)
+    size = x.double().abs() @ w.double().abs().t()
+    plain = x.double() @ w.double().t()
+    for got, want in ((ops.linear(x, w), plain), (ops.linear(x, w, b, residual=r), plain + b.double() + r.double())):
+        assert ((got.double() - want).abs() <= u * want.abs() + 2 ** -20 * (size + want.abs())).all()
+    ops.check_status()
