@@ -9,6 +9,9 @@
 //     taken from the longest length the host allows for, and roles that meet at mbarriers, took 87.5 us for 29 requests of 400 to
 //     3400 tokens and 8 kv heads, 128 us for 64 x 2048 and 4 heads, 25.9 us for 8 x 2048 and 8 heads; now 44.1, 53.9 and 20.7 us,
 //     joining included; the bytes take 34, 40 and 10 us.)
+//     The chain in front of the first copy (lengths, table, rows; queries and the table's row beside them; no 64-bit division) and the
+//     meeting of the warps are 4 us of a CTA's time when each load waits for the one before; side by side, and four values a thread:
+//     2 x 1500 (8 kv heads) 11.4 -> 9.3 us, 8 x 2048 20.9 -> 18.2, 1 x 160 7.3 -> 6.8, 29 x 1900 46.0 -> 42.2, joining included.
 //   * A warp owns 16 tokens of a tile and a ring of its own that cp.async fills two tiles ahead: 128 KB are in flight per SM,
 //     and no barrier stands between the arrival of a tile and its use.  Rows come by slot one by one (16 lanes a row), so
 //     a page size of 1 costs what a page size of 16 does.  The TMA engine's gather fell to half the speed there.
@@ -56,8 +59,7 @@ __device__ __forceinline__ int first_key(const DecodeParams& p, int len) {
   if (p.window > 0) return max(0, len - p.window);
   return p.chunk > 0 ? (len - 1) / p.chunk * p.chunk : 0;
 }
-__device__ __forceinline__ int tiles_of(const DecodeParams& p, int b) {
-  const int len = __ldcg(p.seq_lens + b);
+__device__ __forceinline__ int tiles_of(const DecodeParams& p, int len) {
   if (len <= 0) return 0;
   const int lo = first_key(p, len) & ~(kWarpTokens - 1);
   return (len - lo + kTile - 1) / kTile;
@@ -71,7 +73,7 @@ __device__ __forceinline__ int tiles_of(const DecodeParams& p, int b) {
 // kv head).
 constexpr int kStart = 2;
 __device__ __forceinline__ int units_of(const DecodeParams& p, int b) {
-  const int n = tiles_of(p, b);
+  const int n = tiles_of(p, __ldcg(p.seq_lens + b));
   return n > 0 ? n + kStart : 0;
 }
 __device__ __forceinline__ int scan_tiles(const DecodeParams& p, int* warp_sums, int& first, int& last, int& total) {
@@ -104,7 +106,11 @@ __device__ __forceinline__ int ctas_used(const DecodeParams& p, int64_t line) {
   const int64_t want = max(line / 4, min(line / 2, static_cast<int64_t>(64)));
   return static_cast<int>(min(static_cast<int64_t>(p.ctas), max(want, static_cast<int64_t>(1))));
 }
-__device__ __forceinline__ int64_t run_begin(int64_t line, int c, int ctas) { return line * c / ctas; }
+__device__ __forceinline__ int64_t run_begin(int64_t line, int c, int ctas) {
+  // a division of 64 bits takes some 500 cycles of the chain in front of the first copy
+  if (line < 0xFFFFFFFFll / (ctas + 1)) return static_cast<uint32_t>(line) * static_cast<uint32_t>(c) / static_cast<uint32_t>(ctas);
+  return line * c / ctas;
+}
 
 __device__ __forceinline__ uint32_t movmatrix(uint32_t v) {
   uint32_t r;
@@ -125,6 +131,7 @@ struct Cfg {
   static constexpr int kOutStride = HD + 4;                      // floats between the heads of a partial result: no bank conflicts
   static constexpr int kSmem = kWarps * kRingBytes + 128;
   static constexpr int kPerSm = HD == 256 ? 1 : 2;
+  static_assert(kOutStride % 4 == 0 && kRingBytes % 16 == 0, "partial results are read four values at a time");
   static_assert(NT * 8 * kOutStride * 4 <= kRingBytes, "a warp's partial result must fit its ring");
 };
 
@@ -133,17 +140,21 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
   using C = Cfg<HD, NT>;
   extern __shared__ uint8_t smem_raw[];
   __shared__ int warp_sums[kWarps];
-  __shared__ int start[3];                          // where the run begins: request, kv head, tile
+  __shared__ int start[5];                          // where the run begins: request, kv head, tile; its length and row of the table
   __shared__ float part_m[kWarps][NT * 8], part_l[kWarps][NT * 8];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = p.group;
   pdl_wait_loads();
   pdl_launch_dependents();   // the joining kernel may lay out the line while this one streams
 
-  int b, hk, t0;
+  // What stands between here and the first copy is a chain of round trips: lengths, then the table, then the rows.  Everything else
+  // (the table's row, the queries) is on its way beside them.
+  int b, hk, t0, len, row;
   int64_t left;
   {
     int first, last, total;
+    const int mine = min(p.batch - 1, static_cast<int>(threadIdx.x) * ((p.batch + kThreads - 1) / kThreads));
+    const int my_row = __ldcg(p.req_pool_indices + mine);       // of the first of this thread's requests
     const int before = scan_tiles(p, warp_sums, first, last, total);
     const int64_t line = static_cast<int64_t>(total) * p.hkv;
     const int used = ctas_used(p, line);
@@ -155,10 +166,12 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
     for (int r = first; r < last; ++r) {
       const int n = units_of(p, r);
       if (begin >= at && begin < at + static_cast<int64_t>(n) * p.hkv) {
-        const int in = static_cast<int>(begin - at);
+        const int in = static_cast<int>(begin - at), h = in / n;
         start[0] = r;
-        start[1] = in / n;
-        start[2] = in % n;
+        start[1] = h;
+        start[2] = in - h * n;
+        start[3] = __ldcg(p.seq_lens + r);
+        start[4] = r == first ? my_row : __ldcg(p.req_pool_indices + r);
       }
       at += static_cast<int64_t>(n) * p.hkv;
     }
@@ -166,6 +179,8 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
     b = start[0];
     hk = start[1];
     t0 = start[2];
+    len = start[3];
+    row = start[4];
   }
 
   uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~uintptr_t(127)) + warp * C::kRingBytes;
@@ -175,9 +190,12 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
   bool at_run_begin = true;
 
   while (left > 0) {
-    const int len = __ldcg(p.seq_lens + b);
+    if (!at_run_begin) {
+      len = __ldcg(p.seq_lens + b);
+      row = __ldcg(p.req_pool_indices + b);
+    }
     const int key0 = first_key(p, len);
-    const int n_all = tiles_of(p, b);
+    const int n_all = tiles_of(p, len);
     if (t0 >= n_all) {          // behind a pair's tiles, or a request without a token
       if (n_all > 0) left -= n_all + kStart - t0;
       t0 = 0;
@@ -190,7 +208,7 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
     }
     const int n = static_cast<int>(min(static_cast<int64_t>(n_all - t0), left));
     const int base0 = (key0 & ~(kWarpTokens - 1)) + t0 * kTile + warp * kWarpTokens;   // first token of this warp's first tile
-    const int* rtt = p.req_to_token + static_cast<int64_t>(p.req_pool_indices[b]) * p.rtt_stride;
+    const int* rtt = p.req_to_token + static_cast<int64_t>(row) * p.rtt_stride;
     const T* kbase = static_cast<const T*>(p.k_cache) + hk * p.kv_head_stride;
     const T* vbase = static_cast<const T*>(p.v_cache) + hk * p.kv_head_stride;
 
@@ -198,10 +216,26 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
       const int tok = base0 + t * kTile + (lane & 15);
       return (t < n && tok < len) ? __ldcg(rtt + tok) : kNoToken;
     };
-    int slot_next = slot_of(0);
-    auto issue = [&](int t) {
+    int ahead[C::kStages - 1];              // the slots of the first tiles, in one round trip
+#pragma unroll
+    for (int t = 0; t < C::kStages - 1; ++t) ahead[t] = slot_of(t);
+    int slot_next = slot_of(C::kStages - 1);
+    // the queries of the group as the column operand: head nt * 8 + lane / 4, features 2 (lane % 4) of every 8
+    uint32_t qf[HD / 16][NT][2];
+    {
+      const T* q = static_cast<const T*>(p.q) + b * p.q_stride + static_cast<int64_t>(hk) * g * HD;
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt) {
+        const int h = nt * 8 + (lane >> 2);
+#pragma unroll
+        for (int kk = 0; kk < HD / 16; ++kk)
+#pragma unroll
+          for (int i = 0; i < 2; ++i)
+            qf[kk][nt][i] = h < g ? __ldcg(reinterpret_cast<const uint32_t*>(q + h * HD + kk * 16 + i * 8 + 2 * (lane & 3))) : 0u;
+      }
+    }
+    auto issue = [&](int t, int s) {
       if (t < n) {
-        int s = slot_next;
         if (s < 0 || s >= p.num_slots) {
           bad = bad || s != kNoToken;
           s = -1;
@@ -221,25 +255,9 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
         }
       }
       cp_commit();
-      slot_next = slot_of(t + 1);
     };
 #pragma unroll
-    for (int t = 0; t < C::kStages - 1; ++t) issue(t);
-
-    // the queries of the group as the column operand: head nt * 8 + lane / 4, features 2 (lane % 4) of every 8
-    uint32_t qf[HD / 16][NT][2];
-    {
-      const T* q = static_cast<const T*>(p.q) + b * p.q_stride + static_cast<int64_t>(hk) * g * HD;
-#pragma unroll
-      for (int nt = 0; nt < NT; ++nt) {
-        const int h = nt * 8 + (lane >> 2);
-#pragma unroll
-        for (int kk = 0; kk < HD / 16; ++kk)
-#pragma unroll
-          for (int i = 0; i < 2; ++i)
-            qf[kk][nt][i] = h < g ? __ldcg(reinterpret_cast<const uint32_t*>(q + h * HD + kk * 16 + i * 8 + 2 * (lane & 3))) : 0u;
-      }
-    }
+    for (int t = 0; t < C::kStages - 1; ++t) issue(t, ahead[t]);
     float o[HD / 16][NT][4];
     float m[NT][2], l[NT][2];
 #pragma unroll
@@ -255,7 +273,8 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
     for (int t = 0; t < n; ++t) {
       cp_wait<C::kStages - 2>();
       __syncwarp();
-      issue(t + C::kStages - 1);      // into the stage of the tile before, which every lane has left
+      issue(t + C::kStages - 1, slot_next);      // into the stage of the tile before, which every lane has left
+      slot_next = slot_of(t + C::kStages);
       const int base = base0 + t * kTile;
       if (base >= len) continue;
       const uint32_t sk = ring_addr + (t % C::kStages) * (2 * C::kTensorBytes);
@@ -380,23 +399,30 @@ __global__ void __launch_bounds__(kThreads, Cfg<HD, NT>::kPerSm) attn_decode_str
     const int64_t part = (static_cast<int64_t>(blockIdx.x) * 2 + (at_run_begin ? 0 : 1)) * g;
     const float* parts = reinterpret_cast<const float*>(ring - warp * C::kRingBytes);
     // a sum of 0: no key to be seen.  A NaN or infinite score makes it NaN, and that the result
-    for (int i = threadIdx.x; i < g * HD; i += kThreads) {
-      const int h = i / HD, d = i % HD;
+    for (int i = threadIdx.x; i < g * (HD / 4); i += kThreads) {
+      const int h = i / (HD / 4), d = i % (HD / 4) * 4;
       float top = part_m[0][h];
 #pragma unroll
       for (int w = 1; w < kWarps; ++w) top = fmaxf(top, part_m[w][h]);
-      float den = 0.f, acc = 0.f;
+      float den = 0.f, acc[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) {
         const float f = part_m[w][h] == -INFINITY ? 0.f : exp2f(part_m[w][h] - top);
+        const float4 v = *reinterpret_cast<const float4*>(parts + w * (C::kRingBytes / 4) + h * C::kOutStride + d);
         den += f * part_l[w][h];
-        acc += f * parts[w * (C::kRingBytes / 4) + h * C::kOutStride + d];
+        acc[0] += f * v.x;
+        acc[1] += f * v.y;
+        acc[2] += f * v.z;
+        acc[3] += f * v.w;
       }
       if (whole) {
         if (p.sink != nullptr) den += exp2f(p.sink[hk * g + h] * kLog2e - top);
-        static_cast<T*>(p.out)[b * p.out_stride + static_cast<int64_t>(hk * g + h) * HD + d] = from_f32<T>(den == 0.f ? 0.f : acc / den);
+        T* out = static_cast<T*>(p.out) + b * p.out_stride + static_cast<int64_t>(hk * g + h) * HD + d;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) out[e] = from_f32<T>(den == 0.f ? 0.f : acc[e] / den);
       } else {
-        p.part_o[(part + h) * HD + d] = den == 0.f ? 0.f : acc / den;
+        *reinterpret_cast<float4*>(p.part_o + (part + h) * HD + d) =
+            den == 0.f ? make_float4(0.f, 0.f, 0.f, 0.f) : make_float4(acc[0] / den, acc[1] / den, acc[2] / den, acc[3] / den);
         if (d == 0) p.part_lse[part + h] = den == 0.f ? -INFINITY : top + log2f(den);
       }
     }
@@ -424,7 +450,7 @@ __global__ void __launch_bounds__(kThreads) attn_decode_join_kernel(const Decode
   if (b >= first && b < last) {
     for (int r = first; r < b; ++r) before += units_of(p, r);
     mine[0] = before;
-    mine[1] = tiles_of(p, b);
+    mine[1] = tiles_of(p, __ldcg(p.seq_lens + b));
   }
   __syncthreads();
   const int64_t line = static_cast<int64_t>(total) * p.hkv;
@@ -445,11 +471,20 @@ __global__ void __launch_bounds__(kThreads) attn_decode_join_kernel(const Decode
   }
   if (c0 == c1) return;         // one CTA had all of it and has written the output
   const float sink = p.sink != nullptr ? p.sink[head] * kLog2e : -INFINITY;
+  constexpr int kPer = (HD + kThreads - 1) / kThreads, kEarly = 8;
+  // the values of the first CTAs are on their way beside the sums that weigh them
+  float early[kEarly][kPer];
+#pragma unroll
+  for (int i = 0; i < kEarly; ++i)
+#pragma unroll
+    for (int k = 0; k < kPer; ++k) {
+      const int d = threadIdx.x + k * kThreads;
+      early[i][k] = c0 + i <= c1 && d < HD ? __ldcg(p.part_o + slot(c0 + i) * HD + d) : 0.f;
+    }
   float top = sink, den = 0.f;
   for (int c = c0 + static_cast<int>(threadIdx.x & 31); c <= c1; c += 32) top = fmaxf(top, __ldcg(p.part_lse + slot(c)));
   top = warp_max(top);
   if (p.sink != nullptr) den = exp2f(sink - top);
-  constexpr int kPer = (HD + kThreads - 1) / kThreads;
   float acc[kPer] = {};
   for (int at = c0; at <= c1; at += kThreads) {
     const int m = min(kThreads, c1 + 1 - at);
@@ -459,8 +494,20 @@ __global__ void __launch_bounds__(kThreads) attn_decode_join_kernel(const Decode
       weight[threadIdx.x] = lse == -INFINITY ? 0.f : exp2f(lse - top);
     }
     __syncthreads();
+    int from = 0;
+    if (at == c0) {
+#pragma unroll
+      for (int i = 0; i < kEarly; ++i) {
+        if (i >= m) break;
+        const float w = weight[i];
+        den += w;
+#pragma unroll
+        for (int k = 0; k < kPer; ++k) acc[k] += w * early[i][k];
+      }
+      from = min(kEarly, m);
+    }
 #pragma unroll 8
-    for (int i = 0; i < m; ++i) {
+    for (int i = from; i < m; ++i) {
       const float w = weight[i];
       den += w;
 #pragma unroll
