@@ -315,11 +315,11 @@ int launch_stream(const GemmArgs& a, cudaStream_t s) {
   p.ld_res = a.ld_res;
   const int sms = std::max(1, a.num_sms);
   switch (a.swiglu) {
-    case 0: return stream::launch<F16, stream::kHalf, stream::kNone>(p, sms, s);
-    case 1: return stream::launch<F16, stream::kHalf, stream::kSilu>(p, sms, s);
-    case 2: return stream::launch<F16, stream::kHalf, stream::kGelu>(p, sms, s);
-    case 3: return stream::launch<F16, stream::kHalf, stream::kRelu2>(p, sms, s);
-    case 4: return stream::launch<F16, stream::kHalf, stream::kClamped>(p, sms, s);
+    case 0: return stream::launch<F16, stream::kNone>(p, sms, s);
+    case 1: return stream::launch<F16, stream::kSilu>(p, sms, s);
+    case 2: return stream::launch<F16, stream::kGelu>(p, sms, s);
+    case 3: return stream::launch<F16, stream::kRelu2>(p, sms, s);
+    case 4: return stream::launch<F16, stream::kClamped>(p, sms, s);
   }
   return 1;
 }

@@ -1,26 +1,20 @@
-// out[m, n] = x[m, k] * W[n, k]^T for up to 8 rows of x, the weights in 16 bits or in packed 4 bits with group scales: the
-// projections of a decode step.
+// out[m, n] = x[m, k] * W[n, k]^T for up to 8 rows of x and 16-bit weights: the projections of a decode step.  (Packed 4-bit weights:
+// gemm_smallm_w4.cu.)
 //
 // The product is a stream of the weight matrix; what costs time beside its bytes is everything that keeps the stream from
 // running: the launch, the first round trip to memory, the exchange of partial sums at the end.
 //   * A unit is 16 weight rows over the CTA's part of k, the row operand of warp-level MMAs (m16n8k16) whose 8 columns are
-//     the rows of x.  The 8 warps take the k steps of a unit in turn (32 k of 16-bit weights, 128 k of 4-bit ones: 16 bytes of
-//     row g and of row g + 8 per lane).  k is permuted alike for both operands, which a dot product does not notice, so a lane's
-//     16 bytes are its fragments as they come.
+//     the rows of x.  The 8 warps take the k steps of a unit in turn (32 k: 16 bytes of row g and of row g + 8 per
+//     lane).  k is permuted alike for both operands, which a dot product does not notice, so a lane's 16 bytes are its fragments as they
+//     come.
 //   * The rows of x are loaded once, into registers: a warp only ever meets its own k steps.  So there is nothing to stage, no
 //     barrier before the first product, and the shared memory of a CTA is the copy queue alone: per lane a ring of cp.async
 //     copies that the lane itself reads back, 48 KB per CTA, two CTAs per SM.
-//   * k that needs more registers than that (16-bit: over 4096, 4-bit: over 4096) is cut over a cluster; its CTAs keep the sums
-//     of all their units in shared memory and exchange them once, through distributed shared memory, at the end.
+//   * k that needs more registers than that (over 4096) is cut over a cluster; its CTAs keep the sums of all their units in shared
+//     memory and exchange them once, through distributed shared memory, at the end.
 //   * Every kernel of the chain lets the next one start as soon as it runs itself.  With half an SM per CTA the CTAs of the next
 //     product move in as these leave, and fill their rings with weights, which no kernel writes, before they wait for their
 //     input: the end of one stream and the start of the next overlap.
-//   * 4-bit weights: a nibble under an exponent's bits is base + q; one operation per pair takes base and zero point off, exactly,
-//     and the group's scale multiplies the fp32 sum of the group's step, so nothing of a weight is rounded (rounding the product of q
-//     and scale to 16 bits cost four operations more per eight weights, and precision).  In bf16 that operation also divides by 2048,
-//     which the sums get back at their end: a group's sum is then no larger than the largest x in it, and x may be as large as the
-//     type allows.  (Taking the base off the sum, as base times the sum of x, turns an infinite x into NaN:
-//     2 rows of 24576 x 4096 24.6 us that way, 24.2 this way, with zero points 26.3 and 25.7.)
 #pragma once
 
 #include "common.cuh"
@@ -38,14 +32,11 @@ constexpr int kRingBytes = kWarps * kDepth * kSlotBytes;  // 48 KB
 struct Params {
   const uint8_t* x;
   const uint8_t* w;
-  const uint8_t* scales;    // 4-bit: [n, groups] 16-bit
-  const uint8_t* zeros;     // 4-bit: [n, groups] bytes, or null (zero point 8)
   const void* bias;
   const void* residual;
   void* out;
   int m, n;
   int steps;                // k steps of the whole row
-  int groups, steps_per_group;
   int units, units_per_cluster, cluster;
   int up_rows;              // gated: rows between a gate row and its up row inside a block of gate_block rows
   int gate_block;           // gated: gate rows of a block, followed by as many up rows
@@ -83,29 +74,6 @@ __device__ __forceinline__ void mma(float (&c)[4], uint32_t a0, uint32_t a1, uin
                  : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
-// A pair of nibbles under the exponent's bits, base + q, to q - zero (fp16, base 1024) or (q - zero) / 2048 (bf16, base 128); both are
-// exact.  `off2`: base + zero, or -(base + zero) / 2048
-constexpr float kScaled = 2048.f;
-template <bool F16>
-__device__ __forceinline__ uint32_t expand(uint32_t v, uint32_t off2) {
-  constexpr uint32_t kMagic = F16 ? 0x64006400u : 0x43004300u;
-  v = (v & 0x000F000Fu) | kMagic;
-  if constexpr (F16) {
-    const __half2 r = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&off2));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  } else {
-    const __nv_bfloat162 r = __hfma2(*reinterpret_cast<const __nv_bfloat162*>(&v), __float2bfloat162_rn(1.f / kScaled),
-                                     *reinterpret_cast<const __nv_bfloat162*>(&off2));
-    return *reinterpret_cast<const uint32_t*>(&r);
-  }
-}
-// what `expand` takes off for a zero point: the bits of 1024 + zero, or of -(128 + zero) / 2048, whose last place is 2 / 2048 from
-// zero points of 128 on.  (Conversions from fp32 instead: 2 rows of 24576 x 4096 26.2 us, so 25.7.)
-template <bool F16>
-__device__ __forceinline__ uint32_t zero_bits(int zero) {
-  if constexpr (F16) return (0x6400u + zero) * 0x10001u;
-  return (0xBD80u + zero - ((max(zero, 128) - 127) >> 1)) * 0x10001u;
-}
 __device__ __forceinline__ uint32_t cluster_rank() {
   uint32_t r;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
@@ -123,13 +91,10 @@ __device__ __forceinline__ float ld_peer(uint32_t local, uint32_t rank) {
   return v;
 }
 
-// 16-bit weights, or 4-bit ones: in the nibble order of ops.w4a16_interleave or in natural order, with a zero point of 8 or with zero
-// points.  JX: k steps of one warp that the registers hold x for
-enum Weights { kHalf = 0, kInt4 = 1, kInt4Natural = 2, kInt4Zeros = 3, kInt4NaturalZeros = 4 };
-template <bool F16, int WT, int ACT, int JX>
+// JX: k steps of one warp that the registers hold x for
+template <bool F16, int ACT, int JX>
 __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p) {
-  constexpr bool W4 = WT != kHalf, kNatural = WT == kInt4Natural || WT == kInt4NaturalZeros, kZeros = WT == kInt4Zeros || WT == kInt4NaturalZeros;
-  constexpr int kStepK = W4 ? 128 : 32;                  // k of a step
+  constexpr int kStepK = 32;                             // k of a step
   constexpr int kStepBytes = 64;                         // of one weight row
   constexpr int kXRegs = kStepK / 8;                     // registers of x per step: a lane's quarter of the step, two k each
   constexpr bool kGated = kGatedAct<ACT>;
@@ -183,40 +148,12 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
   };
   auto commit = [&]() { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
-  // 4-bit: scales (and zero points) of the steps of one unit, fetched a unit ahead
-  constexpr int kSc = W4 ? JX : 1;
-  uint16_t sc0[kSc], sc1[kSc];
-  uint8_t z0[kZeros ? kSc : 1], z1[kZeros ? kSc : 1];
-  int group_of[kSc];
-  if constexpr (W4) {
-#pragma unroll
-    for (int j = 0; j < JX; ++j) group_of[j] = min(s0 + j * kWarps + warp, p.steps - 1) / p.steps_per_group;
-  }
-  auto fetch_scales = [&](int u) {
-    if constexpr (W4) {
-      const int64_t r0 = row_of(u) * p.groups, r1 = second(row_of(u)) * p.groups;
-#pragma unroll
-      for (int j = 0; j < JX; ++j) {
-        if (j < J) {
-          const int grp = group_of[j];
-          sc0[j] = __ldg(reinterpret_cast<const uint16_t*>(p.scales) + r0 + grp);
-          sc1[j] = __ldg(reinterpret_cast<const uint16_t*>(p.scales) + r1 + grp);
-          if constexpr (kZeros) {
-            z0[j] = __ldg(p.zeros + r0 + grp);
-            z1[j] = __ldg(p.zeros + r1 + grp);
-          }
-        }
-      }
-    }
-  };
-
   if (!p.w_static) pdl_wait_loads();
 #pragma unroll
   for (int i = 0; i < kDepth - 1; ++i) {
     if (i < total) issue();
     commit();          // one group per step, empty past the end
   }
-  if (u0 < u1) fetch_scales(u0);
   if (p.w_static) pdl_wait_loads();
 
   uint32_t x[JX][kXRegs];
@@ -268,20 +205,6 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
   int slot = 0, buf = 0, done = 0;
   for (int u = u0; u < u1; ++u) {
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
-    uint32_t o0[kZeros ? kSc : 1], o1[kZeros ? kSc : 1];
-    float f0[kSc], f1[kSc];
-    if constexpr (W4) {
-#pragma unroll
-      for (int j = 0; j < JX; ++j) {
-        f0[j] = half_to_f<F16>(sc0[j]);
-        f1[j] = half_to_f<F16>(sc1[j]);
-        if constexpr (kZeros) {
-          o0[j] = zero_bits<F16>(z0[j]);
-          o1[j] = zero_bits<F16>(z1[j]);
-        }
-      }
-      if (u + 1 < u1) fetch_scales(u + 1);
-    }
 #pragma unroll
     for (int j = 0; j < JX; ++j) {
       if (j < J) {
@@ -293,35 +216,8 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
           uint4 a, b;
           asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w) : "r"(at) : "memory");
           asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(b.x), "=r"(b.y), "=r"(b.z), "=r"(b.w) : "r"(at + 512) : "memory");
-          if constexpr (W4) {
-            float s[2][4] = {};
-            const uint32_t oa = kZeros ? o0[kZeros ? j : 0] : zero_bits<F16>(8), ob = kZeros ? o1[kZeros ? j : 0] : oa;
-            const uint32_t wa[4] = {a.x, a.y, a.z, a.w}, wb[4] = {b.x, b.y, b.z, b.w};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-              uint32_t ea[4], eb[4];
-#pragma unroll
-              for (int q = 0; q < 4; ++q) {
-                if constexpr (kNatural) {
-                  const uint32_t va = wa[i] >> (8 * q), vb = wb[i] >> (8 * q);
-                  ea[q] = expand<F16>((va & 0xFu) | ((va & 0xF0u) << 12), oa);
-                  eb[q] = expand<F16>((vb & 0xFu) | ((vb & 0xF0u) << 12), ob);
-                } else {
-                  ea[q] = expand<F16>(wa[i] >> (4 * q), oa);
-                  eb[q] = expand<F16>(wb[i] >> (4 * q), ob);
-                }
-              }
-              mma<F16>(s[0], ea[0], eb[0], ea[1], eb[1], x[j][4 * i], x[j][4 * i + 1]);
-              mma<F16>(s[1], ea[2], eb[2], ea[3], eb[3], x[j][4 * i + 2], x[j][4 * i + 3]);
-            }
-            acc[0] = fmaf(f0[j], s[0][0] + s[1][0], acc[0]);
-            acc[1] = fmaf(f0[j], s[0][1] + s[1][1], acc[1]);
-            acc[2] = fmaf(f1[j], s[0][2] + s[1][2], acc[2]);
-            acc[3] = fmaf(f1[j], s[0][3] + s[1][3], acc[3]);
-          } else {
-            mma<F16>(acc, a.x, b.x, a.y, b.y, x[j][0], x[j][1]);
-            mma<F16>(acc, a.z, b.z, a.w, b.w, x[j][2], x[j][3]);
-          }
+          mma<F16>(acc, a.x, b.x, a.y, b.y, x[j][0], x[j][1]);
+          mma<F16>(acc, a.z, b.z, a.w, b.w, x[j][2], x[j][3]);
         }
         // the slot of the step before is free: its values were used by the products above it in program order
         if (done + kDepth - 1 < total) issue();
@@ -340,7 +236,6 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
       float v = 0.f;
 #pragma unroll
       for (int w = 0; w < kWarps; ++w) v += partial[buf][w][tok][r];
-      if constexpr (W4 && !F16) v *= kScaled;
       if (p.cluster > 1) {
         unit_sums[(u - u0) * 128 + threadIdx.x] = v;
       } else if constexpr (kGated) {
@@ -374,9 +269,12 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
 }
 
 // Launches the kernel for a problem whose Params hold everything but the split; 1 when the shape does not fit.
-template <bool F16, int WT, int ACT>
+template <bool F16, int ACT>
 int launch(Params p, int num_sms, cudaStream_t s) {
-  constexpr int kJ = WT != kHalf ? 4 : 16;
+  constexpr int kJ = 16;
+  auto kern = gemm_stream_kernel<F16, ACT, kJ>;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), 100 * 1024) != cudaSuccess) return -3;
+  ensure_max_carveout(reinterpret_cast<const void*>(kern));
   const int per_warp = (p.steps + kWarps - 1) / kWarps;
   p.cluster = 1;
   while (p.cluster < 8 && (per_warp + p.cluster - 1) / p.cluster > kJ) p.cluster *= 2;
@@ -387,9 +285,6 @@ int launch(Params p, int num_sms, cudaStream_t s) {
   const int grid = (p.units + p.units_per_cluster - 1) / p.units_per_cluster * p.cluster;
   const int smem = kRingBytes + (p.cluster > 1 ? p.units_per_cluster * 512 : 0);
   if (smem > 100 * 1024) return 1;
-  auto kern = gemm_stream_kernel<F16, WT, ACT, kJ>;
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), 100 * 1024) != cudaSuccess) return -3;
-  ensure_max_carveout(reinterpret_cast<const void*>(kern));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3(kThreads);

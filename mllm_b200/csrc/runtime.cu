@@ -4,6 +4,7 @@
 #include <cstdlib>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <utility>
 
 #include "common.cuh"
@@ -34,6 +35,35 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes) {
   err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
   if (err == cudaSuccess) set_to[{kernel, dev}] = bytes;
   return err;
+}
+
+int max_clusters(const void* kernel, int cluster, int threads, int smem, int fallback) {
+  static std::mutex mu;
+  static std::map<std::tuple<const void*, int, int, int, int>, int> known;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return fallback;
+  std::lock_guard<std::mutex> lock(mu);
+  const auto key = std::make_tuple(kernel, dev, cluster, threads, smem);
+  auto it = known.find(key);
+  if (it != known.end()) return it->second;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = static_cast<unsigned>(cluster);
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    n = fallback;
+  }
+  known[key] = n;
+  return n;
 }
 
 void ensure_max_carveout(const void* kernel) {
