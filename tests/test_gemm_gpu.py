@@ -219,3 +219,16 @@ def test_gemm_pair_tiles_of_other_widths(m, n, k, kind):
     for got, want in ((ops.linear(x, w), plain), (ops.linear(x, w, b, residual=r), plain + b.double() + r.double())):
         assert ((got.double() - want).abs() <= u * want.abs() + 2 ** -20 * (size + want.abs())).all()
     ops.check_status()
+
+
+@pytest.mark.parametrize("N,K", [(4744, 16896), (1200, 17408), (4656, 8704)])
+def test_weight_stream_over_as_many_clusters_as_the_device_holds(N, K):
+    """One row block more than there are clusters at once, so that the first of them have one more than the last.  fp32 sums in any
+    order, the output rounded to 8 bits: 2^-8 of it, and 2^-18 of the sum of the magnitudes."""
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x = torch.randn(3, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    got = ops.linear(x, w).double()
+    ops.check_status()
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert ((got - want).abs() <= 2 ** -8 * want.abs() + 2 ** -18 * size).all()
