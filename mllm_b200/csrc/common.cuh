@@ -478,10 +478,11 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes);
 // shared-memory array.
 void ensure_max_carveout(const void* kernel);
 
-// Host side: how many clusters of `cluster` CTAs of `kernel` (`threads` threads, `smem` dynamic bytes) the device holds at once; asked
-// once per set of arguments and device.  A cluster lies in one group of SMs, so the groups' remainders stay empty: of 296 places two per
-// SM, 284 in clusters of four and 264 in clusters of eight on the device measured.  `fallback`: what to take when the query fails.
-int max_clusters(const void* kernel, int cluster, int threads, int smem, int fallback);
+// Host side: how many clusters of `cluster` CTAs (`threads` threads, `smem` bytes of shared memory) the device holds at once; asked once
+// per set of arguments and device.  A cluster lies in one group of SMs, so the groups' remainders stay empty: of 296 places two per SM,
+// 284 in clusters of four and 264 in clusters of eight on the device measured.  The query is for a kernel that does nothing: for one that
+// allocates tensor memory it counts one CTA per SM, where two run.  `fallback`: what to take when the query fails.
+int max_clusters(int cluster, int threads, int smem, int fallback);
 
 // Host side: launch with the programmatic-stream-serialization attribute (MLLM_B200_PDL=0 turns
 // it off).  Works under stream capture: the dependency becomes a programmatic graph edge.

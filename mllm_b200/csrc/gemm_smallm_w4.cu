@@ -581,7 +581,7 @@ int launch(Params p, int num_sms, cudaStream_t s) {
   // 4096 x 12288 16.5 us instead of 12.8.  (Clusters where x fits without them, for fewer steps at most: 24576 x 4096 20.3 us, without 17.4.)
   const int all = (p.n + 15) / 16;
   const int places =
-      p.cluster == 1 ? 2 * num_sms : max_clusters(reinterpret_cast<const void*>(kern), p.cluster, kThreads, 100 * 1024, 2 * num_sms / (p.cluster + 1));
+      p.cluster == 1 ? 2 * num_sms : max_clusters(p.cluster, kThreads, 100 * 1024, 2 * num_sms / (p.cluster + 1));
   const int clusters = std::min(all, std::max(1, places));
   p.units_each = all / clusters;
   p.units_more = all % clusters;

@@ -272,7 +272,7 @@ __global__ void __launch_bounds__(kThreads, 2) gemm_stream_kernel(const Params p
 template <bool F16, int ACT>
 int launch(Params p, int num_sms, cudaStream_t s) {
   constexpr int kJ = 16;
-  constexpr int kMaxSmem = 110 * 1024, kSmem = 100 * 1024;      // at most; what two CTAs per SM may have beside the static part
+  constexpr int kMaxSmem = 110 * 1024;
   auto kern = gemm_stream_kernel<F16, ACT, kJ>;
   if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kMaxSmem) != cudaSuccess) return -3;
   ensure_max_carveout(reinterpret_cast<const void*>(kern));
@@ -284,8 +284,7 @@ int launch(Params p, int num_sms, cudaStream_t s) {
   // (n x k 5120 x 25600, 1 row: in 36 clusters of eight, of which the device holds 33 at once, 60.8 us, in 32 of them 41.4; 4096 x 12288
   // is 64 clusters of four either way)
   const int clusters =
-      p.cluster == 1 ? 2 * num_sms
-                     : std::max(1, max_clusters(reinterpret_cast<const void*>(kern), p.cluster, kThreads, kSmem, 2 * num_sms / (p.cluster + 1)));
+      p.cluster == 1 ? 2 * num_sms : std::max(1, max_clusters(p.cluster, kThreads, 110 * 1024, 2 * num_sms / (p.cluster + 1)));
   p.units_per_cluster = (p.units + clusters - 1) / clusters;
   const int grid = (p.units + p.units_per_cluster - 1) / p.units_per_cluster * p.cluster;
   const int smem = kRingBytes + (p.cluster > 1 ? p.units_per_cluster * 512 : 0);

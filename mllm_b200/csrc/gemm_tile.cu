@@ -336,12 +336,19 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   }
 }
 
+// Clusters of c CTAs that the device holds at once, one CTA per SM or two
+int places(int c, int per_sm, int num_sms) {
+  return c == 1 ? per_sm * num_sms : max_clusters(c, kTileThreads, (per_sm == 2 ? 104 : 200) * 1024, per_sm * num_sms / (c + 1));
+}
+
 template <int BN, int SWIGLU>
 int launch_tile(const CUtensorMap& tw, const CUtensorMap& tx, TileParams p, int grid, int num_sms, cudaStream_t s) {
   constexpr int kStageBytes = kWeightBytes + BN * kRowBytes;
   constexpr int kTail = 1024 + 512;
-  // a ring for one CTA per SM, or half of it for two; deep enough for the sums, which take its place
-  const int budget = (grid <= num_sms ? 200 : 104) * 1024;
+  // A ring for one CTA per SM, or half of it for two; deep enough for the sums, which take its place.  (One per SM, the device measured
+  // holds 15 clusters of eight.  With the whole ring for 16 of them the last ran behind the others: 29 rows of 2048 x 4096 11.0 us, with
+  // half of it 7.0.)
+  const int budget = (grid <= places(p.cluster, 1, num_sms) * p.cluster ? 200 : 104) * 1024;
   const int blocks = (p.k_blocks + p.cluster - 1) / p.cluster;
   p.stages = std::max(2, std::min(std::min((budget - kTail) / kStageBytes, 12), blocks));
   while (p.stages * kStageBytes < BN * kTileRows * 4) ++p.stages;
@@ -397,16 +404,21 @@ int launch_gemm_tile(const GemmArgs& a, cudaStream_t s) {
   // few weight rows: narrower tiles, until a cluster of eight per tile would fill the GPU
   while (bn > 32 && tiles(bn) * 8 <= sms) bn /= 2;
   if (tiles(bn) > 2 * sms) return 1;
+  // Clusters grow while every CTA keeps four stages (29 rows of 4096 x 1024: in clusters of eight, with two stages, 5.9 us, of four 5.1)
+  // and the device holds all of them at once, one CTA per SM: 128 rows of 6144 x 4096 17.7 us in 48 clusters of
+  // four, two CTAs per SM, and 15.2 in 48 of two; 29 rows of 9216 x 2560, 72 of four of which 71 fit, 15.7 and 10.7.  With up to 32
+  // columns a stage is little work and what a CTA waits for is memory: two CTAs per SM in clusters of four and eight (29 rows of
+  // 2048 x 4096: of four 7.5, of eight 7.0; 5120 x 5120: of two 13.4, of four 12.6).
   auto cluster_of = [&](int bn) {
     int c = 1;
-    while (c < 8 && tiles(bn) * c * 2 <= 2 * sms && p.k_blocks >= 4 * c) c *= 2;
+    while (c < 8 && p.k_blocks >= 8 * c &&
+           (tiles(bn) <= places(2 * c, 1, sms) || (bn <= 32 && c >= 2 && tiles(bn) <= places(2 * c, 2, sms))))
+      c *= 2;
     return c;
   };
   // Short k: what a CTA exchanges grows with the tile's width, what it multiplies with its share of k.  Narrower tiles in smaller
-  // clusters while the share is under bn / 16 stages (128 rows: 4096 x 1024 12.2 us with 128 columns and 2 stages per CTA, 8.4 with
-  // 64 and 4, 8.7 with 32 and 8; 6144 x 1024 gated 12.1, 9.9 with 64 and 8, 11.7 with 32 and 16; 200 rows of 4096 x 2560 14.4 with
-  // 128 and 10, 15.1 with 64 and 20).
-  while (bn > 32 && cluster_of(bn) > 1 && p.k_blocks / cluster_of(bn) * 16 < bn) bn /= 2;
+  // clusters while the share is under bn / 8 stages (200 rows of 4096 x 1024: 128 columns in clusters of two 8.6 us, 64 without 7.6).
+  while (bn > 32 && cluster_of(bn) > 1 && p.k_blocks / cluster_of(bn) * 8 < bn) bn /= 2;
   p.cluster = cluster_of(bn);
   p.out = a.out;
   p.bias = a.bias;

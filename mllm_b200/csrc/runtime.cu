@@ -37,13 +37,18 @@ cudaError_t ensure_dynamic_smem(const void* kernel, int bytes) {
   return err;
 }
 
-int max_clusters(const void* kernel, int cluster, int threads, int smem, int fallback) {
+namespace {
+__global__ void no_kernel() {}
+}  // namespace
+
+int max_clusters(int cluster, int threads, int smem, int fallback) {
   static std::mutex mu;
-  static std::map<std::tuple<const void*, int, int, int, int>, int> known;
+  static std::map<std::tuple<int, int, int, int>, int> known;
+  const void* kernel = reinterpret_cast<const void*>(no_kernel);
   int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess) return fallback;
+  if (cudaGetDevice(&dev) != cudaSuccess || ensure_dynamic_smem(kernel, 227 * 1024) != cudaSuccess) return fallback;
   std::lock_guard<std::mutex> lock(mu);
-  const auto key = std::make_tuple(kernel, dev, cluster, threads, smem);
+  const auto key = std::make_tuple(dev, cluster, threads, smem);
   auto it = known.find(key);
   if (it != known.end()) return it->second;
   cudaLaunchConfig_t cfg = {};

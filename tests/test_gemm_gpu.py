@@ -221,12 +221,13 @@ def test_gemm_pair_tiles_of_other_widths(m, n, k, kind):
     ops.check_status()
 
 
-@pytest.mark.parametrize("N,K", [(4744, 16896), (1200, 17408), (4656, 8704)])
-def test_weight_stream_over_as_many_clusters_as_the_device_holds(N, K):
-    """One row block more than there are clusters at once, so that the first of them have one more than the last.  fp32 sums in any
-    order, the output rounded to 8 bits: 2^-8 of it, and 2^-18 of the sum of the magnitudes."""
+@pytest.mark.parametrize("N,K", [(4744, 16896), (1200, 17408), (4656, 8704), (2048, 4096), (2304, 4096), (9216, 512)])
+@pytest.mark.parametrize("M", [3, 29, 128])
+def test_about_as_many_clusters_as_the_device_holds(M, N, K):
+    """Row blocks and tiles whose number is just over or under that of the clusters that run at once.  fp32 sums in any order, the
+    output rounded to 8 bits: 2^-8 of it, and 2^-18 of the sum of the magnitudes."""
     g = torch.Generator(device="cuda").manual_seed(N)
-    x = torch.randn(3, K, device="cuda", generator=g).bfloat16()
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
     w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
     got = ops.linear(x, w).double()
     ops.check_status()
