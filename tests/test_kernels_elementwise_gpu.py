@@ -131,3 +131,33 @@ def test_argmax(dtype):
     # bf16 ties: the kernel returns the lowest index among equal maxima
     assert torch.equal(logits.float().gather(1, got[:, None]), logits.float().gather(1, want[:, None]))
     assert got[3] == 77 and got[4] == 151935
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,k", [(1, 16), (3, 2064), (1023, 2048), (1025, 2048), (1027, 2064), (1026, 4112), (1030, 8192), (1025, 16400), (2, 32768)])
+def test_per_token_quant_int8_is_the_rounded_quotient(rows, k, dtype):
+    """Reciprocals are a short cut, not another result: whole numbers and the scale equal those of divisions in fp32, halves between two
+    integers, zeros, infinities and NaN included."""
+    g = torch.Generator(device=DEV).manual_seed(rows + k)
+    x = (torch.randn(rows, k, device=DEV, generator=g) * 3).to(dtype)
+    x[0, ::5] = torch.arange(-127, 128, device=DEV).repeat(k)[: (k + 4) // 5].to(dtype) / 2      # quotients at halves where absmax is 127 / 2
+    if rows > 2:
+        x[1] = 0
+        x[2, 3] = float("inf")
+        x[2, 4] = float("nan")
+    q, s = ops.per_token_quant_int8(x)
+    xf = x.float()
+    want_s = torch.where(xf.isnan(), 0.0, xf.abs()).amax(-1, keepdim=True).clamp_min(1e-10) / torch.full((1, 1), 127.0, device=DEV)
+    assert torch.equal(s, want_s)
+    # NaN goes to the lower bound, as fmaxf(NaN, -128) does
+    want = torch.round(xf / want_s).nan_to_num(nan=-128.0).clamp(-128, 127).to(torch.int8)
+    assert torch.equal(q, want)
+
+
+@pytest.mark.parametrize("rows,inter", [(1, 8), (5, 24), (2048, 3080), (301, 6144)])
+def test_act_and_mul_over_two_vectors_a_thread(rows, inter):
+    """Remainders of the loop: the second vector of a thread is there or not.  One rounding to 8 bits, at most 2^-8 of the result."""
+    g = torch.Generator(device=DEV).manual_seed(inter)
+    x = torch.randn(rows, 2 * inter, device=DEV, generator=g).bfloat16()
+    got, want = ops.silu_and_mul(x).double(), torch.nn.functional.silu(x[:, :inter].double()) * x[:, inter:].double()
+    assert ((got - want).abs() <= 2 ** -8 * want.abs() + 1e-30).all()
