@@ -420,6 +420,10 @@ int launch_gemm_tile(const GemmArgs& a, cudaStream_t s) {
   // clusters while the share is under bn / 8 stages (200 rows of 4096 x 1024: 128 columns in clusters of two 8.6 us, 64 without 7.6).
   while (bn > 32 && cluster_of(bn) > 1 && p.k_blocks / cluster_of(bn) * 8 < bn) bn /= 2;
   p.cluster = cluster_of(bn);
+  // Whole tiles of 128 x 128, more than half a wave of them and no gate: the persistent kernel, whose epilogue stores rows of the output as
+  // they come (512 rows of 4096 x 1024 9.3 us here, 8.0 there; 1024 of 2048 x 2048 12.4 and 11.1; 384 of 6144 x 4096 19.8 and 19.3; with
+  // SwiGLU 11.3 and 15.5, in two rounds instead of two per SM, 192 tiles of 512 x 6144 x 4096, 29.0 and 31.6, with 8-bit operands the same).
+  if (a.m > 256 && a.swiglu == 0 && !a.is_int8 && bn == 128 && tiles(bn) > places(2, 1, sms) && tiles(bn) <= sms) return 1;
   p.out = a.out;
   p.bias = a.bias;
   p.residual = a.residual;

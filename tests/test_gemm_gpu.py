@@ -233,3 +233,17 @@ def test_about_as_many_clusters_as_the_device_holds(M, N, K):
     ops.check_status()
     want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     assert ((got - want).abs() <= 2 ** -8 * want.abs() + 2 ** -18 * size).all()
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 3072, 264), (300, 3208, 264), (512, 4736, 136), (512, 4744, 136), (257, 6144, 1024)])
+def test_tiles_of_half_a_wave_to_one_wave(M, N, K):
+    """Either side of the two limits between the one-wave and the persistent kernel, with a bias.  fp32 sums in any order
+    (2^-18 of the magnitudes) and one rounding to 8 bits (2^-8 of the result)."""
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    x = torch.randn(M, K, device="cuda", generator=g).bfloat16()
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).bfloat16()
+    b = torch.randn(N, device="cuda", generator=g).bfloat16()
+    got = ops.linear(x, w, b).double()
+    ops.check_status()
+    want, size = x.double() @ w.double().t() + b.double(), x.double().abs() @ w.double().abs().t() + b.double().abs()
+    assert ((got - want).abs() <= 2 ** -8 * want.abs() + 2 ** -18 * size).all()
