@@ -508,12 +508,17 @@ __global__ void __launch_bounds__(kScanThreads, 1) gdn_scan_kernel(const Prefill
         for (int kk = 0; kk < 4; ++kk)
           umma_f16(t_ds, k0 + off + kk * (2048 >> 4), u_desc + ((2 * kPlane + kk * 2048) >> 4), id_kt, kk > 0 ? 1u : 0u);
         umma_commit(ds_full);
+        // rows 64 - 127 of the left operand are the scores; the plane in front fills the others.  16 tokens at a time, into the rows of
+        // these tokens and of those behind them: above the diagonal the scores are 0, and 0 times an infinity or a NaN is a NaN
+        auto scores_by_u = [&](int plane, uint32_t idesc, bool first) {
 #pragma unroll
-        for (int kk = 0; kk < 4; ++kk)      // rows 64 - 127 of the left operand are the scores; the plane in front fills the others
-          umma_f16(t_d3, st0 + off + ((Slot::kP - kPlane) >> 4) + kk * 2, u_desc + kk * (2048 >> 4), id_128, kk > 0 ? 1u : 0u);
-#pragma unroll
-        for (int kk = 0; kk < 4; ++kk)
-          umma_f16(t_d3, st0 + off + (Slot::kP >> 4) + kk * 2, u_desc + kk * (2048 >> 4), id_64, 1u);
+          for (int kk = 0; kk < 4; ++kk) {
+            const uint32_t off_rows[4] = {~0u, ~0u, kk == 0 ? 0u : kk == 1 ? 0xFFFFu : ~0u, kk == 3 ? 0xFFFFu : 0u};
+            umma_f16_rows(t_d3, st0 + off + ((plane - kPlane) >> 4) + kk * 2, u_desc + kk * (2048 >> 4), idesc, first && kk == 0 ? 0u : 1u, off_rows);
+          }
+        };
+        scores_by_u(Slot::kP, id_128, true);
+        scores_by_u(Slot::kP + kPlane, id_64, false);
         umma_commit(&left[st]);
       }
       if (!ok) *abort_flag = 1;

@@ -72,7 +72,7 @@ def test_decays(decay):
 def test_spans_of_the_workspace(lens, chunks, monkeypatch):
     """Room for one to five chunks at a time: spans of several chunks, the last one in part, that take the state up where the span before
     left it; fewer chunks than requests, which then come in groups."""
-    heads, slot = 6, 2 * 64 * 128 * 2 + 2 * 64 * 64 * 2 + 160 * 4 + 64 * 128 * 4      # of a (chunk, head): W and P in two terms, scalars, U0
+    heads, slot = 6, (2 * 64 * 128 + 2 * 64 * 128 + 2 * 64 * 64) * 2 + 160 * 4 + 64 * 128 * 4      # of a (chunk, head): W in two terms, Q, K, P in two terms, scalars, U0
     monkeypatch.setattr(ops, "GDN_WORKSPACE_BYTES", chunks * heads * slot)
     _check(lens, heads, 3, 128, 128)
 
@@ -128,3 +128,30 @@ def test_gated_norm_of_many_rows(tokens, heads, width, sigmoid):
     g = gate.double().reshape(tokens, heads, width)
     want = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-6) * w.double() * (torch.sigmoid(g) if sigmoid else g * torch.sigmoid(g))
     assert ((got - want).abs() <= (2 ** -8 + 2 ** -18) * want.abs() + 1e-30).all()
+
+
+@pytest.mark.parametrize("where", ["q", "k", "v", "g", "beta"])
+@pytest.mark.parametrize("value", [float("nan"), float("inf")])
+@pytest.mark.parametrize("token", [16, 31, 60, 64 + 50])
+def test_tokens_before_one_that_is_no_number(token, value, where):
+    """Tokens of the 16-token tiles in front of it, and other requests, are what they are without it, bit for bit."""
+    gen = torch.Generator(device="cuda").manual_seed(token)
+    lens, heads, d = [150, 70], 2, 128
+    x = {n: torch.randn((220, heads, d), generator=gen, device="cuda").bfloat16() for n in "qkv"}
+    x["g"], x["beta"] = -torch.rand((220, heads), generator=gen, device="cuda") * 0.1, torch.rand((220, heads), generator=gen, device="cuda")
+    i32 = dict(dtype=torch.int32, device="cuda")
+
+    def run():
+        state = torch.zeros(2, heads, d, d, device="cuda")
+        out = ops.gated_delta_rule(x["q"], x["k"], x["v"], x["g"], x["beta"], state, torch.arange(2, **i32), torch.tensor(lens, **i32),
+                                   torch.zeros(2, **i32), max_len=150)
+        ops.check_status()
+        return out, state
+
+    want, state = run()
+    x[where][token, 1] = value
+    got, after = run()
+    clean = token // 16 * 16
+    assert not got[token, 1].isfinite().all()
+    assert torch.equal(got[:clean], want[:clean]) and torch.equal(got[:, 0], want[:, 0]) and torch.equal(got[150:], want[150:])
+    assert torch.equal(after[1], state[1]) and torch.equal(after[0, 0], state[0, 0])
