@@ -326,6 +326,16 @@ class VisionLanguageMixin:
         (None, None) when the batch carries no image."""
         if fb.pixel_values is None or fb.image_grid_thw is None or fb.forward_mode.is_decode():
             return None, None
+        # The image rows are found on the host, in the ids that the positions were made from, and their indices are on the device before the
+        # tower is queued: the copy waits for what the stream holds by then, and asking the device for them would too.
+        ids = fb.extra.get("input_ids_cpu")
+        ids = (input_ids.cpu() if ids is None else ids).numpy()
+        mask = ids == self.image_token_id
+        if self.video_token_id is not None:
+            mask |= ids == self.video_token_id
+        rows = np.flatnonzero(mask)
+        n_tok = len(rows)
+        where = torch.from_numpy(rows).to(input_ids.device)
         sync = bool(getattr(fb, "benchmark_vision_timing", False)) and input_ids.is_cuda
         if sync:
             torch.cuda.synchronize()
@@ -334,19 +344,10 @@ class VisionLanguageMixin:
         if sync:
             torch.cuda.synchronize()
         fb.vit_prefill_ms = (time.perf_counter() - t0) * 1e3
-        # the rows are found on the host, in the ids that the positions were made from: asking the device for them would wait for the tower
-        ids = fb.extra.get("input_ids_cpu")
-        ids = (input_ids.cpu() if ids is None else ids).numpy()
-        mask = ids == self.image_token_id
-        if self.video_token_id is not None:
-            mask |= ids == self.video_token_id
-        rows = np.flatnonzero(mask)
-        n_tok = len(rows)
         fb.vit_prefill_tokens = n_tok
         if n_tok != feats.shape[0]:
             raise ValueError(f"Image features and image tokens do not match, tokens: {n_tok}, features: {feats.shape[0]}")
         input_embeds = self.model.embed_tokens(input_ids)
-        where = torch.from_numpy(rows).to(input_ids.device)
         input_embeds.index_copy_(0, where, feats[:, : self.hidden_size].to(input_embeds.dtype))
         deepstack = None
         if self.num_deepstack:

@@ -122,3 +122,43 @@ def test_vision_tower_graph_replay_equals_eager(monkeypatch):
             assert torch.equal(got, want[(gi, s)]), (gi, s)
     assert len(vis.__dict__["_graphs"]) == 1
     ops.check_status()
+
+
+def test_no_wait_between_the_tower_and_the_decoder():
+    """Once the tower is queued the host queues the decoder: no call in between waits for the device."""
+    from mllm_b200.bench_one_batch import make_multimodal_inputs
+    from mllm_b200.configs import ServerConfig
+    from mllm_b200.executor import ModelRunner
+    from mllm_b200.models.presets import get_preset
+
+    cfg = get_preset("qwen3-vl-tiny")
+    mr = ModelRunner(ServerConfig(model_path="preset:qwen3-vl-tiny", dtype="bfloat16", max_running_requests=2, max_total_tokens=1024,
+                                  disable_cuda_graph=True), hf_config=cfg, device="cuda:0")
+    mr.initialize()
+    reached = []
+
+    def decoder_begins(*_):
+        torch.cuda.set_sync_debug_mode("default")
+        reached.append(True)
+
+    image = torch.randint(0, 256, (64, 96, 3), dtype=torch.uint8, generator=torch.Generator().manual_seed(0))
+    ids, pix, grid = make_multimodal_inputs(hf_config=cfg, batch_size=1, input_len=40, image=image, seed=0)
+    L = ids.shape[1]
+    slots = mr.req_to_token_pool.alloc(1)
+    loc = mr.token_to_kv_pool_allocator.alloc(L)
+    sl = torch.tensor(slots, device="cuda")
+    mr.req_to_token_pool.req_to_token[sl.long(), :L] = loc.view(1, L).int()
+    lens = torch.full((1,), L, device="cuda", dtype=torch.int32)
+    logits = []
+    try:
+        for step in range(2):            # the first call of a grid captures the tower
+            if step:
+                mr.model.visual.register_forward_hook(lambda *_: torch.cuda.set_sync_debug_mode("error"))
+                mr.model.model.layers[0].register_forward_pre_hook(decoder_begins)
+            fb = mr.prepare_forward_batch_extend(ids.reshape(-1).cuda().long(), sl, lens, lens, torch.zeros_like(lens), loc,
+                                                 extend_seq_lens_cpu=[L], extend_prefix_lens_cpu=[0], pixel_values=pix.cuda(), image_grid_thw=grid.cuda())
+            logits.append(mr.forward(fb).next_token_logits)
+    finally:
+        torch.cuda.set_sync_debug_mode("default")
+    ops.check_status()
+    assert reached and torch.equal(*logits)
