@@ -303,6 +303,7 @@ constexpr int kRingBytes = kWarps * kDepth * kSlotBytes;
 constexpr int kXStep = 2048;                  // x of a step: [8 k per lane][lane], 16 bytes each
 constexpr int kMaxSteps = 32;                 // of a CTA's part of k: 64 KB of x
 constexpr int kPart = 128;                    // sums of a row block: [row of x][weight row]
+constexpr int kHalfSm = 112 * 1024, kWholeSm = 226 * 1024;      // shared memory of a CTA where an SM holds two, and one
 
 struct Params {
   const uint8_t* x;
@@ -570,7 +571,7 @@ __global__ void __launch_bounds__(kThreads, 2) w4_stream_kernel(const Params p) 
 template <bool F16, bool NATURAL, bool ZEROS>
 int launch(Params p, int num_sms, cudaStream_t s) {
   auto kern = w4_stream_kernel<F16, NATURAL, ZEROS>;
-  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), 226 * 1024) != cudaSuccess) return -3;
+  if (ensure_dynamic_smem(reinterpret_cast<const void*>(kern), kWholeSm) != cudaSuccess) return -3;
   ensure_max_carveout(reinterpret_cast<const void*>(kern));
   if ((p.steps + 7) / 8 > kMaxSteps || static_cast<int64_t>(p.n) * p.groups >= (int64_t(1) << 31)) return 1;
   while ((1 << p.m_log) < p.m) ++p.m_log;
@@ -580,16 +581,27 @@ int launch(Params p, int num_sms, cudaStream_t s) {
   // Two CTAs per SM, whole row blocks each, as many clusters as the device holds at once: three more of 71, behind all the others, made
   // 4096 x 12288 16.5 us instead of 12.8.  (Clusters where x fits without them, for fewer steps at most: 24576 x 4096 20.3 us, without 17.4.)
   const int all = (p.n + 15) / 16;
-  const int places =
-      p.cluster == 1 ? 2 * num_sms : max_clusters(p.cluster, kThreads, 100 * 1024, 2 * num_sms / (p.cluster + 1));
-  const int clusters = std::min(all, std::max(1, places));
-  p.units_each = all / clusters;
-  p.units_more = all % clusters;
-  const int units = p.units_each + (p.units_more > 0 ? 1 : 0);
-  // a run is at most ceil(units * steps / kWarps) steps: it touches one row block more than it has whole ones' worth of steps
-  p.slots = std::min(units, (units + kWarps - 1) / kWarps + 1);
-  const int smem = p.max_steps * kXStep + kRingBytes + kWarps * p.slots * kPart * 4 + (p.cluster > 1 ? units * kPart * 4 : 0);
-  if (smem > 226 * 1024) return 1;
+  int smem = 0;
+  auto split = [&](int per_sm) {
+    const int places = p.cluster == 1 ? per_sm * num_sms
+                                      : max_clusters(p.cluster, kThreads, per_sm == 2 ? kHalfSm : kWholeSm, per_sm * num_sms / (p.cluster + 1));
+    const int clusters = std::min(all, std::max(1, places));
+    p.units_each = all / clusters;
+    p.units_more = all % clusters;
+    const int units = p.units_each + (p.units_more > 0 ? 1 : 0);
+    // a run is at most ceil(units * steps / kWarps) steps: it touches one row block more than it has whole ones' worth of steps
+    p.slots = std::min(units, (units + kWarps - 1) / kWarps + 1);
+    smem = p.max_steps * kXStep + kRingBytes + kWarps * p.slots * kPart * 4 + (p.cluster > 1 ? units * kPart * 4 : 0);
+    return clusters;
+  };
+  int clusters = split(2);
+  if (smem > kHalfSm) {
+    // sums of so many row blocks leave an SM room for one: as many clusters as run at once then, if their sums fit (2 rows, n x k, in
+    // two rounds and in one: 10240 x 8192 20.6 and 17.5 us, 28672 x 8192 44.5 and 41.1, 32768 x 16384 136.8 and 96.2)
+    clusters = split(1);
+    if (smem > kWholeSm) clusters = split(2);
+  }
+  if (smem > kWholeSm) return 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(clusters * p.cluster);
   cfg.blockDim = dim3(kThreads);

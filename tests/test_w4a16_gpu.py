@@ -88,12 +88,13 @@ def test_w4a16_streaming_kernel_for_a_handful_of_rows(M, N, K, group, zeros, int
 
 
 @pytest.mark.parametrize("N,K,group", [(8, 128, 128), (200, 256, 256), (1048, 4096, 4096), (4744, 384, 128), (61576, 128, 128), (2056, 4224, 128),
-                                       (1000, 25600, 256)])
+                                       (1000, 25600, 256), (28680, 8192, 128), (57352, 4096, 256), (28000, 32768, 128)])
 @pytest.mark.parametrize("M,zeros", [(3, False), (8, True)])
 def test_w4a16_stream_where_runs_and_row_blocks_do_not_match(M, N, K, group, zeros):
     """Half a row block at the end, fewer steps than warps, runs over several row blocks, scales of many steps, k that a cluster shares
-    unequally.  The fp32 sums of the products are exact up to their order, so only the rounding of the output to 8 bits (at most 2^-8 of
-    it) shows, and 2^-18 of the sum of the magnitudes for k up to 25600."""
+    unequally, sums that leave an SM room for one CTA (with and without clusters), and for none of as few clusters.  The fp32 sums of the
+    products are exact up to their order, so only the rounding of the output to 8 bits (at most 2^-8 of it) shows, and 2^-18 of the sum of
+    the magnitudes for k up to 32768."""
     x, qw, sc, z, b = _case(M, N, K, group, zeros=zeros, bias=True, dtype=torch.bfloat16, seed=N + K)
     w = ref.dequant_w4(qw, sc.float(), z, group).double()
     want = x.double() @ w.t() + b.double()
