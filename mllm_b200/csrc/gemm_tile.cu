@@ -336,19 +336,34 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_constant
   }
 }
 
-// Clusters of c CTAs that the device holds at once, one CTA per SM or two
-int places(int c, int per_sm, int num_sms) {
-  return c == 1 ? per_sm * num_sms : max_clusters(c, kTileThreads, (per_sm == 2 ? 104 : 200) * 1024, per_sm * num_sms / (c + 1));
+// Clusters of 1, 2, 4 and 8 CTAs that the device holds at once, one CTA per SM or two.  A thread keeps the counts of the device that it
+// launched on last: a launch asks for up to a dozen, and from the maps of max_clusters they took the host 1 us of the 12.5 per product.
+struct Places {
+  int of[2][4];
+  int operator()(int c, int per_sm) const { return of[per_sm - 1][c == 1 ? 0 : c == 2 ? 1 : c == 4 ? 2 : 3]; }
+};
+const Places& places_of_device(int num_sms) {
+  thread_local Places known;
+  thread_local int device = -1;
+  int dev = -1;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev != device) {
+    for (int per_sm = 1; per_sm <= 2; ++per_sm)
+      for (int i = 0; i < 4; ++i)
+        known.of[per_sm - 1][i] = i == 0 ? per_sm * num_sms
+                                         : max_clusters(1 << i, kTileThreads, (per_sm == 2 ? 104 : 200) * 1024, per_sm * num_sms / ((1 << i) + 1));
+    device = dev;
+  }
+  return known;
 }
 
 template <int BN, int SWIGLU>
-int launch_tile(const CUtensorMap& tw, const CUtensorMap& tx, TileParams p, int grid, int num_sms, cudaStream_t s) {
+int launch_tile(const CUtensorMap& tw, const CUtensorMap& tx, TileParams p, int grid, const Places& places, cudaStream_t s) {
   constexpr int kStageBytes = kWeightBytes + BN * kRowBytes;
   constexpr int kTail = 1024 + 512;
   // A ring for one CTA per SM, or half of it for two; deep enough for the sums, which take its place.  (One per SM, the device measured
   // holds 15 clusters of eight.  With the whole ring for 16 of them the last ran behind the others: 29 rows of 2048 x 4096 11.0 us, with
   // half of it 7.0.)
-  const int budget = (grid <= places(p.cluster, 1, num_sms) * p.cluster ? 200 : 104) * 1024;
+  const int budget = (grid <= places(p.cluster, 1) * p.cluster ? 200 : 104) * 1024;
   const int blocks = (p.k_blocks + p.cluster - 1) / p.cluster;
   p.stages = std::max(2, std::min(std::min((budget - kTail) / kStageBytes, 12), blocks));
   while (p.stages * kStageBytes < BN * kTileRows * 4) ++p.stages;
@@ -376,12 +391,12 @@ int launch_tile(const CUtensorMap& tw, const CUtensorMap& tx, TileParams p, int 
 }
 
 template <int SWIGLU>
-int launch_bn(int bn, const CUtensorMap& tw, const CUtensorMap& tx, const TileParams& p, int grid, int num_sms, cudaStream_t s) {
+int launch_bn(int bn, const CUtensorMap& tw, const CUtensorMap& tx, const TileParams& p, int grid, const Places& places, cudaStream_t s) {
   switch (bn) {
-    case 16: return launch_tile<16, SWIGLU>(tw, tx, p, grid, num_sms, s);
-    case 32: return launch_tile<32, SWIGLU>(tw, tx, p, grid, num_sms, s);
-    case 64: return launch_tile<64, SWIGLU>(tw, tx, p, grid, num_sms, s);
-    default: return launch_tile<128, SWIGLU>(tw, tx, p, grid, num_sms, s);
+    case 16: return launch_tile<16, SWIGLU>(tw, tx, p, grid, places, s);
+    case 32: return launch_tile<32, SWIGLU>(tw, tx, p, grid, places, s);
+    case 64: return launch_tile<64, SWIGLU>(tw, tx, p, grid, places, s);
+    default: return launch_tile<128, SWIGLU>(tw, tx, p, grid, places, s);
   }
 }
 
@@ -404,6 +419,7 @@ int launch_gemm_tile(const GemmArgs& a, cudaStream_t s) {
   // few weight rows: narrower tiles, until a cluster of eight per tile would fill the GPU
   while (bn > 32 && tiles(bn) * 8 <= sms) bn /= 2;
   if (tiles(bn) > 2 * sms) return 1;
+  const Places& places = places_of_device(sms);
   // Clusters grow while every CTA keeps four stages (29 rows of 4096 x 1024: in clusters of eight, with two stages, 5.9 us, of four 5.1)
   // and the device holds all of them at once, one CTA per SM: 128 rows of 6144 x 4096 17.7 us in 48 clusters of
   // four, two CTAs per SM, and 15.2 in 48 of two; 29 rows of 9216 x 2560, 72 of four of which 71 fit, 15.7 and 10.7.  With up to 32
@@ -412,7 +428,7 @@ int launch_gemm_tile(const GemmArgs& a, cudaStream_t s) {
   auto cluster_of = [&](int bn) {
     int c = 1;
     while (c < 8 && p.k_blocks >= 8 * c &&
-           (tiles(bn) <= places(2 * c, 1, sms) || (bn <= 32 && c >= 2 && tiles(bn) <= places(2 * c, 2, sms))))
+           (tiles(bn) <= places(2 * c, 1) || (bn <= 32 && c >= 2 && tiles(bn) <= places(2 * c, 2))))
       c *= 2;
     return c;
   };
@@ -423,7 +439,7 @@ int launch_gemm_tile(const GemmArgs& a, cudaStream_t s) {
   // Whole tiles of 128 x 128, more than half a wave of them and no gate: the persistent kernel, whose epilogue stores rows of the output as
   // they come (512 rows of 4096 x 1024 9.3 us here, 8.0 there; 1024 of 2048 x 2048 12.4 and 11.1; 384 of 6144 x 4096 19.8 and 19.3; with
   // SwiGLU 11.3 and 15.5, in two rounds instead of two per SM, 192 tiles of 512 x 6144 x 4096, 29.0 and 31.6, with 8-bit operands the same).
-  if (a.m > 256 && a.swiglu == 0 && !a.is_int8 && bn == 128 && tiles(bn) > places(2, 1, sms) && tiles(bn) <= sms) return 1;
+  if (a.m > 256 && a.swiglu == 0 && !a.is_int8 && bn == 128 && tiles(bn) > places(2, 1) && tiles(bn) <= sms) return 1;
   p.out = a.out;
   p.bias = a.bias;
   p.residual = a.residual;
@@ -446,11 +462,11 @@ int launch_gemm_tile(const GemmArgs& a, cudaStream_t s) {
   if (!make_tma_operand_map(&tx, a.a, a.m, a.k, a.lda, eb, type, bn)) return -2;
   const int grid = static_cast<int>(tiles(bn)) * p.cluster;
   switch (a.swiglu) {
-    case 1: return launch_bn<1>(bn, tw, tx, p, grid, sms, s);
-    case 2: return launch_bn<2>(bn, tw, tx, p, grid, sms, s);
-    case 3: return launch_bn<3>(bn, tw, tx, p, grid, sms, s);
-    case 4: return launch_bn<4>(bn, tw, tx, p, grid, sms, s);
-    default: return launch_bn<0>(bn, tw, tx, p, grid, sms, s);
+    case 1: return launch_bn<1>(bn, tw, tx, p, grid, places, s);
+    case 2: return launch_bn<2>(bn, tw, tx, p, grid, places, s);
+    case 3: return launch_bn<3>(bn, tw, tx, p, grid, places, s);
+    case 4: return launch_bn<4>(bn, tw, tx, p, grid, places, s);
+    default: return launch_bn<0>(bn, tw, tx, p, grid, places, s);
   }
 }
 
