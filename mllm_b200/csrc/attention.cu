@@ -1033,7 +1033,8 @@ int decode_num_splits(int batch, int hkv, int max_seq_len, int num_sms) {
 }
 
 // Prefill through the warp-specialised kernel; returns 1 when this launch is not for it (storage that is neither
-// head-major nor slot-major, or MLLM_B200_ATTN_PREFILL=legacy) and the single-role kernel should run instead.
+// head-major nor slot-major, too few registers for its roles, or MLLM_B200_ATTN_PREFILL=legacy) and the single-role kernel should run
+// instead.
 int launch_prefill_ws(AttnParams p, const AttnArgs& a, cudaStream_t s) {
   const char* knob = std::getenv("MLLM_B200_ATTN_PREFILL");   // read per call: tests switch it
   const bool legacy = knob != nullptr && std::string(knob) == "legacy";
@@ -1053,12 +1054,13 @@ int launch_prefill_ws(AttnParams p, const AttnArgs& a, cudaStream_t s) {
   const int q_tiles = (a.max_q_len + p.tokens_per_tile - 1) / p.tokens_per_tile;
   if (q_tiles <= 0) return 0;
   {
-    // the softmax warps take registers that the others give back: together no more than the kernel is launched with
+    // the softmax warps take registers that the others give back: together no more than the kernel is launched with.  A compiler that
+    // gives it fewer leaves the launch to the single-role kernel
     static const int regs = [] {
       cudaFuncAttributes at{};
       return cudaFuncGetAttributes(&at, reinterpret_cast<const void*>(attn_prefill_ws_kernel)) == cudaSuccess ? at.numRegs : 0;
     }();
-    if (regs * kPfThreads < 128 * (kPfSoftmaxRegs + kPfOtherRegs)) return -3;
+    if (regs * kPfThreads < 128 * (kPfSoftmaxRegs + kPfOtherRegs)) return 1;
   }
   ensure_max_carveout(reinterpret_cast<const void*>(attn_prefill_ws_kernel));
   const cudaError_t err = launch_pdl(attn_prefill_ws_kernel, dim3(q_tiles, a.hkv, a.batch), dim3(kPfThreads), kPfSmem, s,

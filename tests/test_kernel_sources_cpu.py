@@ -74,3 +74,10 @@ def test_read_only_loads_without_a_fence_are_of_parameters(source):
     if "pdl_wait_loads()" in text and "pdl_wait()" not in text:
         for m in re.finditer(r"__ldg\(", text):
             assert any(name in text[m.end():m.end() + 70] for name in PARAMETERS), text[m.start():m.end() + 70]
+
+
+def test_prefill_attention_without_its_registers_is_left_to_the_other_kernel():
+    """Fewer registers than the roles share out are a compiler's choice and no error of the call: 1 takes the single-role kernel."""
+    text = (CSRC / "attention.cu").read_text()
+    launch = text[text.index("int launch_prefill_ws("):]
+    assert re.search(r"if \(regs \*[^;]*\) return (-?\d+);", launch[:launch.index("\n}\n")]).group(1) == "1"
