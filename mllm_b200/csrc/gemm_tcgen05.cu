@@ -850,10 +850,11 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_con
 
 
 // =========================================================================================
-// Two-CTA tiling (large m): a cluster of two CTAs on neighbouring SMs computes one 256 x 256 output
-// tile with tcgen05.mma.cta_group::2.  Each CTA stages 128 activation rows (its half of the tile's M)
-// and 128 weight rows (its half of the tile's N) per 64-element k-block: 32 KB per CTA and k-block
-// instead of the 48 KB a lone CTA needs for its 128 x 256 tile, i.e. a third less traffic from L2 into
+// Two-CTA tiling (large m): a cluster of two CTAs on neighbouring SMs computes one output tile of 256 rows
+// and 256 columns (224 or 192 where that leaves fewer or fuller rounds of tiles) with
+// tcgen05.mma.cta_group::2.  Each CTA stages 128 activation rows (its half of the tile's M)
+// and half the tile's weight rows (its half of the tile's N, 128 at most) per 64-element k-block: 32 KB per CTA and
+// k-block instead of the 48 KB a lone CTA needs for its 128 x 256 tile, i.e. a third less traffic from L2 into
 // shared memory per FLOP, which is what bounds the one-CTA tiling.  The leader CTA (cluster rank 0)
 // issues the MMAs for the pair; the hardware reads the A rows and the B half of each CTA from that CTA's
 // shared memory and writes each CTA's 128 accumulator rows into that CTA's tensor memory.
@@ -965,7 +966,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tm_row, const __grid_consta
 
   const int pair = blockIdx.x >> 1;
   const int num_pairs = gridDim.x >> 1;
-  const int total_tiles = p.tiles_r * p.tiles_c;   // tiles of 256 x 256
+  const int total_tiles = p.tiles_r * p.tiles_c;   // tiles of 256 x bn
   auto get_tile = [&](int idx, int& tr, int& tc) -> bool {
     const int tile = pair + idx * num_pairs;
     if (tile >= total_tiles) return false;
@@ -1438,7 +1439,7 @@ int launch_gemm(const GemmArgs& a, cudaStream_t s) {
   p.gate_flags = a.gate_flags;
   p.gate_epoch = a.gate_epoch;
   if (a.m > 256) {
-    // ---- two-CTA tiling: 256 x 256 tiles per pair of SMs, when there are enough of them to fill the GPU ----
+    // ---- two-CTA tiling: tiles of 256 x 256, 224 or 192 per pair of SMs, when there are enough of 256 x 256 to fill the GPU ----
     static const int pair_knob = env_int("MLLM_B200_GEMM_PAIR", 1);
     const int64_t tiles_pair = static_cast<int64_t>((a.m + 2 * kBM - 1) / (2 * kBM)) * ((a.n + kPairBN - 1) / kPairBN);
     const bool pair_rs_ok = a.rs_tp == 0 || (!gated && (a.m / kBM / a.rs_tp) % 2 == 0);

@@ -198,11 +198,23 @@ def test_add_rmsnorm_fused_into_the_streaming_gemm(monkeypatch, m, n, k, swiglu,
     assert _rel_err(y9, want9) < 8e-3
 
 
-@pytest.mark.parametrize("m,n,k", [(1551, 4096, 512), (1100, 5120, 512), (1100, 5120, 2048), (1300, 4352, 256)])
+def _pair_width(m, n, k_bytes):
+    """Columns of a tile of the two-CTA tiling: rounds of tiles times what a tile costs, two per cent less per step to a narrower one."""
+    rows, pairs = -(-m // 256), torch.cuda.get_device_properties(DEV).multi_processor_count // 2
+    assert n % 256 == 0 and rows * (n // 256) >= pairs
+    cost = {bn: -(-rows * -(-n // bn) // pairs) * (-(-k_bytes // 128) * bn + 4 * 256) for bn in (256, 224, 192)}
+    width = 256
+    for bn in (224, 192):
+        width = bn if cost[bn] * 100 < cost[width] * 98 else width
+    return width
+
+
+@pytest.mark.parametrize("m,n,k,width", [(1551, 4096, 512, 224), (1100, 5120, 512, 192), (1100, 5120, 2048, 192), (1300, 4352, 256, 192)])
 @pytest.mark.parametrize("kind", ["bf16", "fp16", "int8"])
-def test_gemm_pair_tiles_of_other_widths(m, n, k, kind):
+def test_gemm_pair_tiles_of_other_widths(m, n, k, width, kind):
     """Tiles of 224 and 192 columns of the two-CTA tiling, whose last tile ends inside the matrix.  Products of 16-bit values are exact in
     fp32; beside the output's rounding the sums' order shows, below 2^-20 of the sum of the magnitudes at these k."""
+    assert _pair_width(m, n, k if kind == "int8" else 2 * k) == width
     g = torch.Generator(device=DEV).manual_seed(m + n)
     if kind == "int8":
         x, w = (torch.randint(-127, 128, (r, k), generator=g, device=DEV, dtype=torch.int8) for r in (m, n))
