@@ -7,8 +7,8 @@
 //     others leave at most two partial results per CTA, which a second kernel joins.  The line is laid out on the device from
 //     the sequence lengths, so a captured graph serves any batch.  (A grid of requests x heads x splits, with the splits
 //     taken from the longest length the host allows for, and roles that meet at mbarriers, took 87.5 us for 29 requests of 400 to
-//     3400 tokens and 8 kv heads, 128 us for 64 x 2048 and 4 heads, 25.9 us for 8 x 2048 and 8 heads; now 44.1, 53.9 and 20.7 us,
-//     joining included; the bytes take 34, 40 and 10 us.)
+//     3400 tokens and 8 kv heads, 128 us for 64 x 2048 and 4 heads, 25.9 us for 8 x 2048 and 8 heads; dealt evenly 44.1, 53.9 and 20.7
+//     us before what the next lines say, joining included; the bytes take 34, 40 and 10 us.)
 //     The chain in front of the first copy (lengths, table, rows; queries and the table's row beside them; no 64-bit division) and the
 //     meeting of the warps are 4 us of a CTA's time when each load waits for the one before; side by side, and four values a thread:
 //     2 x 1500 (8 kv heads) 11.4 -> 9.3 us, 8 x 2048 20.9 -> 18.2, 1 x 160 7.3 -> 6.8, 29 x 1900 46.0 -> 42.2, joining included.
