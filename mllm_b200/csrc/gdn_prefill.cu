@@ -16,8 +16,8 @@
 // scan's are tcgen05 with accumulators in tensor memory: what bounds the scan is the chain from one chunk's state to the next, and of a
 // chunk's 2032 warp-level MMAs, their fragment loads and the addresses of its copies it made 12300 cycles.
 //
-// Measured (16 heads of 128 x 128; one kernel with tf32 operands, two kernels with warp-level MMAs in both, these): 4 x 2000 tokens
-// 1274, 383, 223 us, 1 x 2048 582, 130, 121; 8 x 1000 395 -> 241, 1 x 300 34.1 -> 32.0.
+// Measured (16 heads of 128 x 128, the longest length given; one kernel with tf32 operands, two kernels with warp-level MMAs in both, these):
+// 4 x 2000 tokens 1274, 375, 212 us, 1 x 2048 582, 128, 113; 8 x 1000 374 -> 217, 8 x 2048 734 -> 412, 1 x 300 33.3 -> 31.5.
 #include <algorithm>
 
 #include "common.cuh"
@@ -671,9 +671,10 @@ static_assert(2 * (kPrepareSmem + 1024) <= 228 * 1024, "two CTAs of the first ke
 bool gdn_prefill_covers(const GdnRuleParams& p) { return p.dt == kBF16 && !p.split_tf32 && gdn_chunk_covers(p); }
 
 // As many chunks of all requests as `most_bytes` have room for; where not even one fits, one chunk of equal groups of requests.  The
-// least is a chunk of one request.  (Groups that fill the GPU once, with longer spans, leave the scan's last CTAs of every group
-// alone: 32 x 1024 tokens 1467 us instead of 1388 with 512 MB.  128 MB instead of 512: 4 x 2000 tokens 450 us instead of 432,
-// 32 x 1024 1651.)
+// least is a chunk of one request.  A (chunk, head) takes 115328 bytes at 128 value features, Q and K as the scan's operands among them:
+// 512 MB are 72 chunks of four requests of 16 heads.  A span costs a start of both kernels and the state's way through memory: 32 x 1024
+// tokens 854 us with 512 MB, 1186 with 128 MB, 788 with 4 GB; 4 x 2000 212, 230 and 212.  (Groups of requests that fill the GPU once, with
+// longer spans, leave the scan's last CTAs of every group alone; with the scan by warp-level MMAs 1467 us instead of 1388.)
 GdnPrefillPlan gdn_prefill_plan(const GdnRuleParams& p, int max_len, int64_t most_bytes) {
   const int64_t chunk = slot_bytes(p.dv) * p.heads, slots = std::max<int64_t>(1, most_bytes / chunk);
   const int64_t batch = std::max(1, p.batch), groups = (batch + slots - 1) / slots, group = (batch + groups - 1) / groups;
